@@ -26,6 +26,7 @@
 #include "snp_common.cuh"
 #include "snp_internal.cuh"
 #include "snp_krylov.cuh"
+#include "snp_reduce.cuh"
 
 namespace snp {
 namespace {
@@ -91,7 +92,20 @@ bool spd_solve(int m, const double *A, const double *g, double *c) {
     return true;
 }
 
-// res[0] += sum over free i of v[i]^2 (deterministic last-block reduction)
+// Block-wide maximum of non-negative values; result valid in thread 0.  `sh` holds 32 values.
+__device__ __forceinline__ double block_max(double v, double *sh) {
+    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        v = threadIdx.x < (blockDim.x >> 5) ? sh[threadIdx.x] : 0.0;
+        for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    }
+    return v;
+}
+
+// res[0] = sum over free i of v[i]^2 (deterministic last-block reduction)
 // res[1]  = max over all i of |v[i]|; res[2] = max |v - w| and res[3] = max |v| (when w != null)
 __global__ void k_vstats(int32_t n, const uint8_t *__restrict__ fm, const double *__restrict__ v,
                          const double *__restrict__ w, double *part, unsigned int *counter, double *res) {
@@ -103,44 +117,32 @@ __global__ void k_vstats(int32_t n, const uint8_t *__restrict__ fm, const double
         mx = fmax(mx, fabs(a));
         if (w) md = fmax(md, fabs(a - w[i]));
     }
-    // sum
+    // this block's partials
+    __shared__ double shx[32], shd[32];
     ss = block_sum(ss, sh);
-    __syncthreads();
-    // max via warp shuffles
-    for (int o = 16; o > 0; o >>= 1) {
-        mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        md = fmax(md, __shfl_xor_sync(0xffffffffu, md, o));
-    }
-    __shared__ double smx[32], smd[32];
-    if ((threadIdx.x & 31) == 0) {
-        smx[threadIdx.x >> 5] = mx;
-        smd[threadIdx.x >> 5] = md;
-    }
-    __syncthreads();
+    mx = block_max(mx, shx);
+    md = block_max(md, shd);
     if (threadIdx.x == 0) {
-        for (int k = 1; k < (int)(blockDim.x >> 5); ++k) {
-            mx = fmax(mx, smx[k]);
-            md = fmax(md, smd[k]);
-        }
         part[3 * blockIdx.x] = ss;
         part[3 * blockIdx.x + 1] = mx;
         part[3 * blockIdx.x + 2] = md;
-        __threadfence();
     }
-    __shared__ bool last;
-    __syncthreads();
-    if (threadIdx.x == 0) last = atomicInc(counter, gridDim.x - 1) == gridDim.x - 1;
-    __syncthreads();
-    if (last && threadIdx.x == 0) {
-        double s = 0.0, m = 0.0, d = 0.0;
-        for (unsigned int b = 0; b < gridDim.x; ++b) {
-            s += __ldcg(part + 3 * b);
+    // The last block's threads share the partials (592 of them at full size).  One thread walking
+    // them serially was most of the launch: 46 us at 1.39M DoFs and 15 us at 44k.
+    if (last_block(counter)) {
+        double m = 0.0, d = 0.0;
+        for (unsigned int b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
             m = fmax(m, __ldcg(part + 3 * b + 1));
             d = fmax(d, __ldcg(part + 3 * b + 2));
         }
-        res[0] = s;
-        res[1] = m;
-        res[2] = d;
+        const double s = reduce_parts(part, (int)gridDim.x, 3, 0, sh);
+        m = block_max(m, shx);
+        d = block_max(d, shd);
+        if (threadIdx.x == 0) {
+            res[0] = s;
+            res[1] = m;
+            res[2] = d;
+        }
     }
 }
 
@@ -151,17 +153,11 @@ __global__ void k_vdot(int32_t n, const uint8_t *__restrict__ fm, const double *
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         if (fm[i]) s += a[i] * b[i];
     s = block_sum(s, sh);
-    __shared__ bool last;
-    if (threadIdx.x == 0) {
-        part[blockIdx.x] = s;
-        __threadfence();
-        last = atomicInc(counter, gridDim.x - 1) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (last && threadIdx.x == 0) {
-        double t = 0.0;
-        for (unsigned int k = 0; k < gridDim.x; ++k) t += __ldcg(part + k);
-        res[0] = t;
+    if (threadIdx.x == 0) part[blockIdx.x] = s;
+    // the last block's threads share the partials, as in k_vstats (29 us by one thread at 1.39M DoFs)
+    if (last_block(counter)) {
+        const double t = reduce_parts(part, (int)gridDim.x, 1, 0, sh);
+        if (threadIdx.x == 0) res[0] = t;
     }
 }
 
