@@ -279,13 +279,23 @@ class CurlCurlAssembler:
         """B at the mesh nodes by averaging the element fields of the materials ``mat_ids``
         (volume tags) around each node (``curl_curl_assembler.py:2089-2196``); nodes outside
         them get 0.  Returns float64 [N, 3] (numpy)."""
-        mask = np.zeros(self.mesh.num_elements, dtype=np.uint8)
+        return self.nodal_fields_device(x, mat_ids).cpu().numpy()
+
+    def nodal_fields_device(self, x, mat_ids):
+        """``compute_nodal_fields`` as a CUDA tensor.  Each material's element mask is uploaded once."""
+        d = self._device_state()
+        masks = d.setdefault("elem_masks", {})
+        mask = None
         for mid in mat_ids:
             n = list(self.volume_tags).index(mid)
-            mask[self._elems[n]] = 1
-        B = self.element_B_device(x)
-        out = self.mesh.index().nodal_average(B, 3, upload(mask, np.uint8))
-        return out.cpu().numpy()
+            if n not in masks:
+                m = np.zeros(self.mesh.num_elements, dtype=np.uint8)
+                m[self._elems[n]] = 1
+                masks[n] = upload(m, np.uint8)
+            mask = masks[n] if mask is None else mask | masks[n]
+        if mask is None:  # no material: every node gets 0
+            mask = upload(np.zeros(self.mesh.num_elements, dtype=np.uint8), np.uint8)
+        return self.mesh.index().nodal_average(self.element_B_device(x), 3, mask)
 
     def compute_B_at_points(self, x, points, elements=None):
         """B = curl A at arbitrary points (element constant for first order); points outside give 0."""

@@ -11,6 +11,8 @@ import numpy as np
 from . import _lib
 from . import finite_element as fe
 from .device import torch, upload, zeros
+from .fem_c import biot_savart_device
+from .racetrack_coil import RacetrackCoil
 
 
 def _located(mesh, positions, vol_tags):
@@ -21,9 +23,11 @@ def _located(mesh, positions, vol_tags):
     el = elem.cpu().numpy().astype(np.int64)
     dom = np.full(len(el), -1, dtype=np.int32)
     ok = el >= 0
-    tags = list(vol_tags)
-    lookup = {t: i for i, t in enumerate(tags)}
-    dom[ok] = [lookup.get(int(t), -1) for t in mesh.elem_domain[el[ok]]]
+    tag_of = mesh.elem_domain[el[ok]]
+    found = np.full(len(tag_of), -1, dtype=np.int32)
+    for i, t in enumerate(vol_tags):  # a repeated tag: its last position
+        found[tag_of == t] = i
+    dom[ok] = found
     el[dom < 0] = -1
     return upload(el, np.int32), bary, upload(dom, np.int32), el
 
@@ -57,8 +61,8 @@ def evaluate_interpolation(positions, gmsh_model, vol_tags, nodal_values):
     mesh = gmsh_model
     t = torch()
     el_d, bary, dom_d, _ = _located(mesh, positions, vol_tags)
-    first = np.asarray(nodal_values[0] if not hasattr(nodal_values[0], "data_ptr") else nodal_values[0].cpu().numpy())
-    nc = 1 if first.ndim == 1 else first.shape[1]
+    first = nodal_values[0] if hasattr(nodal_values[0], "data_ptr") else np.asarray(nodal_values[0])
+    nc = 1 if first.ndim == 1 else int(first.shape[1])
     stack = []
     for v in nodal_values:
         v_d = v if hasattr(v, "data_ptr") else upload(np.asarray(v, dtype=np.float64), np.float64)
@@ -73,9 +77,16 @@ def evaluate_interpolation(positions, gmsh_model, vol_tags, nodal_values):
 def evaluate_fem_solution_node_interpolation(gmsh_model, points, solver, coil_list, x, domain_list):
     """B at ``points`` by interpolating nodal averages (``evaluators.py:413-454``): per domain of
     ``domain_list`` the element fields averaged at the nodes plus the coils' field at the nodes."""
-    nodes = solver.curl_curl_factory.nodes
-    b_coil = 0.0 * nodes
+    t = torch()
+    asm = solver.curl_curl_factory
+    nodes_d = upload(asm.nodes, np.float64)
+    b_coil = t.zeros_like(nodes_d)
     for coil in coil_list:
-        b_coil = b_coil + coil.compute_B(nodes)
-    b_node_list = [solver.curl_curl_factory.compute_nodal_fields(x, [indx]) + b_coil for indx in domain_list]
+        if type(coil) is RacetrackCoil:  # its compute_B, without the copies to the host and back
+            b = biot_savart_device(upload(coil.get_segments(), np.float64), nodes_d, coil.current, coil.rad)
+        else:
+            b = upload(coil.compute_B(asm.nodes), np.float64)
+        b_coil = b_coil + b[: nodes_d.numel()]
+    b_coil = b_coil.view(-1, 3)
+    b_node_list = [asm.nodal_fields_device(x, [indx]) + b_coil for indx in domain_list]
     return evaluate_interpolation(points, gmsh_model, domain_list, b_node_list)
