@@ -252,7 +252,7 @@ def compute_B_line_segs_cpp(src, tar, current, radius):
 def biot_savart_device(src_t, tar_t, current, radius, out=None):
     """Biot-Savart on device tensors (src [S*6], tar [T*3]) -> B [T*3] device tensor."""
     n_tar = tar_t.numel() // 3
-    B = out if out is not None else zeros(3 * n_tar)
+    B = out if out is not None else torch().empty(max(3 * n_tar, 1), dtype=torch().float64, device=tar_t.device)
     _lib.call("snp_biot_savart", _lib.ptr(src_t), src_t.numel() // 6, _lib.ptr(tar_t), n_tar, float(current),
               float(radius), _lib.ptr(B), _lib.stream_ptr())
     return B

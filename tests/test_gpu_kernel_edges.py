@@ -28,3 +28,115 @@ def test_locate_point_counts(oracle_mod, n_pts, tets):
     assert np.array_equal(el, elo)
     # barycentric coordinates: a few float64 roundings of ratios of order-one determinants
     assert np.abs(bary - baryo).max() < 1e-12
+
+
+NU0 = 0.25e7 / np.pi
+
+
+def _assert_rows_close(a, b, row_ptr, tol):
+    a, b, rp = a.double().cpu().numpy(), b.double().cpu().numpy(), row_ptr.cpu().numpy()
+    rows = np.repeat(np.arange(len(rp) - 1), np.diff(rp))
+    rmax = np.zeros(len(rp) - 1)
+    np.maximum.at(rmax, rows, np.abs(b))
+    assert (np.abs(a - b) <= tol * rmax[rows]).all()
+
+
+@pytest.mark.parametrize("order", [1, 2, 3, 4])
+@pytest.mark.parametrize("n_iron", [1, 127, 129])
+def test_packed_assembly_matches_atomic(order, n_iron):
+    """The packed two-phase assembly: every quadrature branch, iron ranges below, at and above an
+    element tile, against the kernels that add into the CSR (other order of the same sums: a
+    few roundings of the row's largest entry)."""
+    msh = M.window_frame_mesh(2000, jitter=0.15, seed=3)
+    dom = np.full(msh.num_elements, M.TAG_AIR, dtype=np.int32)
+    dom[100:100 + n_iron] = M.TAG_IRON
+    msh.elem_domain = dom
+    A = S.CurlCurlAssembler(msh, [M.TAG_AIR, M.TAG_IRON], [S.ConstantReluctance(NU0), MAT.atan_reluctance()])
+    rng = np.random.default_rng(order)
+    x = rng.normal(0, 2e-3, msh.num_dofs)
+    bs = rng.normal(0, 0.5, (n_iron * A.tables(order).nq, 3))
+    sf = [np.zeros((0, 3)), bs]
+    kw = dict(K=True, J=True, dK=True, rhs=True, F=True)
+    R, T = (A.assemble_device(x, order, sf, method=m, **kw) for m in ("rows", "atomic"))
+    for key in ("K", "dK", "J"):
+        _assert_rows_close(R[key], T[key], A.pattern.row_ptr, 1e-12)
+    for key in ("rhs", "F"):
+        assert rel_max(R[key].cpu().numpy(), T[key].cpu().numpy()) < 1e-12
+
+
+def test_packed_assembly_many_ranges():
+    """40 materials, every other one without a source field and with constant reluctance: more
+    separate ranges than the packed form's tables hold."""
+    msh = M.window_frame_mesh(3000, jitter=0.15, seed=3)
+    n_mat = 40
+    msh.elem_domain = (100 + np.arange(msh.num_elements) * n_mat // msh.num_elements).astype(np.int32)
+    rel = MAT.atan_reluctance()
+    mats = [S.ConstantReluctance(NU0) if i % 2 else rel for i in range(n_mat)]
+    A = S.CurlCurlAssembler(msh, [100 + i for i in range(n_mat)], mats)
+    rng = np.random.default_rng(1)
+    x = rng.normal(0, 2e-3, msh.num_dofs)
+    nq = A.tables(2).nq
+    sf = [np.zeros((0, 3)) if i % 2 else rng.normal(0, 0.5, (len(A._elems[i]) * nq, 3)) for i in range(n_mat)]
+    for kw in (dict(K=True, J=True, dK=True, rhs=True, F=True), dict(K=True, J=True, dK=True, rhs=False, F=True)):
+        R, T = (A.assemble_device(x, 2, sf, method=m, **kw) for m in ("rows", "atomic"))
+        for key in ("K", "dK", "J"):
+            _assert_rows_close(R[key], T[key], A.pattern.row_ptr, 1e-12)
+        assert rel_max(R["F"].cpu().numpy(), T["F"].cpu().numpy()) < 1e-12
+        if kw["rhs"]:
+            assert rel_max(R["rhs"].cpu().numpy(), T["rhs"].cpu().numpy()) < 1e-12
+
+
+def test_block_and_packed_element_values_agree():
+    """The C entry points with the documented block layout and the whole-system call sum the same
+    values in the same order: bitwise equal."""
+    import ctypes
+
+    import torch
+    from snoopy_b200 import _lib
+
+    msh = M.window_frame_mesh(3000, jitter=0.15, seed=9)
+    A = S.CurlCurlAssembler(msh, [M.TAG_IRON, M.TAG_AIR], [MAT.atan_reluctance(), S.ConstantReluctance(NU0)])
+    rng = np.random.default_rng(2)
+    x = torch.from_numpy(rng.normal(0, 2e-3, msh.num_dofs)).cuda()
+    tb, d, pat = A.tables(2), A._device_state(), A.pattern
+    sf = [rng.normal(0, 0.5, (d["mats"][0]["count"] * tb.nq, 3)), np.zeros((0, 3))]
+    R = A.assemble_device(x, 2, sf, method="rows", K=True, J=True, dK=True, rhs=True, F=True)
+    bs = A.upload_source_fields(sf)
+    parts, stride = 1 | 2 | 8 | 16, ctypes.c_int32()
+    _lib.call("snp_curlcurl_terms_stride", parts, ctypes.byref(stride))
+    terms = torch.empty(pat.n_elems * stride.value, dtype=torch.float64, device="cuda")
+    for n, m in enumerate(d["mats"]):
+        n_int, rc, rx = d["rel"][n]
+        _lib.call("snp_curlcurl_terms", pat.handle, m["offset"], m["count"], _lib.ptr(d["nodes"]), _lib.ptr(m["cells"]),
+                  _lib.ptr(m["gids"]), _lib.ptr(m["orient"]), _lib.ptr(tb.curls_d), tb.n_orient, None,
+                  _lib.ptr(tb.d_phi_d), _lib.ptr(tb.w_d), tb.nq, _lib.ptr(x), _lib.ptr(bs[n]), n_int, _lib.ptr(rc),
+                  _lib.ptr(rx), None, parts, _lib.ptr(terms), _lib.stream_ptr())
+    out = {k: torch.empty_like(R[k]) for k in ("K", "dK", "J", "rhs", "F")}
+    _lib.call("snp_curlcurl_rows", pat.handle, _lib.ptr(terms), parts, _lib.ptr(out["K"]), _lib.ptr(out["dK"]),
+              _lib.ptr(out["J"]), None, _lib.ptr(out["rhs"]), _lib.ptr(out["F"]), _lib.stream_ptr())
+    for k in out:
+        assert torch.equal(out[k], R[k]), k
+
+
+@pytest.mark.parametrize("n_tar", [1, 31, 1000, 12000, 25000, 50000, 80000])
+@pytest.mark.parametrize("n_src", [1, 15, 16, 129])
+def test_biot_savart_shapes(oracle_mod, n_tar, n_src):
+    """Every lane split, tiles with a remainder; targets inside cores, near their surface, in line
+    with segments and far away.  The sums of both sides differ by rounding only: within 1e-12 of
+    the sum of the terms' magnitudes, here bounded by the field of the nearest filaments."""
+    rng = np.random.default_rng(n_tar + n_src)
+    a = rng.uniform(-1, 1, (n_src, 3))
+    src = np.concatenate([a, a + rng.normal(0, 0.3, (n_src, 3))], axis=1)
+    rad = 0.02
+    tar = rng.uniform(-1.5, 1.5, (n_tar, 3))
+    k = min(n_tar, 400)
+    j = rng.integers(0, n_src, k)
+    t = rng.uniform(-1.0, 2.0, k)[:, None]
+    axis = src[j, 3:] - src[j, :3]
+    off = np.cross(axis, rng.normal(size=(k, 3)))
+    off *= (rad * rng.choice([0.1, 0.5, 0.999, 1.001, 1.5, 40.0], k) / np.linalg.norm(off, axis=1))[:, None]
+    tar[:k] = src[j, :3] + t * axis + off
+    got = fem_c.compute_B_line_segs_cpp(src, tar, 250.0, rad)
+    ref = oracle_mod.compute_B_line_segs_cpp(src, tar, 250.0, rad)
+    scale = 250.0 * 1e-7 * 2.0 / rad * max(1.0, np.sqrt(n_src))  # field at the surface of a core
+    assert np.isfinite(ref).all() and np.abs(got - ref).max() < 1e-12 * scale
