@@ -170,6 +170,27 @@ int snp_curlcurl_rows(const snp_pattern *pat, const double *terms, int32_t parts
                       double *K_vals, double *dK_vals, double *J_vals, float *J32_vals,
                       double *rhs, double *F, void *stream);
 
+/* The same two-phase assembly of a whole system in one call, with element values kept in a layout
+ * of its own in `work` (snp_curlcurl_system_work doubles; contents are not an output): the
+ * materials' elements together are the pattern's, in order.  Every requested output is
+ * overwritten; J = K + dK per entry; results are bitwise repeatable and equal those of
+ * snp_curlcurl_terms + snp_curlcurl_rows. */
+typedef struct {
+    int64_t elem_offset, n_elems;   /* the pattern's elements [elem_offset, elem_offset + n_elems) */
+    const int32_t *cells, *glob_ids, *orientations;
+    const double *B_s;              /* [n_elems][Q][3] or NULL */
+    const double *rel_c, *rel_x;    /* reluctance tables, n_int intervals (-1: constant) */
+    const double *phi;              /* diluted steel: nodal basis f64[Q][4], else NULL */
+    double dilution[4];             /* with phi: {c_num, m_num, c_den, m_den} */
+    int32_t n_int, reserved;
+} snp_curlcurl_material;
+int snp_curlcurl_system_work(const snp_pattern *pat, int32_t want_K, int32_t want_dK, int32_t want_J, int32_t want_rhs,
+                             int32_t want_F, int64_t *n_doubles);
+int snp_curlcurl_system(const snp_pattern *pat, int32_t n_mats, const snp_curlcurl_material *mats /* host */,
+                        const double *nodes, const double *curls, int32_t n_orient, const double *d_phi,
+                        const double *w, int32_t n_quad, const double *x, double *work, double *K_vals,
+                        double *dK_vals, double *J_vals, double *rhs, double *F, void *stream);
+
 /* ------------------------------------------------------------------ grad-grad assembly
  * Replaces fem_c.compute_stiffness_and_jacobi_matrix (fem_c/interface_c.pyx:11-160)
  * -> compute_K_dK (fem_c/ctools.c:730-919).  P1 nodal elements [elem_offset, +n_elems)

@@ -59,6 +59,15 @@ class BatchInfo(ctypes.Structure):
         return d
 
 
+class CurlCurlMaterial(ctypes.Structure):
+    """``snp_curlcurl_material``: one material of ``snp_curlcurl_system``."""
+
+    _fields_ = [("elem_offset", ctypes.c_int64), ("n_elems", ctypes.c_int64), ("cells", ctypes.c_void_p),
+                ("glob_ids", ctypes.c_void_p), ("orientations", ctypes.c_void_p), ("B_s", ctypes.c_void_p),
+                ("rel_c", ctypes.c_void_p), ("rel_x", ctypes.c_void_p), ("phi", ctypes.c_void_p),
+                ("dilution", ctypes.c_double * 4), ("n_int", ctypes.c_int32), ("reserved", ctypes.c_int32)]
+
+
 # name -> argtypes (every function returns int32 status unless listed in _RESTYPES)
 _SIGS = {
     "snp_last_error": [],
@@ -79,6 +88,9 @@ _SIGS = {
     "snp_curlcurl_rows_supported": [_vp, ctypes.POINTER(_c_i32)],
     "snp_curlcurl_terms": [_vp, _c_i64, _c_i64, _vp, _vp, _vp, _vp, _vp, _c_i32, _vp, _vp, _vp, _c_i32, _vp, _vp,
                            _c_i32, _vp, _vp, _vp, _c_i32, _vp, _vp],
+    "snp_curlcurl_system_work": [_vp, _c_i32, _c_i32, _c_i32, _c_i32, _c_i32, ctypes.POINTER(_c_i64)],
+    "snp_curlcurl_system": [_vp, _c_i32, _vp, _vp, _vp, _c_i32, _vp, _vp, _c_i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp,
+                            _vp],
     "snp_curlcurl_rows": [_vp, _vp, _c_i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp],
     "snp_solver_set_krylov": [_vp, _c_i32, _c_i32],
     "snp_curlcurl_rhs_red": [_c_i64, _vp, _vp, _vp, _vp, _vp, _c_i32, _vp, _vp, _c_i32, _vp, _vp, _c_i32, _vp, _vp,

@@ -99,203 +99,260 @@ __device__ __forceinline__ double nu_at(const CurlArgs &a, const double *relc, c
     }
 }
 
-// HAS_BS: reduced formulation with a source field at each quadrature point.
-// NQ: compile-time number of quadrature points (0 = runtime count).
-// DIL: diluted steel (with HAS_BS only).
-template <bool HAS_BS, int NQ, typename VT, bool DIL>
-__global__ void __launch_bounds__(kBlock)
-    k_curlcurl(CurlArgs a, int quad_stride_ctab) {
-    extern __shared__ double sm[];
-    const SmemLayout L = smem_layout(a.n_orient, a.nq, a.n_int);
-    double *s_ctab = sm + L.off_ctab;
-    double *s_dphi = sm + L.off_dphi;
-    double *s_w = sm + L.off_w;
-    double *s_phi = sm + L.off_phi;
-    double *s_relc = sm + L.off_relc;
-    double *s_relx = sm + L.off_relx;
-    // stage tables: curls at q = 0 for every orientation, d_phi at q = 0, weights, PCHIP
-    for (int t = threadIdx.x; t < a.n_orient * 18; t += blockDim.x) {
-        int o = t / 18, r = t - o * 18;
-        s_ctab[t] = a.ctab[(int64_t)o * quad_stride_ctab + r];
-    }
-    for (int t = threadIdx.x; t < 12; t += blockDim.x) s_dphi[t] = a.dphi0[t];
-    for (int t = threadIdx.x; t < a.nq; t += blockDim.x) s_w[t] = a.w[t];
-    if (a.phi)
-        for (int t = threadIdx.x; t < 4 * a.nq; t += blockDim.x) s_phi[t] = a.phi[t];
-    const int nc = a.n_int < 0 ? 1 : 4 * a.n_int;
-    const int nx = a.n_int < 0 ? 1 : a.n_int + 1;
-    for (int t = threadIdx.x; t < nc; t += blockDim.x) s_relc[t] = a.rel_c[t];
-    for (int t = threadIdx.x; t < nx; t += blockDim.x) s_relx[t] = (a.n_int < 0) ? 0.0 : a.rel_x[t];
-    __syncthreads();
-
+// One element's K and dK (upper triangle), residual terms Fj = (K x)_j - r_j and reduced-rhs terms
+// r_j.  emit(tri, j, k, kv, dv) is called for the 21 pairs j <= k row by row; r is set only with
+// HAS_BS (a source field at each quadrature point).  NQ: compile-time number of quadrature points
+// (0 = runtime count); DIL: diluted steel (with HAS_BS only).  The tables sit in shared memory.
+template <bool HAS_BS, int NQ, bool DIL, typename Emit>
+__device__ __forceinline__ void curl_element(const CurlArgs &a, int64_t e, const double *s_ctab, const double *s_dphi,
+                                             const double *s_w, const double *s_phi, const double *s_relc,
+                                             const double *s_relx, double wsum, int (&g)[6], double (&Fj)[6],
+                                             double (&r)[6], Emit emit) {
     const int nq = NQ > 0 ? NQ : a.nq;
-    double wsum = 0.0;
-    for (int q = 0; q < nq; ++q) wsum += s_w[q];
+    const int4 cv = __ldg(reinterpret_cast<const int4 *>(a.cells) + e);
+    const int cidx[4] = {cv.x, cv.y, cv.z, cv.w};
+    // Jacobian J[k][l] = sum_i X[i][k] dphi[i][l]
+    double Jm[9], Zn[4];
+#pragma unroll
+    for (int t = 0; t < 9; ++t) Jm[t] = 0.0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const double X0 = __ldg(a.nodes + 3 * (int64_t)cidx[i]);
+        const double X1 = __ldg(a.nodes + 3 * (int64_t)cidx[i] + 1);
+        const double X2 = __ldg(a.nodes + 3 * (int64_t)cidx[i] + 2);
+        Zn[i] = X2;
+#pragma unroll
+        for (int l = 0; l < 3; ++l) {
+            const double d = s_dphi[3 * i + l];
+            Jm[0 + l] += X0 * d;
+            Jm[3 + l] += X1 * d;
+            Jm[6 + l] += X2 * d;
+        }
+    }
+    const double det = Jm[0] * (Jm[4] * Jm[8] - Jm[7] * Jm[5]) - Jm[1] * (Jm[3] * Jm[8] - Jm[5] * Jm[6]) +
+                       Jm[2] * (Jm[3] * Jm[7] - Jm[4] * Jm[6]);
+    const double idet = 1.0 / det;
+    const int o = __ldg(a.orient + e);
+    const double *ct = s_ctab + o * 18;
+    {
+        const int2 *gp = reinterpret_cast<const int2 *>(a.gids + 6 * e);
+        int2 g01 = __ldg(gp), g23 = __ldg(gp + 1), g45 = __ldg(gp + 2);
+        g[0] = g01.x; g[1] = g01.y; g[2] = g23.x; g[3] = g23.y; g[4] = g45.x; g[5] = g45.y;
+    }
+    double c[6][3], xv[6];
+    double Bc[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+    for (int j = 0; j < 6; ++j) {
+        const double h0 = ct[3 * j], h1 = ct[3 * j + 1], h2 = ct[3 * j + 2];
+        c[j][0] = Jm[0] * h0 + Jm[1] * h1 + Jm[2] * h2;
+        c[j][1] = Jm[3] * h0 + Jm[4] * h1 + Jm[5] * h2;
+        c[j][2] = Jm[6] * h0 + Jm[7] * h1 + Jm[8] * h2;
+        xv[j] = __ldg(a.x + g[j]);
+        Bc[0] += c[j][0] * xv[j];
+        Bc[1] += c[j][1] * xv[j];
+        Bc[2] += c[j][2] * xv[j];
+    }
+    Bc[0] *= idet;
+    Bc[1] *= idet;
+    Bc[2] *= idet;
 
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < a.n_elems; e += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t eo = a.t_offset + e;
-        const int4 cv = __ldg(reinterpret_cast<const int4 *>(a.cells) + e);
-        const int cidx[4] = {cv.x, cv.y, cv.z, cv.w};
-        // Jacobian J[k][l] = sum_i X[i][k] dphi[i][l]
-        double Jm[9], Zn[4];
+    double kfac;  // sum_q nu_q w_q / det
+    if constexpr (!HAS_BS) {
+        const double bm = sqrt(Bc[0] * Bc[0] + Bc[1] * Bc[1] + Bc[2] * Bc[2]);
+        double dnu;
+        const double nu = pchip_eval<double>(a.n_int, s_relc, s_relx, bm, dnu);
+        kfac = nu * wsum * idet;
+        const double af = (bm >= 1e-14) ? dnu * wsum * idet / bm : 0.0;
+        double p[6];
 #pragma unroll
-        for (int r = 0; r < 9; ++r) Jm[r] = 0.0;
+        for (int j = 0; j < 6; ++j) p[j] = c[j][0] * Bc[0] + c[j][1] * Bc[1] + c[j][2] * Bc[2];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const double X0 = __ldg(a.nodes + 3 * (int64_t)cidx[i]);
-            const double X1 = __ldg(a.nodes + 3 * (int64_t)cidx[i] + 1);
-            const double X2 = __ldg(a.nodes + 3 * (int64_t)cidx[i] + 2);
-            Zn[i] = X2;
-#pragma unroll
-            for (int l = 0; l < 3; ++l) {
-                const double d = s_dphi[3 * i + l];
-                Jm[0 + l] += X0 * d;
-                Jm[3 + l] += X1 * d;
-                Jm[6 + l] += X2 * d;
-            }
-        }
-        const double det = Jm[0] * (Jm[4] * Jm[8] - Jm[7] * Jm[5]) - Jm[1] * (Jm[3] * Jm[8] - Jm[5] * Jm[6]) +
-                           Jm[2] * (Jm[3] * Jm[7] - Jm[4] * Jm[6]);
-        const double idet = 1.0 / det;
-        const int o = __ldg(a.orient + e);
-        const double *ct = s_ctab + o * 18;
-        int g[6];
-        {
-            const int2 *gp = reinterpret_cast<const int2 *>(a.gids + 6 * e);
-            int2 g01 = __ldg(gp), g23 = __ldg(gp + 1), g45 = __ldg(gp + 2);
-            g[0] = g01.x; g[1] = g01.y; g[2] = g23.x; g[3] = g23.y; g[4] = g45.x; g[5] = g45.y;
-        }
-        double c[6][3], xv[6];
-        double Bc[3] = {0.0, 0.0, 0.0};
+        for (int j = 0; j < 6; ++j) Fj[j] = 0.0;
+        int tri = 0;
 #pragma unroll
         for (int j = 0; j < 6; ++j) {
-            const double h0 = ct[3 * j], h1 = ct[3 * j + 1], h2 = ct[3 * j + 2];
-            c[j][0] = Jm[0] * h0 + Jm[1] * h1 + Jm[2] * h2;
-            c[j][1] = Jm[3] * h0 + Jm[4] * h1 + Jm[5] * h2;
-            c[j][2] = Jm[6] * h0 + Jm[7] * h1 + Jm[8] * h2;
-            xv[j] = __ldg(a.x + g[j]);
-            Bc[0] += c[j][0] * xv[j];
-            Bc[1] += c[j][1] * xv[j];
-            Bc[2] += c[j][2] * xv[j];
+#pragma unroll
+            for (int k = j; k < 6; ++k, ++tri) {
+                const double kv = kfac * (c[j][0] * c[k][0] + c[j][1] * c[k][1] + c[j][2] * c[k][2]);
+                const double dv = af * p[j] * p[k];
+                emit(tri, j, k, kv, dv);
+                Fj[j] = __fma_rn(kv, xv[k], Fj[j]);  // the same rounding in every kernel built on this
+                if (k != j) Fj[k] = __fma_rn(kv, xv[j], Fj[k]);
+            }
         }
-        Bc[0] *= idet;
-        Bc[1] *= idet;
-        Bc[2] *= idet;
-
-        double kfac;                 // sum_q nu_q w_q / det
-        double Fj[6];
-        const bool want_mat = (a.K != nullptr) | (a.dK != nullptr) | (a.J != nullptr) | (a.J32 != nullptr);
-        const int32_t *sl = want_mat ? a.slots + 36 * e : nullptr;
-        if constexpr (!HAS_BS) {
-            const double bm = sqrt(Bc[0] * Bc[0] + Bc[1] * Bc[1] + Bc[2] * Bc[2]);
+    } else {
+        // one pass over the quadrature points: accumulate sum_q nu w, the reduced rhs
+        // and the 21 dK pair sums (any number of points, fixed register footprint)
+        double dk[21];
+#pragma unroll
+        for (int t = 0; t < 21; ++t) dk[t] = 0.0;
+#pragma unroll
+        for (int j = 0; j < 6; ++j) r[j] = 0.0;
+        kfac = 0.0;
+        const double *bs = a.Bs + (int64_t)e * nq * 3;
+#pragma unroll(NQ > 0 ? NQ : 1)
+        for (int q = 0; q < nq; ++q) {
+            const double s0 = __ldg(bs + 3 * q), s1 = __ldg(bs + 3 * q + 1), s2 = __ldg(bs + 3 * q + 2);
+            const double B0 = s0 + Bc[0], B1 = s1 + Bc[1], B2 = s2 + Bc[2];
+            const double bm = sqrt(B0 * B0 + B1 * B1 + B2 * B2);
             double dnu;
-            const double nu = pchip_eval<double>(a.n_int, s_relc, s_relx, bm, dnu);
-            kfac = nu * wsum * idet;
-            const double af = (bm >= 1e-14) ? dnu * wsum * idet / bm : 0.0;
+            const double nu = nu_at<DIL>(a, s_relc, s_relx, s_phi + 4 * q, Zn, bm, dnu);
+            const double wq = s_w[q];
+            kfac += nu * wq;
+            const double aq = (bm >= 1e-14) ? dnu * wq * idet / bm : 0.0;
+            const double rq = (kNu0 - nu) * wq;
             double p[6];
 #pragma unroll
-            for (int j = 0; j < 6; ++j) p[j] = c[j][0] * Bc[0] + c[j][1] * Bc[1] + c[j][2] * Bc[2];
-#pragma unroll
-            for (int j = 0; j < 6; ++j) Fj[j] = 0.0;
-            int tri = 0;
-#pragma unroll
             for (int j = 0; j < 6; ++j) {
-#pragma unroll
-                for (int k = j; k < 6; ++k, ++tri) {
-                    const double kv = kfac * (c[j][0] * c[k][0] + c[j][1] * c[k][1] + c[j][2] * c[k][2]);
-                    const double dv = af * p[j] * p[k];
-                    if (a.ET) store_pair(a, tri, eo, kv, dv);
-                    const int s1 = want_mat ? __ldg(sl + j * 6 + k) : 0;
-                    if (a.K) red_add(a.K + s1, kv);
-                    if (a.dK) red_add(a.dK + s1, dv);
-                    if (a.J) red_add(a.J + s1, kv + dv);
-                    if (a.J32) red_add(a.J32 + s1, (float)(kv + dv));
-                    Fj[j] += kv * xv[k];
-                    if (k != j) {
-                        const int s2 = want_mat ? __ldg(sl + k * 6 + j) : 0;
-                        if (a.K) red_add(a.K + s2, kv);
-                        if (a.dK) red_add(a.dK + s2, dv);
-                        if (a.J) red_add(a.J + s2, kv + dv);
-                        if (a.J32) red_add(a.J32 + s2, (float)(kv + dv));
-                        Fj[k] += kv * xv[j];
-                    }
-                }
-            }
-            if (a.F) {
-#pragma unroll
-                for (int j = 0; j < 6; ++j) red_add(a.F + g[j], Fj[j]);
-            }
-            if (a.ET) store_vectors(a, eo, Fj, nullptr);
-        } else {
-            // one pass over the quadrature points: accumulate sum_q nu w, the reduced rhs
-            // and the 21 dK pair sums (any number of points, fixed register footprint)
-            double dk[21], r[6];
-#pragma unroll
-            for (int t = 0; t < 21; ++t) dk[t] = 0.0;
-#pragma unroll
-            for (int j = 0; j < 6; ++j) r[j] = 0.0;
-            kfac = 0.0;
-            const double *bs = a.Bs + (int64_t)e * nq * 3;
-#pragma unroll(NQ > 0 ? NQ : 1)
-            for (int q = 0; q < nq; ++q) {
-                const double s0 = __ldg(bs + 3 * q), s1 = __ldg(bs + 3 * q + 1), s2 = __ldg(bs + 3 * q + 2);
-                const double B0 = s0 + Bc[0], B1 = s1 + Bc[1], B2 = s2 + Bc[2];
-                const double bm = sqrt(B0 * B0 + B1 * B1 + B2 * B2);
-                double dnu;
-                const double nu = nu_at<DIL>(a, s_relc, s_relx, s_phi + 4 * q, Zn, bm, dnu);
-                const double wq = s_w[q];
-                kfac += nu * wq;
-                const double aq = (bm >= 1e-14) ? dnu * wq * idet / bm : 0.0;
-                const double rq = (kNu0 - nu) * wq;
-                double p[6];
-#pragma unroll
-                for (int j = 0; j < 6; ++j) {
-                    p[j] = c[j][0] * B0 + c[j][1] * B1 + c[j][2] * B2;
-                    r[j] += rq * (c[j][0] * s0 + c[j][1] * s1 + c[j][2] * s2);
-                }
-                int t = 0;
-#pragma unroll
-                for (int j = 0; j < 6; ++j) {
-                    const double apj = aq * p[j];
-#pragma unroll
-                    for (int k = j; k < 6; ++k) dk[t++] += apj * p[k];
-                }
-            }
-            kfac *= idet;
-#pragma unroll
-            for (int j = 0; j < 6; ++j) {
-                if (a.rhs) red_add(a.rhs + g[j], r[j]);
-                Fj[j] = -r[j];
+                p[j] = c[j][0] * B0 + c[j][1] * B1 + c[j][2] * B2;
+                r[j] += rq * (c[j][0] * s0 + c[j][1] * s1 + c[j][2] * s2);
             }
             int t = 0;
 #pragma unroll
             for (int j = 0; j < 6; ++j) {
+                const double apj = aq * p[j];
 #pragma unroll
-                for (int k = j; k < 6; ++k) {
-                    const double kv = kfac * (c[j][0] * c[k][0] + c[j][1] * c[k][1] + c[j][2] * c[k][2]);
-                    if (a.ET) store_pair(a, t, eo, kv, dk[t]);
-                    const double dv = dk[t++];
-                    const int s1 = want_mat ? __ldg(sl + j * 6 + k) : 0;
-                    if (a.K) red_add(a.K + s1, kv);
-                    if (a.dK) red_add(a.dK + s1, dv);
-                    if (a.J) red_add(a.J + s1, kv + dv);
-                    if (a.J32) red_add(a.J32 + s1, (float)(kv + dv));
-                    Fj[j] += kv * xv[k];
-                    if (k != j) {
-                        const int s2 = want_mat ? __ldg(sl + k * 6 + j) : 0;
-                        if (a.K) red_add(a.K + s2, kv);
-                        if (a.dK) red_add(a.dK + s2, dv);
-                        if (a.J) red_add(a.J + s2, kv + dv);
-                        if (a.J32) red_add(a.J32 + s2, (float)(kv + dv));
-                        Fj[k] += kv * xv[j];
-                    }
+                for (int k = j; k < 6; ++k) dk[t++] += apj * p[k];
+            }
+        }
+        kfac *= idet;
+#pragma unroll
+        for (int j = 0; j < 6; ++j) Fj[j] = -r[j];
+        int tri = 0;
+#pragma unroll
+        for (int j = 0; j < 6; ++j) {
+#pragma unroll
+            for (int k = j; k < 6; ++k, ++tri) {
+                const double kv = kfac * (c[j][0] * c[k][0] + c[j][1] * c[k][1] + c[j][2] * c[k][2]);
+                emit(tri, j, k, kv, dk[tri]);
+                Fj[j] = __fma_rn(kv, xv[k], Fj[j]);  // the same rounding in every kernel built on this
+                if (k != j) Fj[k] = __fma_rn(kv, xv[j], Fj[k]);
+            }
+        }
+    }
+}
+
+// Shared-memory tables of the element kernels: curls at q = 0 for every orientation, d_phi at
+// q = 0, weights, nodal basis (diluted steel) and PCHIP.
+struct ElemTables {
+    double *ctab, *dphi, *w, *phi, *relc, *relx;
+};
+
+__device__ __forceinline__ ElemTables stage_tables(const CurlArgs &a, int quad_stride_ctab, double *sm) {
+    const SmemLayout L = smem_layout(a.n_orient, a.nq, a.n_int);
+    const ElemTables T{sm + L.off_ctab, sm + L.off_dphi, sm + L.off_w, sm + L.off_phi, sm + L.off_relc, sm + L.off_relx};
+    for (int t = threadIdx.x; t < a.n_orient * 18; t += blockDim.x) {
+        int o = t / 18, r = t - o * 18;
+        T.ctab[t] = a.ctab[(int64_t)o * quad_stride_ctab + r];
+    }
+    for (int t = threadIdx.x; t < 12; t += blockDim.x) T.dphi[t] = a.dphi0[t];
+    for (int t = threadIdx.x; t < a.nq; t += blockDim.x) T.w[t] = a.w[t];
+    if (a.phi)
+        for (int t = threadIdx.x; t < 4 * a.nq; t += blockDim.x) T.phi[t] = a.phi[t];
+    const int nc = a.n_int < 0 ? 1 : 4 * a.n_int;
+    const int nx = a.n_int < 0 ? 1 : a.n_int + 1;
+    for (int t = threadIdx.x; t < nc; t += blockDim.x) T.relc[t] = a.rel_c[t];
+    for (int t = threadIdx.x; t < nx; t += blockDim.x) T.relx[t] = (a.n_int < 0) ? 0.0 : a.rel_x[t];
+    __syncthreads();
+    return T;
+}
+
+template <bool HAS_BS, int NQ, typename VT, bool DIL>
+__global__ void __launch_bounds__(kBlock)
+    k_curlcurl(CurlArgs a, int quad_stride_ctab) {
+    extern __shared__ double sm[];
+    const ElemTables T = stage_tables(a, quad_stride_ctab, sm);
+    const int nq = NQ > 0 ? NQ : a.nq;
+    double wsum = 0.0;
+    for (int q = 0; q < nq; ++q) wsum += T.w[q];
+
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < a.n_elems; e += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t eo = a.t_offset + e;
+        const bool want_mat = (a.K != nullptr) | (a.dK != nullptr) | (a.J != nullptr) | (a.J32 != nullptr);
+        const int32_t *sl = want_mat ? a.slots + 36 * e : nullptr;
+        int g[6];
+        double Fj[6], r[6];
+        curl_element<HAS_BS, NQ, DIL>(a, e, T.ctab, T.dphi, T.w, T.phi, T.relc, T.relx, wsum, g, Fj, r,
+                                      [&](int tri, int j, int k, double kv, double dv) {
+            if (a.ET) store_pair(a, tri, eo, kv, dv);
+            const int s1 = want_mat ? __ldg(sl + j * 6 + k) : 0;
+            if (a.K) red_add(a.K + s1, kv);
+            if (a.dK) red_add(a.dK + s1, dv);
+            if (a.J) red_add(a.J + s1, kv + dv);
+            if (a.J32) red_add(a.J32 + s1, (float)(kv + dv));
+            if (k != j) {
+                const int s2 = want_mat ? __ldg(sl + k * 6 + j) : 0;
+                if (a.K) red_add(a.K + s2, kv);
+                if (a.dK) red_add(a.dK + s2, dv);
+                if (a.J) red_add(a.J + s2, kv + dv);
+                if (a.J32) red_add(a.J32 + s2, (float)(kv + dv));
+            }
+        });
+        if constexpr (HAS_BS) {
+            if (a.rhs) {
+#pragma unroll
+                for (int j = 0; j < 6; ++j) red_add(a.rhs + g[j], r[j]);
+            }
+        }
+        if (a.F) {
+#pragma unroll
+            for (int j = 0; j < 6; ++j) red_add(a.F + g[j], Fj[j]);
+        }
+        if (a.ET) store_vectors(a, eo, Fj, HAS_BS ? r : nullptr);
+    }
+}
+
+// Element values of the two-phase assembly with an element's values side by side (PackedTerms).
+// A CSR row takes up to six values of each of its elements, so phase 2 reads runs of neighbouring
+// doubles here, where blocks of equal-numbered values give it one useful double per 32-byte sector
+// (entry kernel, 1.16M tets: 571 us from the block layout, 2.7 GB through L2).  The values
+// leave through a shared tile so that the stores are whole lines.
+template <bool HAS_BS, int NQ, bool DIL>
+__global__ void __launch_bounds__(kBlock)
+    k_curlcurl_packed(CurlArgs a, int quad_stride_ctab, int table_doubles, PackedTerms out) {
+    extern __shared__ double sm[];
+    const ElemTables T = stage_tables(a, quad_stride_ctab, sm);
+    double *tile = sm + table_doubles;                              // K or J, then F and r
+    double *tile_d = tile + kBlock * kPackPairs;                    // dK
+    const int nq = NQ > 0 ? NQ : a.nq;
+    double wsum = 0.0;
+    for (int q = 0; q < nq; ++q) wsum += T.w[q];
+    double *const first = out.J ? out.J : out.K;
+
+    for (int64_t base = (int64_t)blockIdx.x * kBlock; base < a.n_elems; base += (int64_t)gridDim.x * kBlock) {
+        const int cnt = (int)(a.n_elems - base < kBlock ? a.n_elems - base : kBlock);
+        const int64_t eo = a.t_offset + base;
+        int g[6];
+        double Fj[6], r[6];
+        if ((int)threadIdx.x < cnt)
+            curl_element<HAS_BS, NQ, DIL>(a, base + threadIdx.x, T.ctab, T.dphi, T.w, T.phi, T.relc, T.relx, wsum, g,
+                                          Fj, r, [&](int tri, int, int, double kv, double dv) {
+                if (first) tile[threadIdx.x * kPackPairs + tri] = out.J ? kv + dv : kv;
+                if (out.D) tile_d[threadIdx.x * kPackPairs + tri] = dv;
+            });
+        __syncthreads();
+        if (first)
+            for (int t = threadIdx.x; t < cnt * kPackPairs; t += kBlock) first[eo * kPackPairs + t] = tile[t];
+        if (out.D)
+            for (int t = threadIdx.x; t < cnt * kPackPairs; t += kBlock) out.D[eo * kPackPairs + t] = tile_d[t];
+        __syncthreads();
+        if (out.F || out.R) {
+            double *tile_r = tile + kBlock * 6;
+            if ((int)threadIdx.x < cnt) {
+#pragma unroll
+                for (int j = 0; j < 6; ++j) {
+                    tile[threadIdx.x * 6 + j] = Fj[j];
+                    if constexpr (HAS_BS) tile_r[threadIdx.x * 6 + j] = r[j];
                 }
             }
-            if (a.F) {
-#pragma unroll
-                for (int j = 0; j < 6; ++j) red_add(a.F + g[j], Fj[j]);
+            __syncthreads();
+            if (out.F)
+                for (int t = threadIdx.x; t < cnt * 6; t += kBlock) out.F[eo * 6 + t] = tile[t];
+            if constexpr (HAS_BS) {
+                if (out.R)
+                    for (int t = threadIdx.x; t < cnt * 6; t += kBlock) out.R[eo * 6 + t] = tile_r[t];
             }
-            if (a.ET) store_vectors(a, eo, Fj, r);
+            __syncthreads();
         }
     }
 }
@@ -669,7 +726,41 @@ int launch_t(const CurlArgs &a, cudaStream_t st, size_t smem, int qstride) {
     return SNP_OK;
 }
 
+template <bool HAS_BS, int NQ, bool DIL = false>
+int launch_packed_t(const CurlArgs &a, cudaStream_t st, int qstride, const PackedTerms &out) {
+    if (a.n_elems == 0) return SNP_OK;
+    auto kern = k_curlcurl_packed<HAS_BS, NQ, DIL>;
+    const int tables = smem_layout(a.n_orient, a.nq, a.n_int).total;
+    const size_t smem = sizeof(double) * ((size_t)tables + (out.D ? 2 : 1) * kBlock * kPackPairs);
+    SNP_REQUIRE(smem <= 227 * 1024, "curl-curl assembly: tables need %zu bytes of shared memory", smem);
+    if (smem > 48 * 1024) SNP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<wave_grid(kern, a.n_elems, kBlock, smem), kBlock, smem, st>>>(a, qstride, tables, out);
+    SNP_LAUNCH_CHECK();
+    return SNP_OK;
+}
+
 }  // namespace
+
+int launch_curlcurl_packed(const CurlArgs &a, const PackedTerms &out, cudaStream_t st) {
+    const int qstride = a.nq * 18;
+    if (a.Bs == nullptr) {
+        if (a.nq == 1) return launch_packed_t<false, 1>(a, st, qstride, out);
+        if (a.nq == 4) return launch_packed_t<false, 4>(a, st, qstride, out);
+        return launch_packed_t<false, 0>(a, st, qstride, out);
+    }
+    if (a.phi) {
+        if (a.nq == 4) return launch_packed_t<true, 4, true>(a, st, qstride, out);
+        return launch_packed_t<true, 0, true>(a, st, qstride, out);
+    }
+    if (a.nq == 1) return launch_packed_t<true, 1>(a, st, qstride, out);
+    if (a.nq == 4) return launch_packed_t<true, 4>(a, st, qstride, out);
+    if (a.nq == 5) return launch_packed_t<true, 5>(a, st, qstride, out);
+    return launch_packed_t<true, 0>(a, st, qstride, out);
+}
+
+bool packed_fits(int32_t n_orient, int32_t nq, int32_t n_int) {
+    return sizeof(double) * ((size_t)smem_layout(n_orient, nq, n_int).total + 2 * kBlock * kPackPairs) <= 227 * 1024;
+}
 
 int check_affine_tables(const double *curls, int32_t n_orient, const double *d_phi, int32_t nq, cudaStream_t st,
                         bool *affine) {

@@ -14,6 +14,8 @@
 // from the pattern's sorted coupling list (cid / cptr) and incidence lists (inc / inc_ptr): one
 // thread per CSR entry and one per DoF, no atomics, every output written exactly once.  Each
 // entry is the same sum whatever the launch shape, so the results are bitwise repeatable.
+#include <vector>
+
 #include "snp_common.cuh"
 #include "snp_internal.cuh"
 
@@ -22,12 +24,6 @@ namespace snp {
 namespace {
 
 constexpr int kEntryBlock = 256;
-
-// upper-triangle index of the element pair (a, b): rows j = min, columns k = max, row by row
-__device__ __forceinline__ int tri_index(int a, int b) {
-    const int j = a < b ? a : b, k = a < b ? b : a;
-    return j * 6 - (j * (j - 1)) / 2 + (k - j);
-}
 
 // What the entry kernel writes, from which blocks.
 enum EntryMode {
@@ -46,11 +42,10 @@ struct EntryArgs {
     float *J32;
 };
 
-// value index of coupling id t = e * 36 + a * 6 + b in its block: q * n_elems + e
+// value index of coupling word t = e * 21 + q (the pattern's cid) in the block layout: q * n_elems + e
 __device__ __forceinline__ int64_t coupling_index(uint32_t t, int64_t S) {
-    const int64_t e = (int64_t)(t / 36u);
-    const int ab = (int)(t - (uint32_t)e * 36u);
-    return (int64_t)tri_index(ab / 6, ab % 6) * S + e;
+    const uint32_t e = t / (uint32_t)kPackPairs;
+    return (int64_t)(t - e * (uint32_t)kPackPairs) * S + (int64_t)e;
 }
 
 // Each thread sums kEntU consecutive entries.  The entries' first two contributions are
@@ -138,6 +133,142 @@ __global__ void __launch_bounds__(kEntryBlock)
     }
 }
 
+// ---------------------------------------------------------------- packed element values
+
+// Element ranges whose dK (constant reluctance) or reduced-rhs terms (no source field) are zero:
+// phase 1 does not store them and phase 2 does not read them.
+constexpr int kMaxRanges = 16;
+struct ZeroRanges {
+    int n = 0;
+    int32_t lo[kMaxRanges], hi[kMaxRanges];
+    bool add(int64_t l, int64_t h) {
+        if (n > 0 && hi[n - 1] == l) {
+            hi[n - 1] = (int32_t)h;
+            return true;
+        }
+        if (n == kMaxRanges) return false;
+        lo[n] = (int32_t)l;
+        hi[n] = (int32_t)h;
+        ++n;
+        return true;
+    }
+};
+
+__device__ __forceinline__ bool in_ranges(const ZeroRanges &z, int32_t e) {
+    bool in = false;
+    for (int i = 0; i < z.n; ++i) in |= e >= z.lo[i] && e < z.hi[i];
+    return in;
+}
+
+struct PackedEntryArgs {
+    int64_t nnz;
+    const int32_t *cptr, *cid;
+    const double *m0, *m1;  // K (or J) and dK values
+    double *K, *dK, *J;
+    float *J32;
+    // value indices [lo, hi) whose dK is zero and not stored (up to two ranges)
+    uint32_t lo[2], hi[2];
+};
+
+// One thread per CSR entry: its contributions' values (the pattern's coupling words are the value
+// indices) summed in element order, the first two requested together (an entry has 1.9 on
+// average; a diagonal about five).  Bound by the gathers' sectors and the streams of the outputs and
+// words, about 1.0 GB a call at 1.16M tets; a warp's 32 consecutive entries are two rows, whose
+// elements' values are runs of doubles, so most of each sector is used.  Decoding element and
+// pair from a coupling id and four entries a thread took 1600 instructions per 128 entries
+// (422 us at 1.16M tets); from the block layout the sums took 571 us, this way 205 us.
+template <int MODE>
+__global__ void __launch_bounds__(kEntryBlock) k_cc_entries_packed(PackedEntryArgs r) {
+    auto stored = [&](uint32_t t) {
+        if constexpr (MODE == kEntKD || MODE == kEntD)
+            return !((t >= r.lo[0] && t < r.hi[0]) || (t >= r.lo[1] && t < r.hi[1]));
+        else
+            return true;
+    };
+    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < r.nnz; p += (int64_t)gridDim.x * blockDim.x) {
+        const int c0 = __ldcs(r.cptr + p), c1 = __ldg(r.cptr + p + 1);
+        double s0 = 0.0, s1 = 0.0;
+        if (c1 > c0) {  // every entry of a pattern has a contribution
+            const bool two = c1 > c0 + 1;
+            const uint32_t t0 = (uint32_t)__ldg(r.cid + c0), t1 = two ? (uint32_t)__ldg(r.cid + c0 + 1) : t0;
+            const bool n0 = stored(t0), n1 = stored(t1) && two;
+            double b0 = 0.0, b1 = 0.0, e0 = 0.0, e1 = 0.0;
+            if constexpr (MODE == kEntD) {
+                if (n0) b0 = __ldg(r.m0 + t0);
+                if (n1) b1 = __ldg(r.m0 + t1);
+            } else {
+                b0 = __ldg(r.m0 + t0);
+                if (two) b1 = __ldg(r.m0 + t1);
+                if constexpr (MODE == kEntKD) {
+                    if (n0) e0 = __ldg(r.m1 + t0);
+                    if (n1) e1 = __ldg(r.m1 + t1);
+                }
+            }
+            s0 = two ? b0 + b1 : b0;
+            s1 = two ? e0 + e1 : e0;
+            for (int k = c0 + 2; k < c1; ++k) {
+                const uint32_t t = (uint32_t)__ldg(r.cid + k);
+                if constexpr (MODE == kEntD) {
+                    if (stored(t)) s0 += __ldg(r.m0 + t);
+                } else {
+                    s0 += __ldg(r.m0 + t);
+                    if constexpr (MODE == kEntKD)
+                        if (stored(t)) s1 += __ldg(r.m1 + t);
+                }
+            }
+        }
+        if constexpr (MODE == kEntKD) {
+            if (r.K) __stcs(r.K + p, s0);
+            if (r.dK) __stcs(r.dK + p, s1);
+            if (r.J) __stcs(r.J + p, s0 + s1);
+            if (r.J32) r.J32[p] = (float)(s0 + s1);
+        } else if constexpr (MODE == kEntJ) {
+            if (r.J) __stcs(r.J + p, s0);
+            if (r.J32) r.J32[p] = (float)s0;
+        } else if constexpr (MODE == kEntK) {
+            __stcs(r.K + p, s0);
+        } else {
+            __stcs(r.dK + p, s0);
+        }
+    }
+}
+
+// F_i and rhs_i from the packed six-term values over DoF i's incidences, in element order
+__global__ void __launch_bounds__(kEntryBlock)
+    k_cc_dofvec_packed(int32_t n, const int32_t *__restrict__ inc_ptr, const int32_t *__restrict__ inc,
+                       const double *__restrict__ Fe, const double *__restrict__ Re, double *__restrict__ F,
+                       double *__restrict__ rhs, ZeroRanges no_source) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        double f = 0.0, rr = 0.0;
+        for (int t = __ldg(inc_ptr + i); t < __ldg(inc_ptr + i + 1); ++t) {
+            const uint32_t u = (uint32_t)__ldg(inc + t);
+            const int64_t idx = (int64_t)(u >> 3) * 6 + (int64_t)(u & 7u);
+            if (F) f += __ldg(Fe + idx);
+            if (rhs && !in_ranges(no_source, (int32_t)(u >> 3))) rr += __ldg(Re + idx);
+        }
+        if (F) F[i] = f;
+        if (rhs) rhs[i] = rr;
+    }
+}
+
+template <int MODE>
+int launch_packed_entries(const PackedEntryArgs &r, cudaStream_t st) {
+    auto kern = k_cc_entries_packed<MODE>;
+    kern<<<wave_grid(kern, r.nnz, kEntryBlock), kEntryBlock, 0, st>>>(r);
+    SNP_LAUNCH_CHECK();
+    return SNP_OK;
+}
+
+// Which element matrices an output set needs.
+struct PackedNeeds {
+    bool k, d, j;
+};
+PackedNeeds packed_needs(const SystemOut &o) {
+    const bool wj = o.J != nullptr || o.J32 != nullptr;
+    const bool only_j = o.fused_j && wj && !o.K && !o.dK;
+    return {!only_j && (o.K || wj), !only_j && (o.dK || wj), only_j};
+}
+
 template <int MODE>
 int launch_entries(const EntryArgs &r, cudaStream_t st) {
     auto kern = k_cc_entries<MODE>;
@@ -212,9 +343,139 @@ int launch_curlcurl_rows(const snp_pattern *pat, const double *terms, const Term
     return SNP_OK;
 }
 
+size_t curlcurl_system_work(const snp_pattern *pat, const SystemOut &o) {
+    const PackedNeeds nd = packed_needs(o);
+    return (size_t)pat->n_elems * ((nd.k + nd.d + nd.j) * kPackPairs + (o.F ? 6 : 0) + (o.rhs ? 6 : 0));
+}
+
+int launch_curlcurl_system(const snp_pattern *pat, const CurlArgs *mats, int n_mats, double *work, const SystemOut &o,
+                           cudaStream_t st) {
+    SNP_REQUIRE(rows_supported(pat), "curl-curl system: the pattern has no contribution or incidence lists");
+    SNP_REQUIRE(pat->n_elems == 0 || work != nullptr || curlcurl_system_work(pat, o) == 0,
+                "curl-curl system: work is NULL");
+    const PackedNeeds nd = packed_needs(o);
+    const size_t E = (size_t)pat->n_elems;
+    PackedEntryArgs r{};
+    ZeroRanges no_source, zero_dk;
+    bool packed = true;
+    int64_t at = 0;
+    for (int m = 0; m < n_mats; ++m) {
+        const CurlArgs &a = mats[m];
+        SNP_REQUIRE(a.t_offset == at, "curl-curl system: material %d starts at element %lld, expected %lld", m,
+                    (long long)a.t_offset, (long long)at);
+        at += a.n_elems;
+        packed = packed && packed_fits(a.n_orient, a.nq, a.n_int);
+        if (o.rhs && a.n_elems > 0 && a.Bs == nullptr) packed = packed && no_source.add(a.t_offset, at);
+    }
+    SNP_REQUIRE(at == pat->n_elems, "curl-curl system: the materials hold %lld of the pattern's %lld elements",
+                (long long)at, (long long)pat->n_elems);
+    if (!packed) {
+        const TermLayout L = term_layout((nd.k ? SNP_TERMS_K : 0) | (nd.d ? SNP_TERMS_DK : 0) | (nd.j ? SNP_TERMS_J : 0) |
+                                         (o.F ? SNP_TERMS_F : 0) | (o.rhs ? SNP_TERMS_RHS : 0));
+        for (int m = 0; m < n_mats; ++m) SNP_TRY(launch_curlcurl_terms(mats[m], L, work, pat->n_elems, st));
+        return launch_curlcurl_rows(pat, work, L, o.K, o.dK, o.J, o.J32, o.rhs, o.F, st);
+    }
+    PackedTerms all;
+    double *p = work;
+    auto take = [&](bool want, size_t per) {
+        double *q = want ? p : nullptr;
+        if (want) p += per * E;
+        return q;
+    };
+    all.K = take(nd.k, kPackPairs);
+    all.D = take(nd.d, kPackPairs);
+    all.J = take(nd.j, kPackPairs);
+    all.F = take(o.F != nullptr, 6);
+    all.R = take(o.rhs != nullptr, 6);
+    for (int m = 0; m < n_mats; ++m) {
+        const CurlArgs &a = mats[m];
+        if (a.n_elems == 0) continue;
+        PackedTerms out = all;
+        // constant reluctance: dK = 0 (nu' = 0)
+        if (out.D && a.n_int < 0 && zero_dk.n < 2 && zero_dk.add(a.t_offset, a.t_offset + a.n_elems)) out.D = nullptr;
+        if (a.Bs == nullptr) out.R = nullptr;
+        if (out.K || out.D || out.J || out.F || out.R) SNP_TRY(launch_curlcurl_packed(a, out, st));
+    }
+    r.nnz = pat->nnz;
+    r.cptr = pat->cptr.p;
+    r.cid = pat->cid.p;
+    r.K = o.K;
+    r.dK = o.dK;
+    r.J = o.J;
+    r.J32 = o.J32;
+    for (int i = 0; i < zero_dk.n; ++i) {
+        r.lo[i] = (uint32_t)zero_dk.lo[i] * kPackPairs;
+        r.hi[i] = (uint32_t)zero_dk.hi[i] * kPackPairs;
+    }
+    if (r.nnz > 0) {
+        if (nd.j) {
+            r.m0 = all.J;
+            SNP_TRY(launch_packed_entries<kEntJ>(r, st));
+        } else if (nd.k && nd.d) {
+            r.m0 = all.K;
+            r.m1 = all.D;
+            SNP_TRY(launch_packed_entries<kEntKD>(r, st));
+        } else if (nd.k) {
+            r.m0 = all.K;
+            SNP_TRY(launch_packed_entries<kEntK>(r, st));
+        } else if (nd.d) {
+            r.m0 = all.D;
+            SNP_TRY(launch_packed_entries<kEntD>(r, st));
+        }
+    }
+    if ((o.F || o.rhs) && pat->n_rows > 0) {
+        k_cc_dofvec_packed<<<wave_grid(k_cc_dofvec_packed, pat->n_rows, kEntryBlock), kEntryBlock, 0, st>>>(
+            pat->n_rows, pat->inc_ptr.p, pat->inc.p, all.F, all.R, o.F, o.rhs, no_source);
+        SNP_LAUNCH_CHECK();
+    }
+    return SNP_OK;
+}
+
 }  // namespace snp
 
 extern "C" {
+
+int snp_curlcurl_system_work(const snp_pattern *pat, int32_t want_K, int32_t want_dK, int32_t want_J, int32_t want_rhs,
+                             int32_t want_F, int64_t *n_doubles) {
+    snp::clear_error();
+    SNP_REQUIRE(pat != nullptr && n_doubles != nullptr, "snp_curlcurl_system_work: NULL argument");
+    snp::SystemOut o;
+    double d = 0.0;
+    if (want_K) o.K = &d;
+    if (want_dK) o.dK = &d;
+    if (want_J) o.J = &d;
+    if (want_rhs) o.rhs = &d;
+    if (want_F) o.F = &d;
+    *n_doubles = (int64_t)snp::curlcurl_system_work(pat, o);
+    return SNP_OK;
+}
+
+int snp_curlcurl_system(const snp_pattern *pat, int32_t n_mats, const snp_curlcurl_material *mats, const double *nodes,
+                        const double *curls, int32_t n_orient, const double *d_phi, const double *w, int32_t n_quad,
+                        const double *x, double *work, double *K_vals, double *dK_vals, double *J_vals, double *rhs,
+                        double *F, void *stream) {
+    snp::clear_error();
+    SNP_REQUIRE(pat != nullptr && n_mats >= 0 && (n_mats == 0 || mats), "snp_curlcurl_system: NULL argument");
+    std::vector<snp::CurlArgs> args((size_t)n_mats);
+    for (int m = 0; m < n_mats; ++m) {
+        const snp_curlcurl_material &M = mats[m];
+        SNP_TRY(snp::fill_args(args[m], pat, M.elem_offset, M.n_elems, nodes, M.cells, M.glob_ids, M.orientations,
+                               curls, n_orient, d_phi, w, n_quad, x, M.B_s, M.n_int, M.rel_c, M.rel_x));
+        args[m].slots = nullptr;
+        args[m].t_offset = M.elem_offset;
+        if (M.B_s != nullptr && M.phi != nullptr) {
+            args[m].phi = M.phi;
+            for (int i = 0; i < 4; ++i) args[m].dil[i] = M.dilution[i];
+        }
+    }
+    snp::SystemOut o;
+    o.K = K_vals;
+    o.dK = dK_vals;
+    o.J = J_vals;
+    o.rhs = rhs;
+    o.F = F;
+    return snp::launch_curlcurl_system(pat, args.data(), n_mats, work, o, snp::as_stream(stream));
+}
 
 int snp_curlcurl_terms_stride(int32_t parts, int32_t *stride) {
     snp::clear_error();

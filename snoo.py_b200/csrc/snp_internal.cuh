@@ -195,6 +195,33 @@ int launch_curlcurl_terms(const CurlArgs &a, const TermLayout &L, double *terms,
 int launch_curlcurl_rows(const snp_pattern *pat, const double *terms, const TermLayout &L, double *K, double *dK,
                          double *J, float *J32, double *rhs, double *F, cudaStream_t st);
 
+// Element values side by side (the assembly of whole systems, launch_curlcurl_system): value q of
+// element e at X[e * 21 + q] for the upper triangles of K, dK and J = K + dK, at X[e * 6 + k] for
+// the residual and reduced-rhs terms; null: not wanted.
+constexpr int kPackPairs = 21;
+struct PackedTerms {
+    double *K = nullptr, *D = nullptr, *J = nullptr, *F = nullptr, *R = nullptr;
+};
+int launch_curlcurl_packed(const CurlArgs &a, const PackedTerms &out, cudaStream_t st);
+// Whether the packed element kernel's tables and tiles fit in shared memory.
+bool packed_fits(int32_t n_orient, int32_t nq, int32_t n_int);
+
+// Deterministic two-phase assembly of the materials' elements (together all of pat's, in order):
+// each requested output is overwritten.  J = K + dK per entry, or with fused_j and neither K nor dK
+// wanted the sum of the elements' K + dK.  work holds curlcurl_system_work(pat, o) doubles.
+// Element values are packed (PackedTerms); the block layout (launch_curlcurl_terms and _rows, the
+// same values in the same sums) serves tables too large to share the shared memory with the
+// packed kernel's tiles and meshes with more than 16 separate ranges without a source field.
+struct SystemOut {
+    bool fused_j = false;
+    double *K = nullptr, *dK = nullptr, *J = nullptr;
+    float *J32 = nullptr;
+    double *rhs = nullptr, *F = nullptr;
+};
+size_t curlcurl_system_work(const snp_pattern *pat, const SystemOut &o);
+int launch_curlcurl_system(const snp_pattern *pat, const CurlArgs *mats, int n_mats, double *work, const SystemOut &o,
+                           cudaStream_t st);
+
 // Whether launch_curlcurl_rows can serve the pattern (contribution and incidence lists built).
 bool rows_supported(const snp_pattern *pat);
 
@@ -223,8 +250,9 @@ struct snp_pattern {
     int64_t n_elems = 0;
     int32_t dpe = 0;
     snp::DevBuf<int32_t> row_ptr, col_idx, slots, diag_pos;
-    // contributions of every CSR entry p: the coupling ids t = e * dpe^2 + a * dpe + b of the
-    // element pairs that add into it, in element order, cid[cptr[p] .. cptr[p + 1])
+    // contributions of every CSR entry p: the element pairs (e, a, b) that add into it, in element
+    // order, cid[cptr[p] .. cptr[p + 1]); as words e * 21 + (upper-triangle index of (a, b)) with 6
+    // DoFs per element, e * 16 + a * 4 + b with 4
     snp::DevBuf<int32_t> cid, cptr;
     bool has_contrib = false;
     // incidence lists of the rows (6 DoFs per element, fewer than 2^28 elements): row r's

@@ -477,14 +477,16 @@ struct snp_solver {
     // vector entry summed from its element contributions (bitwise repeatable; each output
     // overwritten once)
     int assemble_rows(const double *x, double *Kv, double *Jv, float *J32v, double *rhsv, double *Fv) {
-        int parts = 0;
-        if (Kv) parts |= SNP_TERMS_K | ((Jv || J32v) ? SNP_TERMS_DK : 0);
-        else if (Jv || J32v) parts |= SNP_TERMS_J;
-        if (Fv) parts |= SNP_TERMS_F;
-        if (rhsv) parts |= SNP_TERMS_RHS;
-        const snp::TermLayout L = snp::term_layout(parts);
-        const size_t need = (size_t)pat->n_elems * (size_t)L.stride;
+        snp::SystemOut o;
+        o.fused_j = true;
+        o.K = Kv;
+        o.J = Jv;
+        o.J32 = J32v;
+        o.rhs = rhsv;
+        o.F = Fv;
+        const size_t need = snp::curlcurl_system_work(pat, o);
         if (terms.n < need) SNP_TRY(terms.alloc(need));
+        std::vector<snp::CurlArgs> args;
         for (auto &m : mats) {
             snp::CurlArgs a{};
             a.n_elems = m->count;
@@ -507,10 +509,10 @@ struct snp_solver {
                 for (int i = 0; i < 4; ++i) a.dil[i] = m->dil[i];
             }
             a.t_offset = m->offset;
-            SNP_TRY(snp::launch_curlcurl_terms(a, L, terms.p, pat->n_elems, stream));
+            args.push_back(a);
             if (m->count) ++launches;
         }
-        SNP_TRY(snp::launch_curlcurl_rows(pat, terms.p, L, Kv, nullptr, Jv, J32v, rhsv, Fv, stream));
+        SNP_TRY(snp::launch_curlcurl_system(pat, args.data(), (int)args.size(), terms.p, o, stream));
         ++launches;
         if (Fv && has_extra) {
             snp::k_sub<<<snp::stride_grid(n, snp::kVB, 4), snp::kVB, 0, stream>>>(n, Fv, rhs_extra.p);

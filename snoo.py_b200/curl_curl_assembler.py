@@ -138,23 +138,23 @@ class CurlCurlAssembler:
             for key, want, size in (("K", K, pat.nnz), ("J", J, pat.nnz), ("dK", dK, pat.nnz),
                                     ("rhs", rhs, self.num_dofs), ("F", F, self.num_dofs)):
                 out[key] = t.empty(max(size, 1), dtype=t.float64, device="cuda") if want else None
-            parts = ((_lib.TERMS_K if (K or J) else 0) | (_lib.TERMS_DK if (dK or J) else 0)
-                     | (_lib.TERMS_F if F else 0) | (_lib.TERMS_RHS if rhs else 0))
-            stride = ctypes.c_int32()
-            _lib.call("snp_curlcurl_terms_stride", parts, ctypes.byref(stride))
-            need = pat.n_elems * stride.value
-            if d.get("terms") is None or d["terms"].numel() < need:
-                d["terms"] = t.empty(max(need, 1), dtype=t.float64, device="cuda")
+            need = ctypes.c_int64()
+            _lib.call("snp_curlcurl_system_work", pat.handle, bool(K), bool(dK), bool(J), bool(rhs), bool(F),
+                      ctypes.byref(need))
+            if d.get("terms") is None or d["terms"].numel() < need.value:
+                d["terms"] = t.empty(max(need.value, 1), dtype=t.float64, device="cuda")
+            mats = (_lib.CurlCurlMaterial * len(d["mats"]))()
             for n, m in enumerate(d["mats"]):
                 n_int, rc, rx = d["rel"][n]
                 coef = self._dilution_coef(n)
-                _lib.call("snp_curlcurl_terms", pat.handle, m["offset"], m["count"], _lib.ptr(d["nodes"]),
-                          _lib.ptr(m["cells"]), _lib.ptr(m["gids"]), _lib.ptr(m["orient"]), _lib.ptr(tb.curls_d),
-                          tb.n_orient, _lib.ptr(tb.phi_d) if coef is not None else None, _lib.ptr(tb.d_phi_d),
-                          _lib.ptr(tb.w_d), tb.nq, _lib.ptr(x_d), _lib.ptr(bs[n]), n_int, _lib.ptr(rc), _lib.ptr(rx),
-                          coef, parts, _lib.ptr(d["terms"]), s)
-            _lib.call("snp_curlcurl_rows", pat.handle, _lib.ptr(d["terms"]), parts, _lib.ptr(out["K"]),
-                      _lib.ptr(out["dK"]), _lib.ptr(out["J"]), None, _lib.ptr(out["rhs"]), _lib.ptr(out["F"]), s)
+                mats[n] = _lib.CurlCurlMaterial(
+                    m["offset"], m["count"], m["cells"].data_ptr(), m["gids"].data_ptr(), m["orient"].data_ptr(),
+                    bs[n].data_ptr() if bs[n] is not None else None, rc.data_ptr(), rx.data_ptr(),
+                    tb.phi_d.data_ptr() if coef is not None else None, coef or (0.0, 0.0, 0.0, 0.0), n_int, 0)
+            _lib.call("snp_curlcurl_system", pat.handle, len(mats), mats, _lib.ptr(d["nodes"]), _lib.ptr(tb.curls_d),
+                      tb.n_orient, _lib.ptr(tb.d_phi_d), _lib.ptr(tb.w_d), tb.nq, _lib.ptr(x_d), _lib.ptr(d["terms"]),
+                      _lib.ptr(out["K"]), _lib.ptr(out["dK"]), _lib.ptr(out["J"]), _lib.ptr(out["rhs"]),
+                      _lib.ptr(out["F"]), s)
             for key, want, size in (("K", K, pat.nnz), ("J", J, pat.nnz), ("dK", dK, pat.nnz),
                                     ("rhs", rhs, self.num_dofs), ("F", F, self.num_dofs)):
                 if want:

@@ -79,19 +79,19 @@ def _curlcurl_K_dK_rhs(pat, num_el, num_dofs, nodes_d, cells_d, gids_d, or_d, cu
     ``atomic``; otherwise the element kernel adding into the CSR (diluted when ``dil`` is set)."""
     if pat.rows_supported and os.environ.get("SNP_ASSEMBLY", "rows") != "atomic":
         t = torch()
-        parts = _lib.TERMS_K | _lib.TERMS_DK | _lib.TERMS_RHS
-        stride = ctypes.c_int32()
-        _lib.call("snp_curlcurl_terms_stride", parts, ctypes.byref(stride))
-        terms = t.empty(max(num_el * stride.value, 1), dtype=t.float64, device="cuda")
+        need = ctypes.c_int64()
+        _lib.call("snp_curlcurl_system_work", pat.handle, 1, 1, 0, 1, 0, ctypes.byref(need))
+        work = t.empty(max(need.value, 1), dtype=t.float64, device="cuda")
         K = t.empty(max(pat.nnz, 1), dtype=t.float64, device="cuda")
         dK = t.empty(max(pat.nnz, 1), dtype=t.float64, device="cuda")
         rhs = t.empty(max(num_dofs, 1), dtype=t.float64, device="cuda")
-        _lib.call("snp_curlcurl_terms", pat.handle, 0, num_el, _lib.ptr(nodes_d), _lib.ptr(cells_d), _lib.ptr(gids_d),
-                  _lib.ptr(or_d), _lib.ptr(curls_d), n_orient, _lib.ptr(phi_d) if dil is not None else None,
-                  _lib.ptr(dphi_d), _lib.ptr(w_d), nq, _lib.ptr(x_d), _lib.ptr(bs_d), n_int, _lib.ptr(rc), _lib.ptr(rx),
-                  dil, parts, _lib.ptr(terms), _lib.stream_ptr())
-        _lib.call("snp_curlcurl_rows", pat.handle, _lib.ptr(terms), parts, _lib.ptr(K), _lib.ptr(dK), None, None,
-                  _lib.ptr(rhs), None, _lib.stream_ptr())
+        mat = _lib.CurlCurlMaterial(
+            0, num_el, cells_d.data_ptr(), gids_d.data_ptr(), or_d.data_ptr(),
+            bs_d.data_ptr() if bs_d is not None else None, rc.data_ptr(), rx.data_ptr(),
+            phi_d.data_ptr() if dil is not None else None, dil or (0.0, 0.0, 0.0, 0.0), n_int, 0)
+        _lib.call("snp_curlcurl_system", pat.handle, 1, ctypes.byref(mat), _lib.ptr(nodes_d), _lib.ptr(curls_d),
+                  n_orient, _lib.ptr(dphi_d), _lib.ptr(w_d), nq, _lib.ptr(x_d), _lib.ptr(work), _lib.ptr(K),
+                  _lib.ptr(dK), None, _lib.ptr(rhs), None, _lib.stream_ptr())
         return K[: pat.nnz], dK[: pat.nnz], rhs
     K = zeros(pat.nnz)
     dK = zeros(pat.nnz)
