@@ -11,7 +11,7 @@
 //                 is stored in the slot that (e, k) holds in the DoF-ordered incidence list
 //   DoF pass      q_i = sum of DoF i's slots (a contiguous range, no gathers), then the CG
 //                 update of the DoF: p = z + beta p, x += alpha p, r -= alpha q,
-//                 z = dinv r, r.z and r.r partial sums
+//                 z = M r, r.z and r.r partial sums
 //
 // Every slot has one writer and every sum runs in a fixed order, so the iteration is
 // deterministic without atomics.  The per-DoF CG state is split so the element pass gathers only {z, p}
@@ -23,6 +23,7 @@
 
 #include <cub/cub.cuh>
 
+#include "snp_async.cuh"
 #include "snp_common.cuh"
 #include "snp_elem.cuh"
 #include "snp_internal.cuh"
@@ -34,10 +35,6 @@ namespace snp {
 namespace {
 
 constexpr int kEBlock = 256;
-#ifndef SNP_PASS1_MIN_BLOCKS
-#define SNP_PASS1_MIN_BLOCKS 4
-#endif
-constexpr int kPass1MinBlocks = SNP_PASS1_MIN_BLOCKS;  // resident blocks per SM the element pass asks for
 
 // ---------------------------------------------------------------- topology build
 
@@ -160,20 +157,124 @@ __global__ void __launch_bounds__(kEBlock)
     }
 }
 
+// reference curls of orientation 0 as a kernel parameter (constant-bank operands where the edge
+// is known at compile time)
+template <typename TT>
+struct Chat {
+    TT c[18];
+};
+
+template <typename TT>
+Chat<TT> chat_of(const ElemTopology &top) {
+    Chat<TT> ch;
+    for (int t = 0; t < 18; ++t) ch.c[t] = (TT)top.chat_h[t];
+    return ch;
+}
+
+// u_e of the element's directions pk (signs applied): edges 0-2 and 3-5 summed apart
+template <typename TT>
+__device__ __forceinline__ void element_u(const TT (&pk)[6], const Chat<TT> &ch, TT &u0, TT &u1, TT &u2) {
+    TT u[2][3];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        u[h][0] = u[h][1] = u[h][2] = TT(0);
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const int k = 3 * h + j;
+            u[h][0] += pk[k] * ch.c[3 * k];
+            u[h][1] += pk[k] * ch.c[3 * k + 1];
+            u[h][2] += pk[k] * ch.c[3 * k + 2];
+        }
+    }
+    u0 = u[0][0] + u[1][0];
+    u1 = u[0][1] + u[1][1];
+    u2 = u[0][2] + u[1][2];
+}
+
+template <typename TT>
+__device__ __forceinline__ void apply_tensor(const TT (&t)[6], TT u0, TT u1, TT u2, TT &v0, TT &v1, TT &v2) {
+    v0 = t[0] * u0 + t[1] * u1 + t[2] * u2;
+    v1 = t[1] * u0 + t[3] * u1 + t[4] * u2;
+    v2 = t[2] * u0 + t[4] * u1 + t[5] * u2;
+}
+
+// Element pass of a CG iteration: p from the DoF states, v_e = S_e u_e, p.J p -> alpha, and the six
+// edge terms into their incidence slots.  One element per thread; its slots and tensor and the
+// next element's DoF words are requested while its DoF states are gathered.
+//
+// In float64 (float32: k_epass1_pair).  Bound by the L1 data pipe (a slot per sector of the
+// scattered stores and gathers, 70-80% busy), at small sizes by the launch and its chain of
+// dependent loads.  Two lanes per element with shuffles were slower at every size: 28.3 against 25.4 us per iteration
+// at 287k tets, 17.0 against 15.7 at 100k, 70.7 against 69.9 at 1.16M.  Storing v_e instead of the
+// terms halves this pass (20 us at 1.16M) and adds as much to the DoF pass, which then gathers.
+template <typename TT>
+__global__ void __launch_bounds__(kEBlock, 3)
+    k_epass1(int64_t ne, const int32_t *__restrict__ edof, const int32_t *__restrict__ pos,
+             const TT *__restrict__ T, const Chat<TT> ch, const DofPair<TT> *__restrict__ G, TT *__restrict__ Y,
+             PcgState *st, double *part) {
+    __shared__ double sh[32];
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    int32_t d[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) d[k] = e < ne ? __ldcs(edof + eslot(e, k)) : 0;
+    if (st->done) return;
+    const TT beta = (TT)st->beta;
+    double dot = 0.0;
+#pragma unroll 1
+    for (; e < ne; e += stride) {
+        DofPair<TT> w[6];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) w[k] = G[(uint32_t)d[k] & ~kSignBit];
+        TT t[6];
+        int32_t ps[6], nd[6] = {0, 0, 0, 0, 0, 0};
+#pragma unroll
+        for (int k = 0; k < 6; ++k) t[k] = __ldcs(T + eslot(e, k));
+#pragma unroll
+        for (int k = 0; k < 6; ++k) ps[k] = __ldcs(pos + eslot(e, k));
+        if (e + stride < ne) {
+#pragma unroll
+            for (int k = 0; k < 6; ++k) nd[k] = __ldcs(edof + eslot(e + stride, k));
+        }
+        TT pk[6], u0, u1, u2, v0, v1, v2;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            pk[k] = pnext(beta, w[k].b, w[k].a);
+            if (d[k] < 0) pk[k] = -pk[k];
+        }
+        element_u(pk, ch, u0, u1, u2);
+        apply_tensor(t, u0, u1, u2, v0, v1, v2);
+        dot += (double)u0 * (double)v0 + (double)u1 * (double)v1 + (double)u2 * (double)v2;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) Y[ps[k]] = edge_term(ch.c, k, d[k] < 0, v0, v1, v2);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) d[k] = nd[k];
+    }
+    dot = block_sum(dot, sh);
+    if (threadIdx.x == 0) part[blockIdx.x] = dot;
+    if (last_block(&st->counter)) {
+        const double pq = reduce_parts(part, gridDim.x, 1, 0, sh);
+        if (threadIdx.x == 0) {
+            st->pq = pq;
+            st->alpha = st->rz / pq;
+        }
+    }
+}
+
 template <typename TT>
 __device__ __forceinline__ void load_chat(TT *sc, const TT *chat) {
     if (threadIdx.x < 18) sc[threadIdx.x] = chat[threadIdx.x];
     __syncthreads();
 }
 
-// element pass of a CG iteration: p from the DoF states, v_e = S_e u_e, p.J p -> alpha, and
-// the six edge terms into their incidence slots.  Two lanes per element, three edges each:
+// The element pass in float32, whose rounding the iterates of a mixed-precision solve follow
+// closely: two lanes per element, three edges each:
 // each lane gathers three DoF states, the halves of u_e meet through one shuffle, and each
 // lane stores its three edge terms (half the registers of one lane per element, so twice
 // the resident warps keep the same number of gathers in flight).
 template <typename TT>
-__global__ void __launch_bounds__(kEBlock, kPass1MinBlocks)
-    k_epass1(int64_t ne, const int32_t *__restrict__ edof, const int32_t *__restrict__ pos,
+__global__ void __launch_bounds__(kEBlock, 4)
+    k_epass1_pair(int64_t ne, const int32_t *__restrict__ edof, const int32_t *__restrict__ pos,
              const TT *__restrict__ T, const TT *__restrict__ chat, const DofPair<TT> *__restrict__ G,
              TT *__restrict__ Y, PcgState *st, double *part) {
     __shared__ TT sc[18];
@@ -279,7 +380,45 @@ __global__ void __launch_bounds__(kEBlock, kPass1MinBlocks)
     }
 }
 
-// DoF pass of a CG iteration: q_i = sum of the DoF's incidence slots, then the update of DoF i
+// beta, the norms and the stopping decision of an iteration
+__device__ __forceinline__ int finish_iteration(PcgState *st, double rz_new, double rr_new) {
+    st->beta = rz_new / st->rz;
+    st->rz = rz_new;
+    st->rr = rr_new;
+    st->iter += 1;
+    int done = 0;
+    if (!(rr_new == rr_new) || isinf(rr_new)) done = 3;
+    else if (sqrt(rr_new) < st->atol_eff) done = 1;
+    else if (st->iter >= st->maxit) done = 2;
+    st->done = done;
+    return done;
+}
+
+// block partials of r.z and r.r, their sum by the last block, and the iteration's decision
+__device__ __forceinline__ void close_dof_pass(double rz, double rr, double (*sh2)[32], double *part, PcgState *st,
+                                               int use_cond, cudaGraphConditionalHandle cond) {
+    block_sum2(rz, rr, sh2);
+    if (threadIdx.x == 0) {
+        part[2 * blockIdx.x] = rz;
+        part[2 * blockIdx.x + 1] = rr;
+    }
+    if (last_block(&st->counter)) {
+        double a = 0.0, b = 0.0;
+        if (threadIdx.x < kEBlock)
+            for (int i = threadIdx.x; i < (int)gridDim.x; i += kEBlock) {
+                a += __ldcg(part + 2 * i);
+                b += __ldcg(part + 2 * i + 1);
+            }
+        __syncthreads();
+        block_sum2(a, b, sh2);
+        if (threadIdx.x == 0) {
+            const int done = finish_iteration(st, a, b);
+            if (use_cond && done) cudaGraphSetConditional(cond, 0);
+        }
+    }
+}
+
+// DoF pass of a CG iteration with point Jacobi
 template <typename TT>
 __global__ void __launch_bounds__(kEBlock)
     k_epass2(int32_t n, const uint8_t *__restrict__ free_mask, const int32_t *__restrict__ inc_ptr,
@@ -308,33 +447,279 @@ __global__ void __launch_bounds__(kEBlock)
         rz += (double)r * (double)z;
         rr += (double)r * (double)r;
     }
-    block_sum2(rz, rr, sh2);
-    if (threadIdx.x == 0) {
-        part[2 * blockIdx.x] = rz;
-        part[2 * blockIdx.x + 1] = rr;
-    }
-    if (last_block(&st->counter)) {
-        double a = 0.0, b = 0.0;
-        for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) {
-            a += __ldcg(part + 2 * i);
-            b += __ldcg(part + 2 * i + 1);
+    close_dof_pass(rz, rr, sh2, part, st, use_cond, cond);
+}
+
+// DoF pass with block Jacobi, every operand straight from memory (smaller systems)
+template <typename TT>
+__global__ void __launch_bounds__(kEBlock)
+    k_epass2_direct(int32_t n, const uint8_t *__restrict__ free_mask, const int32_t *__restrict__ inc_ptr,
+                const TT *__restrict__ Y, const uint16_t *__restrict__ meta, const float *__restrict__ binv,
+                DofPair<TT> *__restrict__ G, DofPair<TT> *__restrict__ R, PcgState *st, double *part, int use_cond,
+                cudaGraphConditionalHandle cond) {
+    __shared__ double sh2[2][32];
+    // float64: r of the tile in two alternating buffers, so a tile needs one barrier: it writes
+    // the buffer its predecessor's predecessor read, which every thread has finished with once
+    // past the barrier in between (77.8 -> 77.0 us per iteration at 1.16M tets; in float32 the
+    // second barrier per tile measured slightly faster, 56.3 against 56.8 us, and stays)
+    constexpr bool kTwoBuffers = sizeof(TT) == 8;
+    __shared__ TT s_r2[2][kBjTile];
+    // each tile's slot range is read one tile ahead (the first one before the CG state), so
+    // that a tile's slot values are requested together with its DoF words
+    // In float32 the tile's DoF states {z, p}, {r, x} are read one tile ahead as well (in float64
+    // their registers would cost a resident block per SM).
+    constexpr bool kStateAhead = sizeof(TT) == 4;
+    const int64_t tstride = (int64_t)gridDim.x * kBjTile;
+    int nb0 = 0, nb1 = 0;
+    DofPair<TT> ng{TT(0), TT(0)}, nrx{TT(0), TT(0)};
+    {
+        const int64_t i0 = (int64_t)blockIdx.x * kBjTile + threadIdx.x;
+        if (i0 < n) {
+            nb0 = __ldcs(inc_ptr + i0);
+            nb1 = __ldcs(inc_ptr + i0 + 1);
+            if constexpr (kStateAhead) {
+                ng = G[i0];
+                nrx = R[i0];
+            }
         }
+    }
+    if (st->done) {
+        if (use_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(cond, 0);
+        return;
+    }
+    const TT alpha = (TT)st->alpha, beta = (TT)st->beta;
+    double rz = 0.0, rr = 0.0;
+    int par = 0;
+    for (int64_t base = (int64_t)blockIdx.x * kBjTile; base < n; base += tstride, par ^= (kTwoBuffers ? 1 : 0)) {
+        TT *s_r = s_r2[par];
+        const int64_t i = base + threadIdx.x;
+        const bool fr = i < n && is_free(free_mask, i);
+        const int b0 = nb0, b1 = nb1;
+        DofPair<TT> g = ng, rx = nrx;
+        if (i + tstride < n) {
+            nb0 = __ldcs(inc_ptr + i + tstride);
+            nb1 = __ldcs(inc_ptr + i + tstride + 1);
+            if constexpr (kStateAhead) {
+                ng = G[i + tstride];
+                nrx = R[i + tstride];
+            }
+        }
+        if constexpr (!kStateAhead) {
+            if (fr) {
+                g = G[i];
+                rx = R[i];
+            }
+        }
+        TT r = TT(0);
+        unsigned mt = 0;
+        float4 ma = make_float4(0.f, 0.f, 0.f, 0.f), mb = ma;
+        if (fr) {
+            // the DoF's words are requested before the slot values and the tile barrier; in
+            // float64 the block row only as an L1 prefetch (its registers would cost a block per SM)
+            mt = meta[i];
+            if constexpr (sizeof(TT) == 4) bj_load(binv, i, ma, mb);
+            else bj_prefetch(binv, i);
+            double q = 0.0;
+            for (int t = b0; t < b1; ++t) q += (double)Y[t];
+            r = rx.a - alpha * (TT)q;
+        }
+        s_r[threadIdx.x] = r;
         __syncthreads();
-        block_sum2(a, b, sh2);
-        if (threadIdx.x == 0) {
-            const double rz_new = a, rr_new = b;
-            st->beta = rz_new / st->rz;
-            st->rz = rz_new;
-            st->rr = rr_new;
-            st->iter += 1;
-            int done = 0;
-            if (!(rr_new == rr_new) || isinf(rr_new)) done = 3;
-            else if (sqrt(rr_new) < st->atol_eff) done = 1;
-            else if (st->iter >= st->maxit) done = 2;
-            st->done = done;
-            if (use_cond && done) cudaGraphSetConditional(cond, 0);
+        if (fr) {
+            if constexpr (sizeof(TT) == 8) bj_load(binv, i, ma, mb);
+            const TT z = bj_row(mt, ma, mb, s_r, threadIdx.x);
+            const TT p = pnext(beta, g.b, g.a);
+            G[i] = DofPair<TT>{z, p};
+            R[i] = DofPair<TT>{r, rx.b + alpha * p};
+            rz += (double)r * (double)z;
+            rr += (double)r * (double)r;
+        }
+        if constexpr (!kTwoBuffers) __syncthreads();
+    }
+    close_dof_pass(rz, rr, sh2, part, st, use_cond, cond);
+}
+
+// ---- DoF pass with block Jacobi, staged
+//
+// A tile's slot values, DoF words and packed block inverses are contiguous runs, which a ninth
+// warp copies into shared memory with bulk copies one to two tiles ahead.  Bound by memory: 126 MB
+// read and 44 MB written at 1.16M tets in float64 (25 MB less than with unpacked block rows), 26 us
+// where loads in each thread's own order took 30 (the slot run of a DoF is 40 bytes from the
+// next lane's, so their L1 slots were the limit).  Its start is longer by the copy engine's
+// latency, so it serves blocks with several tiles.
+constexpr int kDofThreads = kEBlock + 32;
+constexpr int kDofStages = 2;
+constexpr int kIncCap = 1536;  // slots of a tile staged in shared memory (1290 on average)
+constexpr int kPackMax = kBjTile / kBjMax * (kBjMax * (kBjMax + 1) / 2);  // packed entries of a tile, at most
+
+template <typename TT>
+struct __align__(128) DofStage {
+    TT y[kIncCap + 8];
+    float m[kPackMax];
+    uint32_t word[kBjTile];
+};
+
+// first slot of the tile, its slots, how far its staged values start before it (-1: not staged)
+struct TileInfo {
+    int32_t first, total, shift;
+};
+
+// barrier of the eight consumer warps; true on all of them when any thread passes fail
+__device__ __forceinline__ bool consumer_sync_any(bool fail) {
+    uint32_t any;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %1, 0;\n\t"
+        "barrier.cta.red.or.pred q, 1, %2, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(any)
+        : "r"((uint32_t)fail), "n"(kEBlock)
+        : "memory");
+    return any != 0;
+}
+template <typename TT>
+struct DofPassArgs {
+    int32_t n, tiles;
+    const uint32_t *word;
+    const int32_t *tile_inc, *tile_m;
+    const int32_t *inc_ptr;  // only for plans whose words do not hold the starts
+    const float *packed;
+    const TT *Y;
+    DofPair<TT> *G, *R;
+};
+
+template <typename TT>
+__global__ void __launch_bounds__(kDofThreads, 4)
+    k_epass2_bj(const DofPassArgs<TT> a, PcgState *st, double *part, int use_cond, cudaGraphConditionalHandle cond) {
+    extern __shared__ __align__(128) unsigned char dof_smem[];
+    DofStage<TT> *stage = reinterpret_cast<DofStage<TT> *>(dof_smem);
+    __shared__ double sh2[2][32];
+    __shared__ TT s_r2[2][kBjTile];
+    __shared__ uint64_t full[kDofStages], empty[kDofStages];
+    __shared__ TileInfo info[kDofStages];
+    __shared__ volatile int s_fail;
+    const bool producer = threadIdx.x >= kEBlock;
+    if (threadIdx.x == 0) {
+        s_fail = 0;
+        for (int s = 0; s < kDofStages; ++s) {
+            mbar_init(full + s, 1);
+            mbar_init(empty + s, kEBlock / 32);
+        }
+        mbar_init_fence();
+    }
+    __syncthreads();
+    double rz = 0.0, rr = 0.0;
+    if (producer) {
+        if (threadIdx.x == kEBlock) {
+            auto issue = [&](int32_t tile, int s) {
+                DofStage<TT> &D = stage[s];
+                constexpr int kA = 16 / (int)sizeof(TT);  // values per 16 bytes
+                const int32_t i0 = __ldg(a.tile_inc + tile), i1 = __ldg(a.tile_inc + tile + 1);
+                const int32_t m0 = __ldg(a.tile_m + tile), m1 = __ldg(a.tile_m + tile + 1);
+                const int32_t c0 = i0 & ~(kA - 1), cn = (i1 - c0 + kA - 1) & ~(kA - 1);
+                const bool staged = i1 - i0 <= kIncCap;
+                info[s] = TileInfo{i0, i1 - i0, staged ? i0 - c0 : -1};
+                const uint32_t mb = (uint32_t)(m1 - m0) * 4u;
+                const uint32_t yb = staged && i1 > i0 ? (uint32_t)(cn * (int)sizeof(TT)) : 0u;
+                mbar_arrive_expect(full + s, kBjTile * 4u + mb + yb);
+                if (yb) bulk_load(D.y, a.Y + c0, yb, full + s);
+                bulk_load(D.word, a.word + (int64_t)tile * kBjTile, kBjTile * 4u, full + s);
+                if (mb) bulk_load(D.m, a.packed + m0, mb, full + s);
+            };
+            int issued = 0;
+            int32_t tile = blockIdx.x;
+            for (; issued < kDofStages && tile < a.tiles; ++issued, tile += gridDim.x) issue(tile, issued);
+            if (*(volatile int *)&st->done) {
+                // a finished solve: the copies in flight end before the block does
+                for (int s = 0; s < issued; ++s) mbar_wait_bounded(full + s, 0);
+            } else {
+                for (int it = issued; tile < a.tiles; ++it, tile += gridDim.x) {
+                    const int s = it % kDofStages;
+                    if (!mbar_wait_bounded(empty + s, (uint32_t)((it / kDofStages - 1) & 1), &s_fail)) {
+                        s_fail = 1;
+                        for (int q = 0; q < kDofStages; ++q)
+                            mbar_wait_bounded(full + q, (uint32_t)(((it - 1 - (it - 1 - q) % kDofStages) / kDofStages) & 1));
+                        break;
+                    }
+                    issue(tile, s);
+                }
+            }
+        }
+        __syncwarp();
+    } else if (!st->done) {
+        const TT alpha = (TT)st->alpha, beta = (TT)st->beta;
+        const int tid = threadIdx.x;
+        int it = 0;
+        for (int32_t tile = blockIdx.x; tile < a.tiles; tile += gridDim.x, ++it) {
+            const int s = it % kDofStages;
+            const DofStage<TT> &D = stage[s];
+            TT *s_r = s_r2[it & 1];
+            const int64_t i = (int64_t)tile * kBjTile + tid;  // the states are padded to whole tiles
+            const DofPair<TT> g = a.G[i], rx = a.R[i];
+            const bool here = mbar_wait_bounded(full + s, (uint32_t)((it / kDofStages) & 1));
+            const TileInfo ti = info[s];
+            const uint32_t w = D.word[tid];
+            const bool fr = here && ((w >> 6) & 1u);
+            TT r = TT(0);
+            if (fr) {
+                int b0, b1;
+                if (a.inc_ptr == nullptr) {
+                    b0 = (int)(w >> 18);
+                    b1 = tid + 1 < kBjTile ? (int)(D.word[tid + 1] >> 18) : ti.total;
+                } else {
+                    b0 = __ldg(a.inc_ptr + i) - ti.first;
+                    b1 = __ldg(a.inc_ptr + i + 1) - ti.first;
+                }
+                double q = 0.0;
+                if (ti.shift >= 0)
+                    for (int t = b0; t < b1; ++t) q += (double)D.y[ti.shift + t];
+                else
+                    for (int t = b0; t < b1; ++t) q += (double)__ldg(a.Y + ti.first + t);
+                r = rx.a - alpha * (TT)q;
+            }
+            s_r[tid] = r;
+            // r alternates between two buffers: a tile writes the one whose readers of two tiles ago
+            // have passed the barrier in between
+            if (consumer_sync_any(!here)) {
+                s_fail = 1;
+                break;
+            }
+            if (fr) {
+                const int o = (int)(w & 7u), size = (int)((w >> 3) & 7u) + 1;
+                const float *m = D.m + ((w >> 7) & 0x7ffu);
+                const TT *rb = s_r + (tid - o);
+                TT z = TT(0);
+#pragma unroll
+                for (int c = 0; c < kBjMax; ++c)
+                    if (c < size) z = fma((TT)m[c <= o ? o * (o + 1) / 2 + c : c * (c + 1) / 2 + o], rb[c], z);
+                const TT p = pnext(beta, g.b, g.a);
+                a.G[i] = DofPair<TT>{z, p};
+                a.R[i] = DofPair<TT>{r, rx.b + alpha * p};
+                rz += (double)r * (double)z;
+                rr += (double)r * (double)r;
+            }
+            __syncwarp();
+            if ((tid & 31) == 0) mbar_arrive(empty + s);
         }
     }
+    __syncthreads();
+    if (s_fail) {
+        if (threadIdx.x == 0) {
+            st->done = 5;
+            if (use_cond) cudaGraphSetConditional(cond, 0);
+        }
+        return;
+    }
+    if (st->done) {
+        if (use_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(cond, 0);
+        return;
+    }
+    close_dof_pass(rz, rr, sh2, part, st, use_cond, cond);
+}
+
+template <typename TT>
+constexpr size_t dof_pass_smem() {
+    return kDofStages * sizeof(DofStage<TT>);
 }
 
 template <typename TT>
@@ -348,32 +733,25 @@ __global__ void k_eextract(int32_t n, const DofPair<TT> *__restrict__ R, double 
 template <typename TT>
 __global__ void __launch_bounds__(kEBlock)
     k_eapply1(int64_t ne, const int32_t *__restrict__ edof, const int32_t *__restrict__ pos,
-              const TT *__restrict__ T, const TT *__restrict__ chat, const uint8_t *__restrict__ free_mask,
+              const TT *__restrict__ T, const Chat<TT> ch, const uint8_t *__restrict__ free_mask,
               const TT *__restrict__ x, TT *__restrict__ Y) {
-    __shared__ TT sc[18];
-    load_chat(sc, chat);
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < ne; e += (int64_t)gridDim.x * blockDim.x) {
         const int64_t eb = eslot(e, 0);
         int32_t d[6];
-        TT u0 = TT(0), u1 = TT(0), u2 = TT(0);
+        TT pk[6], t[6], u0, u1, u2, v0, v1, v2;
 #pragma unroll
         for (int k = 0; k < 6; ++k) {
             d[k] = edof[eb + 32 * k];
             const uint32_t g = (uint32_t)d[k] & ~kSignBit;
-            TT xk = is_free(free_mask, g) ? x[g] : TT(0);
-            if (d[k] < 0) xk = -xk;
-            u0 += xk * sc[3 * k];
-            u1 += xk * sc[3 * k + 1];
-            u2 += xk * sc[3 * k + 2];
+            pk[k] = is_free(free_mask, g) ? x[g] : TT(0);
+            if (d[k] < 0) pk[k] = -pk[k];
         }
-        TT t[6];
 #pragma unroll
         for (int k = 0; k < 6; ++k) t[k] = T[eb + 32 * k];
-        const TT v0 = t[0] * u0 + t[1] * u1 + t[2] * u2;
-        const TT v1 = t[1] * u0 + t[3] * u1 + t[4] * u2;
-        const TT v2 = t[2] * u0 + t[4] * u1 + t[5] * u2;
+        element_u(pk, ch, u0, u1, u2);
+        apply_tensor(t, u0, u1, u2, v0, v1, v2);
 #pragma unroll
-        for (int k = 0; k < 6; ++k) Y[pos[eb + 32 * k]] = edge_term(sc, k, d[k] < 0, v0, v1, v2);
+        for (int k = 0; k < 6; ++k) Y[pos[eb + 32 * k]] = edge_term(ch.c, k, d[k] < 0, v0, v1, v2);
     }
 }
 
@@ -571,11 +949,14 @@ __global__ void __launch_bounds__(kEBlock)
 // one thread per block: the block's inverse (bj_invert_block)
 __global__ void __launch_bounds__(128)
     k_bj_invert(int32_t n, const uint8_t *__restrict__ free_mask, const uint16_t *__restrict__ meta,
-                const double *__restrict__ bmat, float *__restrict__ binv, int *n_fallback) {
+                const uint32_t *__restrict__ word, const int32_t *__restrict__ tile_m,
+                const double *__restrict__ bmat, float *__restrict__ binv, float *__restrict__ packed,
+                int *n_fallback) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const unsigned mt = meta[i];
         if (mt & 0xffu) continue;
-        bj_invert_block(i, (int)(mt >> 8), is_free(free_mask, i), free_mask, bmat, binv, n_fallback);
+        bj_invert_block(i, (int)(mt >> 8), is_free(free_mask, i), free_mask, bmat, binv, n_fallback,
+                        packed + tile_m[i / kBjTile] + ((word[i] >> 7) & 0x7ffu));
     }
 }
 
@@ -639,124 +1020,57 @@ __global__ void __launch_bounds__(kEBlock)
     }
 }
 
-template <typename TT>
-__global__ void __launch_bounds__(kEBlock)
-    k_epass2_bj(int32_t n, const uint8_t *__restrict__ free_mask, const int32_t *__restrict__ inc_ptr,
-                const TT *__restrict__ Y, const uint16_t *__restrict__ meta, const float *__restrict__ binv,
-                DofPair<TT> *__restrict__ G, DofPair<TT> *__restrict__ R, PcgState *st, double *part, int use_cond,
-                cudaGraphConditionalHandle cond) {
-    __shared__ double sh2[2][32];
-    // float64: r of the tile in two alternating buffers, so a tile needs one barrier: it writes
-    // the buffer its predecessor's predecessor read, which every thread has finished with once
-    // past the barrier in between (77.8 -> 77.0 us per iteration at 1.16M tets; in float32 the
-    // second barrier per tile measured slightly faster, 56.3 against 56.8 us, and stays)
-    constexpr bool kTwoBuffers = sizeof(TT) == 8;
-    __shared__ TT s_r2[2][kBjTile];
-    // each tile's slot range is read one tile ahead (the first one before the CG state), so
-    // that a tile's slot values are requested together with its DoF words
-    // In float32 the tile's DoF states {z, p}, {r, x} are read one tile ahead as well (in float64
-    // their registers would cost a resident block per SM).
-    constexpr bool kStateAhead = sizeof(TT) == 4;
-    const int64_t tstride = (int64_t)gridDim.x * kBjTile;
-    int nb0 = 0, nb1 = 0;
-    DofPair<TT> ng{TT(0), TT(0)}, nrx{TT(0), TT(0)};
-    {
-        const int64_t i0 = (int64_t)blockIdx.x * kBjTile + threadIdx.x;
-        if (i0 < n) {
-            nb0 = __ldcs(inc_ptr + i0);
-            nb1 = __ldcs(inc_ptr + i0 + 1);
-            if constexpr (kStateAhead) {
-                ng = G[i0];
-                nrx = R[i0];
-            }
-        }
+// ---- block plan (once per mesh and block partition)
+
+// packed entries of each tile, rounded up to a multiple of 4; first incidence of each tile
+__global__ void __launch_bounds__(kBjTile)
+    k_plan_tiles(int32_t n, int32_t tiles, const uint16_t *__restrict__ meta, const int32_t *__restrict__ inc_ptr,
+                 int32_t *__restrict__ cnt, int32_t *__restrict__ tile_inc) {
+    const int64_t i = (int64_t)blockIdx.x * kBjTile + threadIdx.x;
+    int sz = 0;
+    if (i < n && (meta[i] & 0xffu) == 0) {
+        const int size = meta[i] >> 8;
+        sz = size * (size + 1) / 2;
     }
-    if (st->done) {
-        if (use_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(cond, 0);
-        return;
-    }
-    const TT alpha = (TT)st->alpha, beta = (TT)st->beta;
-    double rz = 0.0, rr = 0.0;
-    int par = 0;
-    for (int64_t base = (int64_t)blockIdx.x * kBjTile; base < n; base += tstride, par ^= (kTwoBuffers ? 1 : 0)) {
-        TT *s_r = s_r2[par];
-        const int64_t i = base + threadIdx.x;
-        const bool fr = i < n && is_free(free_mask, i);
-        const int b0 = nb0, b1 = nb1;
-        DofPair<TT> g = ng, rx = nrx;
-        if (i + tstride < n) {
-            nb0 = __ldcs(inc_ptr + i + tstride);
-            nb1 = __ldcs(inc_ptr + i + tstride + 1);
-            if constexpr (kStateAhead) {
-                ng = G[i + tstride];
-                nrx = R[i + tstride];
-            }
-        }
-        if constexpr (!kStateAhead) {
-            if (fr) {
-                g = G[i];
-                rx = R[i];
-            }
-        }
-        TT r = TT(0);
-        unsigned mt = 0;
-        float4 ma = make_float4(0.f, 0.f, 0.f, 0.f), mb = ma;
-        if (fr) {
-            // the DoF's words are requested before the slot values and the tile barrier; in
-            // float64 the block row only as an L1 prefetch (its registers would cost a block per SM)
-            mt = meta[i];
-            if constexpr (sizeof(TT) == 4) bj_load(binv, i, ma, mb);
-            else bj_prefetch(binv, i);
-            double q = 0.0;
-            for (int t = b0; t < b1; ++t) q += (double)Y[t];
-            r = rx.a - alpha * (TT)q;
-        }
-        s_r[threadIdx.x] = r;
-        __syncthreads();
-        if (fr) {
-            if constexpr (sizeof(TT) == 8) bj_load(binv, i, ma, mb);
-            const TT z = bj_row(mt, ma, mb, s_r, threadIdx.x);
-            const TT p = pnext(beta, g.b, g.a);
-            G[i] = DofPair<TT>{z, p};
-            R[i] = DofPair<TT>{r, rx.b + alpha * p};
-            rz += (double)r * (double)z;
-            rr += (double)r * (double)r;
-        }
-        if constexpr (!kTwoBuffers) __syncthreads();
-    }
-    block_sum2(rz, rr, sh2);
+    __shared__ double sh[32];
+    const double total = block_sum((double)sz, sh);  // at most 1152: exact
     if (threadIdx.x == 0) {
-        part[2 * blockIdx.x] = rz;
-        part[2 * blockIdx.x + 1] = rr;
-    }
-    if (last_block(&st->counter)) {
-        double a = 0.0, b = 0.0;
-        for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) {
-            a += __ldcg(part + 2 * i);
-            b += __ldcg(part + 2 * i + 1);
-        }
-        __syncthreads();
-        block_sum2(a, b, sh2);
-        if (threadIdx.x == 0) {
-            const double rz_new = a, rr_new = b;
-            st->beta = rz_new / st->rz;
-            st->rz = rz_new;
-            st->rr = rr_new;
-            st->iter += 1;
-            int done = 0;
-            if (!(rr_new == rr_new) || isinf(rr_new)) done = 3;
-            else if (sqrt(rr_new) < st->atol_eff) done = 1;
-            else if (st->iter >= st->maxit) done = 2;
-            st->done = done;
-            if (use_cond && done) cudaGraphSetConditional(cond, 0);
+        cnt[blockIdx.x] = ((int)total + 3) & ~3;
+        tile_inc[blockIdx.x] = inc_ptr[i];
+        if (blockIdx.x == tiles - 1) {
+            cnt[tiles] = 0;
+            tile_inc[tiles] = inc_ptr[n];
         }
     }
+}
+
+__global__ void __launch_bounds__(kBjTile)
+    k_plan_words(int32_t n, const uint16_t *__restrict__ meta, const uint8_t *__restrict__ free_mask,
+                 const int32_t *__restrict__ inc_ptr, uint32_t *__restrict__ word, int *__restrict__ wide) {
+    using Scan = cub::BlockScan<int, kBjTile>;
+    __shared__ typename Scan::TempStorage tmp;
+    __shared__ int s_start[kBjTile];
+    const int64_t base = (int64_t)blockIdx.x * kBjTile, i = base + threadIdx.x;
+    const unsigned mt = i < n ? meta[i] : (1u << 8);
+    const int off = (int)(mt & 0xffu), size = (int)(mt >> 8);
+    const int sz = i < n && off == 0 ? size * (size + 1) / 2 : 0;
+    int start;
+    Scan(tmp).ExclusiveSum(sz, start);
+    s_start[threadIdx.x] = start;
+    __syncthreads();
+    const int64_t end = base + kBjTile < n ? base + kBjTile : n;
+    const int total = inc_ptr[end] - inc_ptr[base];
+    if (threadIdx.x == 0 && total > 16383) atomicExch(wide, 1);
+    const int rel = i < n ? inc_ptr[i] - inc_ptr[base] : total;
+    const uint32_t fr = i < n && is_free(free_mask, i) ? 1u : 0u;
+    word[i] = (uint32_t)off | (uint32_t)(size - 1) << 3 | fr << 6 | (uint32_t)(s_start[threadIdx.x - off] & 0x7ff) << 7 |
+              (uint32_t)(rel & 0x3fff) << 18;
 }
 
 // ---------------------------------------------------------------- one-launch PCG (cooperative)
 //
 // The whole Krylov loop of one Newton step in one cooperative launch (every block resident):
-// per iteration the element pass and the DoF pass of k_epass1 / k_epass2_bj (or k_epass2) run
+// per iteration the element pass and the DoF pass of k_epass1_pair / k_epass2_direct (or k_epass2) run
 // back to back, separated by grid barriers instead of kernel boundaries; every block sums the
 // per-block partials itself, in block order, so all blocks take the same alpha, beta and
 // stopping decision without a serial last-block step.  Block 0 mirrors the state into *st for
@@ -807,7 +1121,7 @@ __device__ __forceinline__ double coop_sum(const double *part, int comp, double 
 }
 
 template <typename TT, bool BJ>
-__global__ void __launch_bounds__(kEBlock, kPass1MinBlocks)
+__global__ void __launch_bounds__(kEBlock, 4)
     k_pcg_coop(int64_t ne, int32_t n, const int32_t *__restrict__ edof, const int32_t *__restrict__ pos,
                const TT *__restrict__ T, const TT *__restrict__ chat, const uint8_t *__restrict__ free_mask,
                const int32_t *__restrict__ inc_ptr, const uint16_t *__restrict__ meta, const float *__restrict__ binv,
@@ -830,7 +1144,7 @@ __global__ void __launch_bounds__(kEBlock, kPass1MinBlocks)
     const int h = lane & 1;
     const int64_t wstride = (int64_t)gridDim.x * (blockDim.x >> 5) * 16;
     for (;;) {
-        // ---- element pass (k_epass1)
+        // ---- element pass (k_epass1_pair)
         const TT tb = (TT)beta;
         double dot = 0.0;
 #pragma unroll 1
@@ -892,7 +1206,7 @@ __global__ void __launch_bounds__(kEBlock, kPass1MinBlocks)
         if (!grid_sync(bar, target, err)) return;
         const double pq = coop_sum(part, 0, sh);
         const double alpha = rz / pq;
-        // ---- DoF pass (k_epass2_bj / k_epass2)
+        // ---- DoF pass (k_epass2_direct / k_epass2)
         const TT ta = (TT)alpha;
         double rz_n = 0.0, rr_n = 0.0;
         if constexpr (BJ) {
@@ -1094,6 +1408,7 @@ int build_elem_topology(ElemTopology &top, int32_t n, const ElemBlock *blocks, i
     double c64[18];
     float c32[18];
     for (int t = 0; t < 18; ++t) {
+        top.chat_h[t] = ctab_host[t];
         c64[t] = ctab_host[t];
         c32[t] = (float)ctab_host[t];
     }
@@ -1108,6 +1423,39 @@ int build_elem_topology(ElemTopology &top, int32_t n, const ElemBlock *blocks, i
     top.n_elems = ne;
     top.n = n;
     *usable = true;
+    return SNP_OK;
+}
+
+int build_block_plan(BlockPlan &plan, const ElemTopology &top, const uint8_t *free_mask, const uint16_t *meta,
+                     cudaStream_t s) {
+    SNP_REQUIRE(top.n > 0 && top.n_elems > 0 && meta != nullptr, "block plan: topology not built");
+    const int32_t n = top.n, tiles = (n + kBjTile - 1) / kBjTile;
+    DevBuf<int32_t> cnt;
+    DevBuf<int> wide;
+    DevBuf<unsigned char> temp;
+    SNP_TRY(cnt.alloc((size_t)tiles + 1));
+    SNP_TRY(wide.alloc(1));
+    SNP_TRY(plan.word.alloc((size_t)tiles * kBjTile));
+    SNP_TRY(plan.tile_inc.alloc((size_t)tiles + 1));
+    SNP_TRY(plan.tile_m.alloc((size_t)tiles + 1));
+    SNP_CUDA_TRY(cudaMemsetAsync(wide.p, 0, sizeof(int), s));
+    k_plan_tiles<<<tiles, kBjTile, 0, s>>>(n, tiles, meta, top.inc_ptr.p, cnt.p, plan.tile_inc.p);
+    SNP_LAUNCH_CHECK();
+    size_t tb = 0;
+    SNP_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb, cnt.p, plan.tile_m.p, tiles + 1, s));
+    SNP_TRY(temp.alloc(tb));
+    SNP_CUDA_TRY(cub::DeviceScan::ExclusiveSum(temp.p, tb, cnt.p, plan.tile_m.p, tiles + 1, s));
+    k_plan_words<<<tiles, kBjTile, 0, s>>>(n, meta, free_mask, top.inc_ptr.p, plan.word.p, wide.p);
+    SNP_LAUNCH_CHECK();
+    int32_t total = 0;
+    int hw = 0;
+    SNP_CUDA_TRY(cudaMemcpyAsync(&total, plan.tile_m.p + tiles, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+    SNP_CUDA_TRY(cudaMemcpyAsync(&hw, wide.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    SNP_CUDA_TRY(cudaStreamSynchronize(s));
+    SNP_TRY(plan.packed.alloc((size_t)total));
+    SNP_CUDA_TRY(cudaMemsetAsync(plan.packed.p, 0, sizeof(float) * (size_t)(total > 0 ? total : 1), s));
+    plan.wide = hw != 0;
+    plan.tiles = tiles;
     return SNP_OK;
 }
 
@@ -1141,10 +1489,14 @@ int ElemPcg<TT>::reserve(int32_t n_, int64_t ne_) {
     drop_graph();
     n = n_;
     ne = ne_;
-    SNP_TRY(G.alloc(n));
-    SNP_TRY(R.alloc(n));
+    const size_t padded = ((size_t)n + kBjTile - 1) / kBjTile * kBjTile;
+    SNP_TRY(G.alloc(padded));
+    SNP_TRY(R.alloc(padded));
+    SNP_CUDA_TRY(cudaMemset(G.p, 0, sizeof(DofPair<TT>) * padded));
+    SNP_CUDA_TRY(cudaMemset(R.p, 0, sizeof(DofPair<TT>) * padded));
     SNP_TRY(D.alloc(n));
-    SNP_TRY(Y.alloc(6 * ne));
+    SNP_TRY(Y.alloc(6 * ne + 8));  // whole 16-byte words of it are copied
+    SNP_CUDA_TRY(cudaMemset(Y.p, 0, sizeof(TT) * (6 * ne + 8)));
     const int gmax = sm_count() * 8 + 1;
     SNP_TRY(part.alloc(3 * (size_t)gmax));
     SNP_TRY(st.alloc(1));
@@ -1156,18 +1508,45 @@ int ElemPcg<TT>::reserve(int32_t n_, int64_t ne_) {
 
 template <typename TT>
 int ElemPcg<TT>::launch_iteration(const ElemTopology &top, const TT *T, const uint8_t *free_mask,
-                                  const uint16_t *bj_meta, const float *bj_inv, cudaStream_t s, int use_cond,
+                                  const BlockPlan *plan, cudaStream_t s, int use_cond,
                                   cudaGraphConditionalHandle cond) {
-    const TT *chat = chat_ptr<TT>(top);
-    k_epass1<TT><<<wave_grid(k_epass1<TT>, 2 * ne, kEBlock), kEBlock, 0, s>>>(ne, top.edof.p, top.pos.p, T, chat, G.p,
-                                                                         Y.p, st.p, part.p);
-    SNP_LAUNCH_CHECK();
-    if (bj_meta)
-        k_epass2_bj<TT><<<wave_grid(k_epass2_bj<TT>, n, kEBlock), kEBlock, 0, s>>>(
-            n, free_mask, top.inc_ptr.p, Y.p, bj_meta, bj_inv, G.p, R.p, st.p, part.p, use_cond, cond);
+    const Chat<TT> ch = chat_of<TT>(top);
+    if constexpr (sizeof(TT) == 4)
+        k_epass1_pair<TT><<<wave_grid(k_epass1_pair<TT>, 2 * ne, kEBlock), kEBlock, 0, s>>>(
+            ne, top.edof.p, top.pos.p, T, chat_ptr<TT>(top), G.p, Y.p, st.p, part.p);
     else
-        k_epass2<TT><<<wave_grid(k_epass2<TT>, n, kEBlock), kEBlock, 0, s>>>(n, free_mask, top.inc_ptr.p, Y.p, G.p,
-                                                                            R.p, D.p, st.p, part.p, use_cond, cond);
+        k_epass1<TT><<<wave_grid(k_epass1<TT>, ne, kEBlock), kEBlock, 0, s>>>(ne, top.edof.p, top.pos.p, T, ch, G.p,
+                                                                            Y.p, st.p, part.p);
+    SNP_LAUNCH_CHECK();
+    const int staged_grid =
+        plan ? wave_grid(k_epass2_bj<TT>, (int64_t)plan->tiles * kDofThreads, kDofThreads, dof_pass_smem<TT>()) : 0;
+    // the staged DoF pass in float64 from four tiles per block on: 39.5 against 40.3 us per iteration
+    // at 600k tets, 69.9 against 74.7 at 1.16M; below, 25.7 against 25.4 at 287k and 16.5 against
+    // 15.7 at 100k (float32: 52.4 against 53.1 at 1.16M, 13.3 against 13.3 at 38k)
+    if (plan && (sizeof(TT) == 4 || plan->tiles < 4 * staged_grid)) {
+        k_epass2_direct<TT><<<wave_grid(k_epass2_direct<TT>, n, kEBlock), kEBlock, 0, s>>>(
+            n, free_mask, top.inc_ptr.p, Y.p, plan->meta, plan->binv, G.p, R.p, st.p, part.p, use_cond, cond);
+        SNP_LAUNCH_CHECK();
+        return SNP_OK;
+    }
+    if (plan) {
+        DofPassArgs<TT> a;
+        a.n = n;
+        a.tiles = plan->tiles;
+        a.word = plan->word.p;
+        a.tile_inc = plan->tile_inc.p;
+        a.tile_m = plan->tile_m.p;
+        a.inc_ptr = plan->wide ? top.inc_ptr.p : nullptr;
+        a.packed = plan->packed.p;
+        a.Y = Y.p;
+        a.G = G.p;
+        a.R = R.p;
+        const size_t smem = dof_pass_smem<TT>();
+        k_epass2_bj<TT><<<staged_grid, kDofThreads, smem, s>>>(a, st.p, part.p, use_cond, cond);
+    } else {
+        k_epass2<TT><<<wave_grid(k_epass2<TT>, n, kEBlock), kEBlock, 0, s>>>(
+            n, free_mask, top.inc_ptr.p, Y.p, G.p, R.p, D.p, st.p, part.p, use_cond, cond);
+    }
     SNP_LAUNCH_CHECK();
     return SNP_OK;
 }
@@ -1175,8 +1554,8 @@ int ElemPcg<TT>::launch_iteration(const ElemTopology &top, const TT *T, const ui
 // L2 residency of the slot values between the element pass (which writes them) and the DoF
 // pass (which reads them): the iteration's kernel nodes get an access policy window over Y with
 // persisting hits, and this context's persisting L2 set-aside is raised to cover it (up to the
-// device's maximum; it lasts as long as the context).  Measured on the 1.16M-tet benchmark: 92.5
-// -> 84.1 us per float64 PCG iteration.  SNP_L2_PERSIST=0 leaves the nodes' cache policy alone.
+// device's maximum; it lasts as long as the context).  SNP_L2_PERSIST=0 leaves the nodes' cache
+// policy alone.
 bool l2_window_on_kernels(cudaGraph_t body, const void *base, size_t bytes) {
     const char *env = getenv("SNP_L2_PERSIST");
     if (env && env[0] == '0') return false;
@@ -1189,7 +1568,7 @@ bool l2_window_on_kernels(cudaGraph_t body, const void *base, size_t bytes) {
         return false;
     }
     // only a window that covers the whole array: a partial one (hit ratio below 1) marks the
-    // rest streaming, which evicts it early and made a 187 MB slot array three times slower
+    // rest streaming, which evicts it early and made a 187 MB array three times slower
     if (bytes > (size_t)max_win || bytes > (size_t)max_persist) return false;
     const size_t win = bytes, keep = bytes;
     if (cudaDeviceSetLimit(cudaLimitPersistingL2CacheSize, keep) != cudaSuccess) {
@@ -1222,8 +1601,7 @@ bool l2_window_on_kernels(cudaGraph_t body, const void *base, size_t bytes) {
 }
 
 template <typename TT>
-int ElemPcg<TT>::build_graph(const ElemTopology &top, const TT *T, const uint8_t *free_mask, const uint16_t *bj_meta,
-                             const float *bj_inv) {
+int ElemPcg<TT>::build_graph(const ElemTopology &top, const TT *T, const uint8_t *free_mask, const BlockPlan *plan) {
     drop_graph();
     l2_window = false;
     const char *env = getenv("SNP_PCG_GRAPH");
@@ -1253,7 +1631,7 @@ int ElemPcg<TT>::build_graph(const ElemTopology &top, const TT *T, const uint8_t
             const int unroll = pcg_body_unroll();
             int rc = SNP_OK;
             for (int u = 0; u < unroll && rc == SNP_OK; ++u)
-                rc = launch_iteration(top, T, free_mask, bj_meta, bj_inv, cs, 1, h);
+                rc = launch_iteration(top, T, free_mask, plan, cs, 1, h);
             cudaGraph_t out = nullptr;
             cudaError_t e = cudaStreamEndCapture(cs, &out);
             ok = (rc == SNP_OK) && e == cudaSuccess;
@@ -1277,16 +1655,17 @@ int ElemPcg<TT>::build_graph(const ElemTopology &top, const TT *T, const uint8_t
     key_top = &top;
     key_T = T;
     key_fm = free_mask;
-    key_bm = bj_meta;
-    key_bi = bj_inv;
+    key_plan = plan;
     return SNP_OK;
 }
 
 // The iteration loop as one cooperative launch (k_pcg_coop); false when the device cannot
 // hold the grid (the caller then uses the graph).  *rc: the launch's status and the barrier's.
 template <typename TT>
-bool ElemPcg<TT>::solve_coop(const ElemTopology &top, const TT *T, const uint8_t *free_mask, const uint16_t *bj_meta,
-                             const float *bj_inv, cudaStream_t s, int *rc) {
+bool ElemPcg<TT>::solve_coop(const ElemTopology &top, const TT *T, const uint8_t *free_mask, const BlockPlan *plan,
+                             cudaStream_t s, int *rc) {
+    const uint16_t *bj_meta = plan ? plan->meta : nullptr;
+    const float *bj_inv = plan ? plan->binv : nullptr;
     *rc = SNP_OK;
     auto kern = bj_meta ? k_pcg_coop<TT, true> : k_pcg_coop<TT, false>;
     int dev = 0, coop = 0, per_sm = 0;
@@ -1338,17 +1717,15 @@ bool ElemPcg<TT>::solve_coop(const ElemTopology &top, const TT *T, const uint8_t
 template <typename TT>
 int ElemPcg<TT>::solve(const ElemTopology &top, const TT *T, const double *diag, const uint8_t *free_mask,
                        const double *b, double b_scale, double *h, double rtol, double atol, int64_t maxit,
-                       cudaStream_t s, int64_t *its, double *res, int *status, const uint16_t *bj_meta,
-                       const float *bj_inv) {
+                       cudaStream_t s, int64_t *its, double *res, int *status, const BlockPlan *plan) {
     bool hold = false;  // this solve raised the L2 set-aside
-    SNP_REQUIRE((bj_meta == nullptr) == (bj_inv == nullptr), "element PCG: block Jacobi needs both meta and inverse");
     SNP_REQUIRE(top.n > 0 && top.n_elems > 0, "element PCG: topology not built");
     SNP_TRY(reserve(top.n, top.n_elems));
     if (maxit < 0) maxit = 10 * (int64_t)n;
     SNP_CUDA_TRY(cudaMemsetAsync(bad.p, 0, sizeof(int), s));
-    if (bj_meta)
+    if (plan)
         k_einit_bj<TT><<<wave_grid(k_einit_bj<TT>, n, kEBlock), kEBlock, 0, s>>>(
-            n, free_mask, b, b_scale, diag, bj_meta, bj_inv, G.p, R.p, st.p, part.p, rtol, atol, (long long)maxit, bad.p);
+            n, free_mask, b, b_scale, diag, plan->meta, plan->binv, G.p, R.p, st.p, part.p, rtol, atol, (long long)maxit, bad.p);
     else
         k_einit<TT><<<wave_grid(k_einit<TT>, n, kEBlock), kEBlock, 0, s>>>(n, free_mask, b, b_scale, diag, G.p, R.p,
                                                                           D.p, st.p, part.p, rtol, atol,
@@ -1366,16 +1743,15 @@ int ElemPcg<TT>::solve(const ElemTopology &top, const TT *T, const double *diag,
     const char *coop_env = getenv("SNP_PCG_COOP");
     if (coop_env && coop_env[0] == '1') {
         int coop_rc = SNP_OK;
-        if (solve_coop(top, T, free_mask, bj_meta, bj_inv, s, &coop_rc)) {
+        if (solve_coop(top, T, free_mask, plan, s, &coop_rc)) {
             SNP_TRY(coop_rc);
             chunk_launches = 1;
             goto extract;
         }
     }
     {
-    const bool same = exec && key_top == &top && key_T == T && key_fm == free_mask && key_bm == bj_meta &&
-                      key_bi == bj_inv;
-    if (!same) SNP_TRY(build_graph(top, T, free_mask, bj_meta, bj_inv));
+    const bool same = exec && key_top == &top && key_T == T && key_fm == free_mask && key_plan == plan;
+    if (!same) SNP_TRY(build_graph(top, T, free_mask, plan));
     }
     hold = exec && l2_window && l2_hold;
     if (exec) {
@@ -1386,7 +1762,7 @@ int ElemPcg<TT>::solve(const ElemTopology &top, const TT *T, const double *diag,
         const int chunk = 32;
         int64_t launched = 0;
         while (true) {
-            for (int k = 0; k < chunk; ++k) SNP_TRY(launch_iteration(top, T, free_mask, bj_meta, bj_inv, s, 0, 0));
+            for (int k = 0; k < chunk; ++k) SNP_TRY(launch_iteration(top, T, free_mask, plan, s, 0, 0));
             launched += chunk;
             SNP_CUDA_TRY(cudaMemcpyAsync(hst.p, st.p, sizeof(PcgState), cudaMemcpyDeviceToHost, s));
             SNP_CUDA_TRY(cudaStreamSynchronize(s));
@@ -1407,6 +1783,10 @@ extract:
         cudaGetLastError();
     }
     const PcgState &H = *hst.p;
+    if (H.done == 5) {
+        SNP_CUDA_TRY(cudaMemset(st.p, 0, sizeof(PcgState)));
+        return fail(SNP_CUDA_ERROR, "element PCG: a wait inside the Krylov loop timed out");
+    }
     launches += 1 + (chunk_launches >= 0 ? chunk_launches : 2 * (H.iter > 0 ? H.iter : 1));
     if (its) *its = H.iter;
     if (res) *res = sqrt(H.rr);
@@ -1422,8 +1802,8 @@ int ElemPcg<TT>::apply(const ElemTopology &top, const TT *T, const uint8_t *free
                        cudaStream_t s) {
     SNP_REQUIRE(top.n > 0 && top.n_elems > 0, "element operator: topology not built");
     SNP_TRY(reserve(top.n, top.n_elems));
-    const TT *chat = chat_ptr<TT>(top);
-    k_eapply1<TT><<<wave_grid(k_eapply1<TT>, ne, kEBlock), kEBlock, 0, s>>>(ne, top.edof.p, top.pos.p, T, chat,
+    const Chat<TT> ch = chat_of<TT>(top);
+    k_eapply1<TT><<<wave_grid(k_eapply1<TT>, ne, kEBlock), kEBlock, 0, s>>>(ne, top.edof.p, top.pos.p, T, ch,
                                                                            free_mask, x, Y.p);
     SNP_LAUNCH_CHECK();
     k_eapply2<TT><<<wave_grid(k_eapply2<TT>, n, kEBlock), kEBlock, 0, s>>>(n, free_mask, top.inc_ptr.p, Y.p, y);
@@ -1475,20 +1855,23 @@ int elem_reduced_system(const ElemTopology &top, const TT *T, const uint8_t *fre
 
 template <typename TT>
 int block_jacobi_build(const ElemTopology &top, const TT *T, const uint8_t *free_mask, const uint16_t *meta,
-                       double *bmat, float *binv, int *fallback_count, cudaStream_t s) {
-    SNP_REQUIRE(top.n > 0 && top.n_elems > 0, "block Jacobi: topology not built");
+                       const BlockPlan &plan, double *bmat, float *binv, int *fallback_count, cudaStream_t s) {
+    SNP_REQUIRE(top.n > 0 && top.n_elems > 0 && plan.tiles > 0, "block Jacobi: topology or plan not built");
     SNP_REQUIRE(meta && bmat && binv && fallback_count, "block Jacobi: NULL buffer");
     k_bj_entries<TT><<<wave_grid(k_bj_entries<TT>, top.n, kEBlock), kEBlock, 0, s>>>(
         top.n, free_mask, top.inc_ptr.p, top.inc.p, top.edof.p, T, chat_ptr<TT>(top), meta, bmat);
     SNP_LAUNCH_CHECK();
-    k_bj_invert<<<stride_grid(top.n, 128, 8), 128, 0, s>>>(top.n, free_mask, meta, bmat, binv, fallback_count);
+    k_bj_invert<<<stride_grid(top.n, 128, 8), 128, 0, s>>>(top.n, free_mask, meta, plan.word.p, plan.tile_m.p, bmat,
+                                                          binv, plan.packed.p, fallback_count);
     SNP_LAUNCH_CHECK();
     return SNP_OK;
 }
 
 template int block_jacobi_build<double>(const ElemTopology &, const double *, const uint8_t *, const uint16_t *,
+                                        const BlockPlan &,
                                         double *, float *, int *, cudaStream_t);
 template int block_jacobi_build<float>(const ElemTopology &, const float *, const uint8_t *, const uint16_t *,
+                                        const BlockPlan &,
                                        double *, float *, int *, cudaStream_t);
 
 int block_jacobi_apply(int32_t n, const uint8_t *free_mask, const uint16_t *meta, const float *binv, const double *r,

@@ -99,10 +99,10 @@ __device__ __forceinline__ void bj_entries_row(int64_t i, const int32_t *__restr
 // every loop unrolls with fixed indices (registers, no local arrays); the lower triangle of the
 // inverse is written to both sides (symmetric by construction), rounded to float32.  Point
 // Jacobi (and one count in *n_fallback) for a block whose pivot is not positive enough; fr:
-// the block's first DoF is free.
+// the block's first DoF is free.  packed: the lower triangle row by row as well, or NULL.
 __device__ __forceinline__ void bj_invert_block(int64_t i, int size, bool fr, const uint8_t *__restrict__ free_mask,
                                                 const double *__restrict__ bmat, float *__restrict__ binv,
-                                                int *n_fallback) {
+                                                int *n_fallback, float *__restrict__ packed = nullptr) {
     double L[kBjMax][kBjMax], d0[kBjMax], rl[kBjMax];
 #pragma unroll
     for (int r = 0; r < kBjMax; ++r) {
@@ -159,6 +159,7 @@ __device__ __forceinline__ void bj_invert_block(int64_t i, int size, bool fr, co
                     const float v = (float)x[r];
                     binv[(i + r) * kBjMax + c] = v;
                     binv[(i + c) * kBjMax + r] = v;
+                    if (packed) packed[r * (r + 1) / 2 + c] = v;
                 }
             }
         }
@@ -174,8 +175,11 @@ __device__ __forceinline__ void bj_invert_block(int64_t i, int size, bool fr, co
             if (r >= size) continue;
             const bool f = is_free(free_mask, i + r);
 #pragma unroll
-            for (int c = 0; c < kBjMax; ++c)
-                binv[(i + r) * kBjMax + c] = (c == r && f && d0[r] > 0.0) ? (float)(1.0 / d0[r]) : 0.0f;
+            for (int c = 0; c < kBjMax; ++c) {
+                const float v = (c == r && f && d0[r] > 0.0) ? (float)(1.0 / d0[r]) : 0.0f;
+                binv[(i + r) * kBjMax + c] = v;
+                if (packed && c <= r) packed[r * (r + 1) / 2 + c] = v;
+            }
         }
     }
 }

@@ -42,7 +42,7 @@ struct CsrView {
 struct PcgState {
     double rz, pq, alpha, beta, rr, bnorm, atol_eff;
     long long iter, maxit;
-    int done;  // 0 running, 1 converged, 2 maxiter, 3 non-finite, 4 zero rhs
+    int done;  // 0 running, 1 converged, 2 maxiter, 3 non-finite, 4 zero rhs, 5 a bounded wait ran out
     unsigned int counter;
 };
 
@@ -125,7 +125,25 @@ struct ElemTopology {
     DevBuf<int32_t> pos;      // eslot(e, k): slot of (e, k) in that DoF-ordered list
     DevBuf<double> chat64;    // [18] reference curls of orientation 0
     DevBuf<float> chat32;
+    double chat_h[18];        // the same on the host (kernel parameters)
 };
+
+// What the block-Jacobi DoF pass reads per 256-DoF tile besides the CG state, laid out so that a
+// tile's share of every array is one contiguous copy.
+struct BlockPlan {
+    // per DoF (padded to whole tiles): bits 0-2 offset in the block, 3-5 block size - 1, 6 free,
+    // 7-17 first packed entry of the block within the tile, 18-31 first incidence within the tile
+    DevBuf<uint32_t> word;
+    DevBuf<int32_t> tile_inc;  // [tiles + 1] first incidence of each tile
+    DevBuf<int32_t> tile_m;    // [tiles + 1] first packed entry of each tile, a multiple of 4
+    DevBuf<float> packed;      // block inverses, lower triangles row by row
+    const uint16_t *meta = nullptr;  // the partition and the unpacked rows (block_jacobi_build's binv)
+    const float *binv = nullptr;
+    bool wide = false;         // a tile has more incidences than 14 bits count: starts from inc_ptr
+    int32_t tiles = 0;
+};
+int build_block_plan(BlockPlan &plan, const ElemTopology &top, const uint8_t *free_mask, const uint16_t *meta,
+                     cudaStream_t s);
 
 // One material's elements: gids [count][6], orientation index [count], placed at `offset`.
 struct ElemBlock {
@@ -163,7 +181,7 @@ int elem_reduced_system(const ElemTopology &top, const TT *T, const uint8_t *fre
 constexpr int kBlockJacobiMax = 8;
 template <typename TT>
 int block_jacobi_build(const ElemTopology &top, const TT *T, const uint8_t *free_mask, const uint16_t *meta,
-                       double *bmat, float *binv, int *fallback_count, cudaStream_t s);
+                       const BlockPlan &plan, double *bmat, float *binv, int *fallback_count, cudaStream_t s);
 // z = M r on the free DoFs (0 elsewhere), float64 vectors.
 int block_jacobi_apply(int32_t n, const uint8_t *free_mask, const uint16_t *meta, const float *binv, const double *r,
                        double *z, cudaStream_t s);
@@ -210,10 +228,10 @@ template <typename TT>
 struct ElemPcg {
     int32_t n = 0;
     int64_t ne = 0;
-    DevBuf<DofPair<TT>> G;  // {z, p}
-    DevBuf<DofPair<TT>> R;  // {r, x}
+    DevBuf<DofPair<TT>> G;  // {z, p}, padded to whole 256-DoF tiles
+    DevBuf<DofPair<TT>> R;  // {r, x}, likewise
     DevBuf<TT> D;           // 1 / diag(J)
-    DevBuf<TT> Y;           // [6 n_elems] element-edge terms in DoF-ordered slots
+    DevBuf<TT> Y;           // [6 n_elems] element-edge terms in DoF-ordered slots, padded by 8
     DevBuf<double> part;
     DevBuf<PcgState> st;
     HostBuf<PcgState> hst;
@@ -223,8 +241,7 @@ struct ElemPcg {
     const void *key_top = nullptr;
     const TT *key_T = nullptr;
     const uint8_t *key_fm = nullptr;
-    const uint16_t *key_bm = nullptr;
-    const float *key_bi = nullptr;
+    const BlockPlan *key_plan = nullptr;
     bool l2_window = false;  // the graph's kernels carry the L2 window over Y
     size_t l2_bytes = 0;     // its size, the set-aside raised while a solve runs
     // raise and release the context's persisting-L2 set-aside around each solve (a device-wide
@@ -239,22 +256,21 @@ struct ElemPcg {
     int reserve(int32_t n, int64_t ne);
     void drop_graph();
     // Solve J h = b_scale * b on the free DoFs from h = 0 with Jacobi from diag, or block
-    // Jacobi when bj_meta / bj_inv are given (block_jacobi_build); h (float64) gets the
+    // Jacobi when a plan is given (block_jacobi_build); h (float64) gets the
     // iterate, 0 on constrained DoFs.  SNP_ZERO_PIVOT for a zero/non-finite diagonal entry on
     // a free DoF.
     int solve(const ElemTopology &top, const TT *T, const double *diag, const uint8_t *free_mask, const double *b,
               double b_scale, double *h, double rtol, double atol, int64_t maxit, cudaStream_t s, int64_t *its,
-              double *res, int *status, const uint16_t *bj_meta = nullptr, const float *bj_inv = nullptr);
+              double *res, int *status, const BlockPlan *plan = nullptr);
     // y = J x on the free rows and columns (0 on constrained rows).
     int apply(const ElemTopology &top, const TT *T, const uint8_t *free_mask, const TT *x, TT *y, cudaStream_t s);
 
    private:
-    int launch_iteration(const ElemTopology &top, const TT *T, const uint8_t *free_mask, const uint16_t *bj_meta,
-                         const float *bj_inv, cudaStream_t s, int use_cond, cudaGraphConditionalHandle cond);
-    int build_graph(const ElemTopology &top, const TT *T, const uint8_t *free_mask, const uint16_t *bj_meta,
-                    const float *bj_inv);
-    bool solve_coop(const ElemTopology &top, const TT *T, const uint8_t *free_mask, const uint16_t *bj_meta,
-                    const float *bj_inv, cudaStream_t s, int *rc);
+    int launch_iteration(const ElemTopology &top, const TT *T, const uint8_t *free_mask, const BlockPlan *plan,
+                         cudaStream_t s, int use_cond, cudaGraphConditionalHandle cond);
+    int build_graph(const ElemTopology &top, const TT *T, const uint8_t *free_mask, const BlockPlan *plan);
+    bool solve_coop(const ElemTopology &top, const TT *T, const uint8_t *free_mask, const BlockPlan *plan,
+                    cudaStream_t s, int *rc);
     DevBuf<unsigned long long> coop_bar;
     DevBuf<int> coop_err;
 };

@@ -249,6 +249,7 @@ struct snp_solver {
     snp::DevBuf<double> bj_mat;
     snp::DevBuf<float> bj_inv;
     snp::DevBuf<int> bj_fallback;
+    snp::BlockPlan bj_plan;
 
     // z = M r with the block Jacobi of the current element tensors (test and inspection entry)
     int precond_apply(bool f32, const double *r, double *z, int32_t *fallback_blocks) {
@@ -266,11 +267,11 @@ struct snp_solver {
 
     int build_block_jacobi(bool f32) {
         if (f32)
-            SNP_TRY(snp::block_jacobi_build(etop, T32.p, free_mask.p, bj_meta.p, bj_mat.p, bj_inv.p, bj_fallback.p,
-                                            stream));
+            SNP_TRY(snp::block_jacobi_build(etop, T32.p, free_mask.p, bj_meta.p, bj_plan, bj_mat.p, bj_inv.p,
+                                            bj_fallback.p, stream));
         else
-            SNP_TRY(snp::block_jacobi_build(etop, T64.p, free_mask.p, bj_meta.p, bj_mat.p, bj_inv.p, bj_fallback.p,
-                                            stream));
+            SNP_TRY(snp::block_jacobi_build(etop, T64.p, free_mask.p, bj_meta.p, bj_plan, bj_mat.p, bj_inv.p,
+                                            bj_fallback.p, stream));
         launches += 2;
         return SNP_OK;
     }
@@ -677,6 +678,7 @@ struct snp_solver {
                 SNP_CUDA_TRY(cudaEventRecord(ev[0], stream));
                 if (layout == SNP_LAYOUT_ELEM) {
                     if (bj_on) SNP_TRY(build_block_jacobi(f32));
+                    const snp::BlockPlan *plan = bj_on ? &bj_plan : nullptr;
                     const uint16_t *bm = bj_on ? bj_meta.p : nullptr;
                     const float *bi = bj_on ? bj_inv.p : nullptr;
                     int rc;
@@ -698,9 +700,9 @@ struct snp_solver {
                         launches += gmres.launches;
                     } else {
                         rc = f32 ? epcg32.solve(etop, T32.p, Jdiag.p, free_mask.p, F.p, -1.0, h.p, eta, 0.0, cg_maxit,
-                                                stream, &its, &rn, &st, bm, bi)
+                                                stream, &its, &rn, &st, plan)
                                  : epcg64.solve(etop, T64.p, Jdiag.p, free_mask.p, F.p, -1.0, h.p, eta, 0.0, cg_maxit,
-                                                stream, &its, &rn, &st, bm, bi);
+                                                stream, &its, &rn, &st, plan);
                     }
                     if (rc == SNP_ZERO_PIVOT)
                         return snp::fail(SNP_ZERO_PIVOT, "Newton step %d: zero Jacobian diagonal on a free DoF", it);
@@ -1122,6 +1124,12 @@ int snp_solver_set_block_jacobi(snp_solver *s, const uint16_t *meta) {
     SNP_TRY(s->bj_fallback.alloc(1));
     SNP_CUDA_TRY(cudaMemcpy(s->bj_meta.p, meta, sizeof(uint16_t) * n, cudaMemcpyHostToDevice));
     SNP_CUDA_TRY(cudaMemset(s->bj_fallback.p, 0, sizeof(int)));
+    // the Krylov graphs hold the previous partition's arrays
+    s->epcg64.drop_graph();
+    s->epcg32.drop_graph();
+    SNP_TRY(snp::build_block_plan(s->bj_plan, s->etop, s->free_mask.p, s->bj_meta.p, s->stream));
+    s->bj_plan.meta = s->bj_meta.p;
+    s->bj_plan.binv = s->bj_inv.p;
     s->bj_on = true;
     return SNP_OK;
 }

@@ -140,3 +140,55 @@ def test_biot_savart_shapes(oracle_mod, n_tar, n_src):
     ref = oracle_mod.compute_B_line_segs_cpp(src, tar, 250.0, rad)
     scale = 250.0 * 1e-7 * 2.0 / rad * max(1.0, np.sqrt(n_src))  # field at the surface of a core
     assert np.isfinite(ref).all() and np.abs(got - ref).max() < 1e-12 * scale
+
+
+def _window_solver(tets, **kw):
+    msh = M.window_frame_mesh(tets, jitter=0.15, seed=11)
+    s = S.RedMVPSolver(msh, msh.geometry.coils(), [M.TAG_IRON], [M.TAG_AIR], [MAT.atan_reluctance()],
+                       max_newton_iterations=60, quad_order=2, **kw)
+    s.verbose = False
+    return s
+
+
+@pytest.mark.parametrize("tets", [900, 700000])
+def test_krylov_passes_apply_the_jacobian(tets):
+    """Each form of the float64 CG passes (direct and staged DoF pass) in one Newton step from zero:
+    the step h it takes satisfies J h = -F to the CG tolerance it was given, with J applied by
+    the product kernels."""
+    import torch
+
+    precision = "fp64"
+
+    s = _window_solver(tets)
+    eng = s.newton_engine()
+    x0 = torch.zeros(eng.n, dtype=torch.float64, device="cuda")
+    F = eng.assemble_tensors(x0, precision, torch.empty_like(x0))
+    free = eng.free_mask.bool()
+    h, _ = eng.solve(None, tol=1e-8, max_newton=1, cg_rtol=1e-3, raise_on_failure=False, line_search=False)
+    eng.assemble_tensors(x0, precision, torch.empty_like(x0))
+    Jh = eng.jacobian_apply(h, torch.zeros_like(h), precision)
+    rel = float(torch.linalg.vector_norm((Jh + F)[free]) / torch.linalg.vector_norm(F[free]))
+    assert rel <= 1.0001e-3  # the recursive residual met 1e-3; the true one differs by rounding
+
+
+@pytest.mark.parametrize("size", [1, 3, 8])
+def test_staged_dof_pass_blocks_and_padding(size):
+    """The staged DoF pass with blocks of 1, 3 and 8 DoFs (packed rows of 1 to 36 entries, tiles
+    ended by shorter blocks, a last tile with padding) against the direct pass, which smaller
+    systems take: the same preconditioner, so the same solve to rounding."""
+    import torch
+
+    s = _window_solver(620000)
+    eng = s.newton_engine()
+    assert (eng.n + 255) // 256 >= 4 * 4 * torch.cuda.get_device_properties(0).multi_processor_count
+    free = eng.free_mask.cpu().numpy().astype(bool)
+    keys = np.arange(eng.n) // size
+    from snoopy_b200.newton import dof_blocks
+
+    eng.set_preconditioner("block", meta=dof_blocks(keys, free))
+    x, st = eng.solve(None, tol=1e-8, max_newton=1, cg_rtol=1e-2, raise_on_failure=False, line_search=False)
+    F = eng.assemble_tensors(torch.zeros_like(x), "fp64", torch.empty_like(x))
+    Jh = eng.jacobian_apply(x, torch.zeros_like(x))
+    fm = eng.free_mask.bool()
+    rel = float(torch.linalg.vector_norm((Jh + F)[fm]) / torch.linalg.vector_norm(F[fm]))
+    assert rel <= 1.0001e-2 and st["cg_iterations"] > 10
