@@ -679,6 +679,20 @@ int snp_pcg(int32_t n_rows, const int32_t *row_ptr, const int32_t *col_idx, cons
     SNP_REQUIRE(row_ptr && col_idx && vals && b && x, "snp_pcg: NULL argument");
     SNP_REQUIRE(rtol >= 0 && atol >= 0, "snp_pcg: tolerances must be non-negative");
     cudaStream_t s = snp::as_stream(stream);
+    if (n_rows <= snp::kPcgSmallMaxN) {
+        snp::DevBuf<unsigned char> scratch;
+        SNP_TRY(scratch.alloc(snp::pcg_small_scratch(n_rows)));
+        bool ran = false;
+        int st = SNP_OK;
+        SNP_TRY(snp::pcg_small(n_rows, row_ptr, col_idx, vals, free_mask, b, x, rtol, atol, maxiter, scratch.p, s, &ran,
+                               iterations, res_norm, &st));
+        if (ran) {
+            if (st == SNP_ZERO_PIVOT) return snp::fail(st, "snp_pcg: zero or missing diagonal entry on a free row");
+            if (st == SNP_NOT_CONVERGED) return snp::fail(st, "snp_pcg: maxiter reached");
+            if (st == SNP_NAN_DETECTED) return snp::fail(st, "snp_pcg: non-finite residual");
+            return SNP_OK;
+        }
+    }
     // diagonal positions (rows are sorted; found by a search kernel)
     snp::DevBuf<int32_t> diag;
     SNP_TRY(diag.alloc(n_rows));

@@ -38,6 +38,8 @@ constexpr size_t kOffDiag = kOffDinv + kVecBytes;
 constexpr size_t kOffPart = kOffDiag + align256(sizeof(int32_t) * kMaxRows);
 constexpr size_t kOffState = kOffPart + align256(sizeof(double) * 3 * kMaxBlocks);
 constexpr size_t kOffBad = kOffState + align256(sizeof(PcgState));
+static_assert(kOffDinv - kOffR >= 1024 + sizeof(int32_t) * (2 * (size_t)kPcgSmallRows + kMaxRows),
+              "the small-system path works in the vectors' part of the scratch array");
 constexpr size_t kScratchBytes = kOffBad + 256;
 
 static __device__ __align__(256) unsigned char g_pcg_scratch[kScratchBytes];
@@ -82,6 +84,18 @@ extern "C" int snp_pcg_noalloc(int32_t n_rows, const int32_t *row_ptr, const int
     B.st = reinterpret_cast<snp::PcgState *>(base + snp::kOffState);
     B.bad = reinterpret_cast<int *>(base + snp::kOffBad);
     B.max_blocks = snp::kMaxBlocks;
+    {
+        bool ran = false;
+        int st = SNP_OK;
+        SNP_TRY(snp::pcg_small(n_rows, row_ptr, col_idx, vals, free_mask, b, x, rtol, atol, maxiter,
+                               base + snp::kOffR, s, &ran, iterations, res_norm, &st));
+        if (ran) {
+            if (st == SNP_ZERO_PIVOT) return snp::fail(st, "pcg: zero or missing diagonal entry on a free row");
+            if (st == SNP_NOT_CONVERGED) return snp::fail(st, "snp_pcg_noalloc: maxiter reached");
+            if (st == SNP_NAN_DETECTED) return snp::fail(st, "snp_pcg_noalloc: non-finite residual");
+            return SNP_OK;
+        }
+    }
     int32_t nnz = 0;
     SNP_CUDA_TRY(cudaMemcpyAsync(&nnz, row_ptr + n_rows, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
     SNP_CUDA_TRY(cudaStreamSynchronize(s));

@@ -2,6 +2,8 @@
 smallest problems, every branch of a dispatch.  Each against the CPU oracle or a plain float64
 evaluation of the same formula."""
 
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -192,3 +194,86 @@ def test_staged_dof_pass_blocks_and_padding(size):
     fm = eng.free_mask.bool()
     rel = float(torch.linalg.vector_norm((Jh + F)[fm]) / torch.linalg.vector_norm(F[fm]))
     assert rel <= 1.0001e-2 and st["cg_iterations"] > 10
+
+
+def _masked_system(n, nf, seed, row_len=12):
+    """A symmetric matrix with A_ii = 1 + sum_j |A_ij| (so ||A^-1|| <= 1) on n rows, nf of them free."""
+    import scipy.sparse as sp
+
+    rng = np.random.default_rng(seed)
+    i = np.repeat(np.arange(n), row_len // 2)
+    j = np.clip(i + rng.integers(1, max(2, min(n, 400)), len(i)), 0, n - 1)
+    keep = i < j
+    off = sp.coo_matrix((rng.uniform(-1.0, 1.0, int(keep.sum())), (i[keep], j[keep])), shape=(n, n)).tocsr()
+    off = off + off.T
+    A = (off + sp.diags(1.0 + np.asarray(abs(off).sum(axis=1)).ravel())).tocsr()
+    A.sort_indices()
+    free = np.zeros(n, bool)
+    free[rng.permutation(n)[:nf]] = True
+    return A, free, rng
+
+
+def _pcg(A, free, b, x0, pad=0, rtol=1e-12, atol=0.0, maxiter=-1):
+    """(rc, x, iterations) of snp_pcg; `pad` constrained rows of one entry are appended."""
+    from snoopy_b200 import _lib
+    from snoopy_b200.device import to_host, upload
+
+    n = A.shape[0] + pad
+    rp = np.concatenate([A.indptr, A.nnz + np.arange(1, pad + 1)])
+    ci = np.concatenate([A.indices, np.arange(A.shape[0], n)])
+    if free is None and pad:
+        free = np.ones(A.shape[0], bool)
+    fm = None if free is None else upload(np.concatenate([free, np.zeros(pad, bool)]).astype(np.uint8), np.uint8)
+    x = upload(np.concatenate([x0, np.zeros(pad)]), np.float64)
+    args = [upload(rp, np.int32), upload(ci, np.int32), upload(np.concatenate([A.data, np.ones(pad)]), np.float64), fm,
+            upload(np.concatenate([b, np.zeros(pad)]), np.float64), x]
+    its, res = ctypes.c_int64(-1), ctypes.c_double(-1.0)
+    rc = _lib.load().snp_pcg(n, *[_lib.ptr(a) for a in args], rtol, atol, maxiter, ctypes.byref(its),
+                             ctypes.byref(res), _lib.stream_ptr())
+    return rc, to_host(x)[:A.shape[0]], its.value
+
+
+@pytest.mark.parametrize("n,nf,row_len", [(1, 1, 2), (40, 7, 8), (40, 8, 8), (1000, 9, 12), (5000, 1023, 12),
+                                          (5000, 1025, 40), (70001, 4100, 12), (9000, 8192, 12), (9000, 8193, 12),
+                                          (8192, 8192, 4), (8192, 8192, 12), (8192, 8192, 60), (262144, 300, 4)])
+def test_small_pcg_matches_the_general_path(n, nf, row_len):
+    """Few free rows: the cluster solve against the same system padded to more rows than it takes.
+
+    ||x - A^-1 b|| <= ||A^-1|| ||r|| <= 1e-12 ||b|| for either, ten times that for the drift of the
+    recursive residual; the counts may differ where ||r|| meets the tolerance within its rounding."""
+    A, free, rng = _masked_system(n, nf, 7 + nf, row_len)
+    b = rng.normal(size=n)
+    x0 = rng.normal(size=n)
+    x0[~free] = np.nan  # never read
+    b[~free] = np.nan
+    mask = None if nf == n else free
+    for maxiter in (-1, 0, 3):
+        rc, x, its = _pcg(A, mask, b, x0, maxiter=maxiter)
+        rc_g, x_g, its_g = _pcg(A, mask, b, x0, 262145 - n, maxiter=maxiter)
+        assert rc == rc_g and abs(its - its_g) <= (1 if maxiter < 0 else 0)
+        assert not x[~free].any()
+        assert np.linalg.norm((x - x_g)[free]) <= 2e-11 * np.linalg.norm(b[free])
+    x = _pcg(A, mask, b, x0)[1][free]
+    assert np.linalg.norm(A[free][:, free] @ x - b[free]) <= 1e-11 * np.linalg.norm(b[free])
+
+
+def test_small_pcg_status_codes_match_the_general_path():
+    A, free, rng = _masked_system(3000, 600, 3)
+    b, x0 = rng.normal(size=3000), rng.normal(size=3000)
+    row = int(np.flatnonzero(free)[77])
+    cases = {"zero rhs": (A, np.zeros(3000), x0), "exact start": (A, A @ (x0 * free), x0)}
+    for name, value in (("zero pivot", 0.0), ("nan pivot", np.nan)):
+        Z = A.copy()
+        Z.data[(Z.indices == row) & (np.repeat(np.arange(3000), np.diff(Z.indptr)) == row)] = value
+        cases[name] = (Z, b, x0)
+    Z = cases["zero pivot"][0].copy()
+    Z.eliminate_zeros()
+    cases["no diagonal entry"] = (Z, b, x0)
+    nan_b = b.copy()
+    nan_b[row] = np.nan
+    cases["nan rhs"] = (A, nan_b, x0)
+    for name, (mat, rhs, start) in cases.items():
+        rc, x, its = _pcg(mat, free, rhs, start)
+        rc_g, x_g, its_g = _pcg(mat, free, rhs, start, 262145 - 3000)
+        assert (rc, its) == (rc_g, its_g), name
+        np.testing.assert_allclose(x, x_g, rtol=0, atol=1e-11 * np.linalg.norm(b), err_msg=name)
