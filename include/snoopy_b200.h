@@ -207,6 +207,21 @@ int snp_gradgrad_assemble(const snp_pattern *pat, int64_t elem_offset, int64_t n
                           const double *ctrl, double H_min, double mu_H_min,
                           double *K_vals, double *dK_vals, double *J_vals, void *stream);
 
+/* All materials of a nodal system in one call: the materials' elements are the pattern's first
+ * ones, in order (elements behind them contribute nothing).  Requested outputs are overwritten:
+ * K, dK, and J = dK + sum over the materials of J_weight K_material (the weights must be 1 when all
+ * three are asked for).  Bitwise repeatable unless SNP_ASSEMBLY=atomic. */
+typedef struct {
+    int64_t n_elems;
+    const int32_t *cells;           /* [n_elems][4], 16-byte aligned */
+    const double *knots, *ctrl;     /* perm_type 1: B-spline in log10 |H| (n_ctrl + degree + 1, n_ctrl) */
+    double H_min, mu_H_min, J_weight;
+    int32_t perm_type, degree, n_ctrl, reserved;
+} snp_gradgrad_material;
+int snp_gradgrad_system(const snp_pattern *pat, int32_t n_mats, const snp_gradgrad_material *mats /* host */,
+                        const double *nodes, const double *d_phi, const double *w, int32_t n_quad, const double *x,
+                        double *K_vals, double *dK_vals, double *J_vals, void *stream);
+
 /* ------------------------------------------------------------------ fields
  * B at quadrature points.  Replaces fem_c.compute_B_Hcurl (fem_c/interface_c.pyx:555-696)
  * -> compute_B_Hcurl (fem_c/ctools.c:1500-1563).  points[E][Q][3], B[E][Q][3]. */

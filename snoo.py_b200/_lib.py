@@ -68,6 +68,15 @@ class CurlCurlMaterial(ctypes.Structure):
                 ("dilution", ctypes.c_double * 4), ("n_int", ctypes.c_int32), ("reserved", ctypes.c_int32)]
 
 
+class GradGradMaterial(ctypes.Structure):
+    """``snp_gradgrad_material``: one material of ``snp_gradgrad_system``."""
+
+    _fields_ = [("n_elems", ctypes.c_int64), ("cells", ctypes.c_void_p), ("knots", ctypes.c_void_p),
+                ("ctrl", ctypes.c_void_p), ("H_min", ctypes.c_double), ("mu_H_min", ctypes.c_double),
+                ("J_weight", ctypes.c_double), ("perm_type", ctypes.c_int32), ("degree", ctypes.c_int32),
+                ("n_ctrl", ctypes.c_int32), ("reserved", ctypes.c_int32)]
+
+
 # name -> argtypes (every function returns int32 status unless listed in _RESTYPES)
 _SIGS = {
     "snp_last_error": [],
@@ -95,6 +104,7 @@ _SIGS = {
     "snp_solver_set_krylov": [_vp, _c_i32, _c_i32],
     "snp_curlcurl_rhs_red": [_c_i64, _vp, _vp, _vp, _vp, _vp, _c_i32, _vp, _vp, _c_i32, _vp, _vp, _c_i32, _vp, _vp,
                              _vp, _vp],
+    "snp_gradgrad_system": [_vp, _c_i32, _vp, _vp, _vp, _vp, _c_i32, _vp, _vp, _vp, _vp, _vp],
     "snp_gradgrad_assemble": [_vp, _c_i64, _c_i64, _vp, _vp, _vp, _vp, _c_i32, _vp, _c_i32, _c_i32, _c_i32, _vp, _vp,
                               _c_f64, _c_f64, _vp, _vp, _vp, _vp],
     "snp_b_hcurl": [_c_i64, _vp, _vp, _vp, _vp, _vp, _c_i32, _vp, _vp, _c_i32, _vp, _vp, _vp, _vp],

@@ -94,13 +94,14 @@ __global__ void k_max_row(int32_t n, const int32_t *__restrict__ rp, int *__rest
     atomicMax(mx, m);
 }
 
-// coupling ids e * 36 + a * 6 + b -> value indices e * 21 + (upper-triangle index of (a, b), rows
-// min(a, b) one after another)
+// coupling ids e * D * D + a * D + b -> value indices e * P + (upper-triangle index of (a, b), rows
+// min(a, b) one after another), P = D (D + 1) / 2
+template <uint32_t D>
 __global__ void k_pair_words(int64_t n, const uint32_t *__restrict__ ids, int32_t *__restrict__ cid) {
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
-        const uint32_t id = ids[t], e = id / 36u, ab = id - e * 36u, a = ab / 6u, b = ab - a * 6u;
+        const uint32_t id = ids[t], e = id / (D * D), ab = id - e * (D * D), a = ab / D, b = ab - a * D;
         const uint32_t j = a < b ? a : b, k = a < b ? b : a;
-        cid[t] = (int32_t)(e * (uint32_t)kPackPairs + j * 6u - (j * (j - 1u)) / 2u + (k - j));
+        cid[t] = (int32_t)(e * (D * (D + 1) / 2) + j * D - (j * (j - 1u)) / 2u + (k - j));
     }
 }
 
@@ -233,7 +234,9 @@ int pattern_create(const int32_t *elem_dofs, int64_t n_elems, int32_t dpe, int32
         if (n < ((int64_t)1 << 31)) {
             if ((rc = P->cid.alloc(n)) || (rc = P->cptr.alloc(P->nnz + 1))) return cleanup_fail(rc);
             if (dpe == 6)
-                k_pair_words<<<stride_grid(n, 256, 16), 256, 0, st>>>(n, dv.Current(), P->cid.p);
+                k_pair_words<6><<<stride_grid(n, 256, 16), 256, 0, st>>>(n, dv.Current(), P->cid.p);
+            else if (dpe == 4)
+                k_pair_words<4><<<stride_grid(n, 256, 16), 256, 0, st>>>(n, dv.Current(), P->cid.p);
             else if (cudaMemcpyAsync(P->cid.p, dv.Current(), sizeof(int32_t) * n, cudaMemcpyDeviceToDevice, st) !=
                      cudaSuccess)
                 return cleanup_fail(fail(SNP_CUDA_ERROR, "snp_pattern_create: copy of the sorted couplings failed"));

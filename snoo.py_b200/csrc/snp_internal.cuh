@@ -199,6 +199,7 @@ int launch_curlcurl_rows(const snp_pattern *pat, const double *terms, const Term
 // element e at X[e * 21 + q] for the upper triangles of K, dK and J = K + dK, at X[e * 6 + k] for
 // the residual and reduced-rhs terms; null: not wanted.
 constexpr int kPackPairs = 21;
+constexpr int kPackPairs4 = 10;  // of an element with 4 DoFs
 struct PackedTerms {
     double *K = nullptr, *D = nullptr, *J = nullptr, *F = nullptr, *R = nullptr;
 };

@@ -132,8 +132,9 @@ def reluctance_tables(reluctance):
     return n_int, c, x
 
 
-def permeability_tables(permeability):
-    """(type, degree, n_ctrl, knots, ctrl, H_min, mu_H_min) as ``fem_c/interface_c.pyx:56-68``."""
+def permeability_spec(permeability):
+    """(type, degree, n_ctrl, knots, ctrl, H_min, mu_H_min) as ``fem_c/interface_c.pyx:56-68``, the
+    tables as given."""
     spl_t, spl_c, spl_k, H_min, mu_H_min, n = np.zeros((1,)), np.zeros((1,)), 1, 0.0, 4 * np.pi * 1e-7, 0
     ts = permeability.get_type_spec()
     if ts == 0:
@@ -143,8 +144,13 @@ def permeability_tables(permeability):
         n = len(spl_t) - spl_k - 1
     else:
         print("Type specifyer of permeability not found!")
-    return (int(ts) if ts in (0, 1) else 0, int(spl_k), int(n), upload(spl_t, np.float64), upload(spl_c, np.float64),
-            float(H_min), float(mu_H_min))
+    return int(ts) if ts in (0, 1) else 0, int(spl_k), int(n), spl_t, spl_c, float(H_min), float(mu_H_min)
+
+
+def permeability_tables(permeability):
+    """``permeability_spec`` with the tables on the device."""
+    ts, k, n, t, c, H_min, mu_H_min = permeability_spec(permeability)
+    return ts, k, n, upload(t, np.float64), upload(c, np.float64), H_min, mu_H_min
 
 
 def check_affine(curls, d_phi, n_quad):

@@ -3,14 +3,14 @@ duplicated as ``snoopy/grad_grad_assembler.py``), plus the sparse row/column hel
 ``matrix_assembly.py:16-90``.
 
 Nodal P1 assembly of div(mu grad phi) and its Newton Jacobian through the sm_100a kernel
-``snp_gradgrad_assemble``; one CSR pattern over all domains is built once and cached.
+``snp_gradgrad_system``; one CSR pattern over all domains is built once and cached.
 """
 
 import numpy as np
 
 from . import _lib
 from . import finite_element as fe
-from .device import Pattern, permeability_tables, upload, zeros
+from .device import Pattern, permeability_spec, torch, upload
 
 
 def recover_full_solution(u, u_g, b):
@@ -80,22 +80,42 @@ class GradGradAssembler:
     def pattern(self):
         return self._device_state()["pattern"]
 
-    def assemble_device(self, x, mu_list, quad_order=8, K=True, dK=False, J=True):
-        """Assemble into the cached pattern; returns CUDA tensors (those requested) and ``pattern``."""
+    def _assemble(self, x, mu_list, quad_order, K, dK, J, running):
+        """K, dK, J (device, or None) of the domains that ``mu_list`` covers.  ``running``: J adds
+        the sum of K so far after every domain, else K once."""
         d = self._device_state()
         nq, w_d, dphi_d = self._tabs(quad_order)
-        pat = d["pattern"]
+        pat, offs, cells = d["pattern"], d["offsets"], d["cells"]
         x_d = x if hasattr(x, "data_ptr") else upload(x, np.float64)
-        out = {"pattern": pat, "K": zeros(pat.nnz) if K else None, "dK": zeros(pat.nnz) if dK else None,
-               "J": zeros(pat.nnz) if J else None}
-        for n, perm in enumerate(mu_list):
-            typ, k, nc, t, c, hmin, muh = permeability_tables(perm)
-            off, cnt = int(d["offsets"][n]), int(d["offsets"][n + 1] - d["offsets"][n])
-            _lib.call("snp_gradgrad_assemble", pat.handle, off, cnt, _lib.ptr(d["nodes"]),
-                      _lib.ptr(d["cells"][4 * off:]) if cnt else _lib.ptr(d["cells"]), _lib.ptr(dphi_d), _lib.ptr(w_d),
-                      nq, _lib.ptr(x_d), typ, k, nc, _lib.ptr(t), _lib.ptr(c), hmin, muh, _lib.ptr(out["K"]),
-                      _lib.ptr(out["dK"]), _lib.ptr(out["J"]), _lib.stream_ptr())
-        return out
+        t = torch()
+        K, dK, J = (t.empty(max(pat.nnz, 1), dtype=t.float64, device=cells.device) if want else None
+                    for want in (K, dK, J))
+        specs = [permeability_spec(perm) for perm in mu_list]
+        # all splines' knots and control points in one upload
+        parts, where, n = [], [], 0
+        for typ, k, nc, knots, ctrl, _, _ in specs:
+            if typ == 1:
+                parts += [np.asarray(knots, dtype=np.float64).reshape(-1), np.asarray(ctrl, dtype=np.float64).reshape(-1)]
+                where.append((n, n + len(parts[-2])))
+                n += len(parts[-2]) + len(parts[-1])
+            else:
+                where.append(None)
+        tab = upload(np.concatenate(parts), np.float64) if parts else None
+        mats = (_lib.GradGradMaterial * max(len(specs), 1))()
+        for i, (typ, k, nc, _, _, hmin, muh) in enumerate(specs):
+            at = where[i]
+            mats[i] = _lib.GradGradMaterial(
+                int(offs[i + 1] - offs[i]), cells.data_ptr() + 16 * int(offs[i]),
+                tab.data_ptr() + 8 * at[0] if at else None, tab.data_ptr() + 8 * at[1] if at else None, hmin, muh,
+                float(len(specs) - i) if running else 1.0, typ, k, nc, 0)
+        _lib.call("snp_gradgrad_system", pat.handle, len(specs), mats, _lib.ptr(d["nodes"]), _lib.ptr(dphi_d),
+                  _lib.ptr(w_d), nq, _lib.ptr(x_d), _lib.ptr(K), _lib.ptr(dK), _lib.ptr(J), _lib.stream_ptr())
+        return pat, K, dK, J
+
+    def assemble_device(self, x, mu_list, quad_order=8, K=True, dK=False, J=True):
+        """Assemble into the cached pattern; returns CUDA tensors (those requested) and ``pattern``."""
+        pat, K, dK, J = self._assemble(x, mu_list, quad_order, K, dK, J, running=False)
+        return {"pattern": pat, "K": K, "dK": dK, "J": J}
 
     def compute_stiffness_and_jacobi_matrix_c(self, x, mu_list, quad_order=8, device=False):
         """``(K, J)`` (``matrix_assembly.py:1059-1135``), scipy CSR without exact zeros; with
@@ -105,22 +125,7 @@ class GradGradAssembler:
         material loop), so J = dK + sum_n (K of materials 0..n).  This is kept as is: with one
         domain, the Laplace subdomain case, it is K + dK.
         """
-        d = self._device_state()
-        nq, w_d, dphi_d = self._tabs(quad_order)
-        pat = d["pattern"]
-        x_d = x if hasattr(x, "data_ptr") else upload(x, np.float64)
-        K = zeros(pat.nnz)
-        dK = zeros(pat.nnz)
-        Ksum = zeros(pat.nnz)
-        for n, perm in enumerate(mu_list):
-            typ, k, nc, t, c, hmin, muh = permeability_tables(perm)
-            off, cnt = int(d["offsets"][n]), int(d["offsets"][n + 1] - d["offsets"][n])
-            _lib.call("snp_gradgrad_assemble", pat.handle, off, cnt, _lib.ptr(d["nodes"]),
-                      _lib.ptr(d["cells"][4 * off:]) if cnt else _lib.ptr(d["cells"]), _lib.ptr(dphi_d), _lib.ptr(w_d),
-                      nq, _lib.ptr(x_d), typ, k, nc, _lib.ptr(t), _lib.ptr(c), hmin, muh, _lib.ptr(K), _lib.ptr(dK),
-                      None, _lib.stream_ptr())
-            Ksum += K
-        J = dK + Ksum
+        pat, K, _, J = self._assemble(x, mu_list, quad_order, True, False, True, running=True)
         if device:
             return pat.to_torch(K), pat.to_torch(J)
         return pat.to_scipy(K, drop_zeros=True), pat.to_scipy(J, drop_zeros=True)

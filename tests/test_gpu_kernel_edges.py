@@ -277,3 +277,60 @@ def test_small_pcg_status_codes_match_the_general_path():
         rc_g, x_g, its_g = _pcg(mat, free, rhs, start, 262145 - 3000)
         assert (rc, its) == (rc_g, its_g), name
         np.testing.assert_allclose(x, x_g, rtol=0, atol=1e-11 * np.linalg.norm(b), err_msg=name)
+
+
+@pytest.mark.parametrize("wanted", ["K", "dK", "J", "K,dK", "K,J", "dK,J", "K,dK,J"])
+@pytest.mark.parametrize("sizes", [[1], [128, 129], [127, 0, 1, 300], [40] * 17 + [1000]])
+def test_gradgrad_system_matches_material_by_material(sizes, wanted):
+    """One launch over all materials (17 and more take two) against the accumulating call per
+    material, by atomics: sums of the same values in another order."""
+    from snoopy_b200 import _lib
+    from snoopy_b200.device import Pattern, permeability_tables, upload, zeros
+
+    msh = M.window_frame_mesh(4000, jitter=0.1, seed=4)
+    n = sum(sizes)
+    cells = upload(msh.cells[: n + 50], np.int32)  # 50 elements of no material
+    pat = Pattern(cells, n + 50, 4, msh.num_nodes)
+    w, q = FE.quadrature_rule(2)
+    tabs = [upload(a, np.float64) for a in (msh.nodes, FE.evaluate_basis_derivative(q), w)]
+    x = upload(np.random.default_rng(1).normal(0, 30.0, msh.num_nodes), np.float64)
+    spline = permeability_tables(MAT.atan_permeability())
+    flat = permeability_tables(S.ConstantPermeability(3e-6))
+    mats = (_lib.GradGradMaterial * len(sizes))()
+    ref = {k: zeros(pat.nnz) for k in ("K", "dK", "J")}
+    weights = [1.0 if wanted == "K,dK,J" else float(len(sizes) - i) for i in range(len(sizes))]
+    off = 0
+    for i, cnt in enumerate(sizes):
+        typ, k, nc, t, c, hmin, muh = spline if i % 2 == 0 else flat
+        cp = cells.data_ptr() + 16 * off
+        mats[i] = _lib.GradGradMaterial(cnt, cp, t.data_ptr(), c.data_ptr(), hmin, muh, weights[i], typ, k, nc, 0)
+        part = {k: zeros(pat.nnz) for k in ("K", "dK")}
+        with pytest.MonkeyPatch.context() as mp:
+            mp.setenv("SNP_ASSEMBLY", "atomic")
+            _lib.call("snp_gradgrad_assemble", pat.handle, off, cnt, _lib.ptr(tabs[0]), ctypes.c_void_p(cp),
+                      _lib.ptr(tabs[1]), _lib.ptr(tabs[2]), len(w), _lib.ptr(x), typ, k, nc, _lib.ptr(t), _lib.ptr(c),
+                      hmin, muh, _lib.ptr(part["K"]), _lib.ptr(part["dK"]), None, _lib.stream_ptr())
+        ref["K"] += part["K"]
+        ref["dK"] += part["dK"]
+        ref["J"] += part["dK"] + weights[i] * part["K"]
+        off += cnt
+    for mode in ("rows", "atomic"):
+        out = {k: zeros(pat.nnz).fill_(7.0) if k in wanted.split(",") else None for k in ("K", "dK", "J")}
+        with pytest.MonkeyPatch.context() as mp:
+            mp.setenv("SNP_ASSEMBLY", mode)
+            _lib.call("snp_gradgrad_system", pat.handle, len(sizes), mats, _lib.ptr(tabs[0]), _lib.ptr(tabs[1]),
+                      _lib.ptr(tabs[2]), len(w), _lib.ptr(x), _lib.ptr(out["K"]), _lib.ptr(out["dK"]),
+                      _lib.ptr(out["J"]), _lib.stream_ptr())
+        for k, v in out.items():
+            if v is not None:
+                # a row's entries are sums of up to 30 values no larger than its diagonal's
+                _assert_rows_close(v, ref[k], pat.row_ptr, 1e-12)
+    # entry by entry the accumulating call (rows) is the system call's sum
+    if sizes == [1] and wanted == "K,dK":
+        acc = {k: zeros(pat.nnz) for k in ("K", "dK")}
+        typ, k, nc, t, c, hmin, muh = spline
+        _lib.call("snp_gradgrad_assemble", pat.handle, 0, 1, _lib.ptr(tabs[0]), _lib.ptr(cells), _lib.ptr(tabs[1]),
+                  _lib.ptr(tabs[2]), len(w), _lib.ptr(x), typ, k, nc, _lib.ptr(t), _lib.ptr(c), hmin, muh,
+                  _lib.ptr(acc["K"]), _lib.ptr(acc["dK"]), None, _lib.stream_ptr())
+        _assert_rows_close(acc["K"], ref["K"], pat.row_ptr, 1e-12)
+        _assert_rows_close(acc["dK"], ref["dK"], pat.row_ptr, 1e-12)
