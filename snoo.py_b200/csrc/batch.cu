@@ -1173,13 +1173,13 @@ struct snp_batch {
 
     // One pass of the solver's loop as graph nodes in `nb`: for each phase, a flag kernel and an
     // IF node over that phase's kernels; then the loop's own condition.  The CG phase's node
-    // holds pcg_body_unroll() CG iterations (a problem whose CG ends inside it leaves the phase,
+    // holds pcg_body_unroll(4) CG iterations (a problem whose CG ends inside it leaves the phase,
     // and the remaining iterations skip its units), so a pass's fixed cost (six flag kernels,
     // five conditional nodes) is shared by several CG iterations.
     template <typename TT>
     int build_pass(Seq &nb, cudaStream_t cs, const cudaGraphConditionalHandle *hp, cudaGraphConditionalHandle hn) {
         const int phases[5] = {snp::PH_HEAD, snp::PH_CG, snp::PH_EXTRACT, snp::PH_LS, snp::PH_ACCEPT};
-        const int cg_unroll = snp::pcg_body_unroll();
+        const int cg_unroll = snp::pcg_body_unroll(4);
         for (int k = 0; k < 5; ++k) {
             const int ph = phases[k];
             SNP_TRY(capture(nb, cs, [&](cudaStream_t s) { return flag(s, ph, 1, hp[k]); }));

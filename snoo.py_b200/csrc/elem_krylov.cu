@@ -171,6 +171,19 @@ Chat<TT> chat_of(const ElemTopology &top) {
     return ch;
 }
 
+// The passes of the iterations are launched so that a pass may start while the one before it
+// drains.  Here a pass waits until the one before it has completed (which had waited for its own
+// predecessor), and lets the next one start.  Only the topology, the tensors and the block inverses
+// may be read before, nothing may be written; what the other passes write (G, R, Y, the CG state) is
+// read with plain loads, since a read-only path's data may not change while the kernel is resident.
+__device__ __forceinline__ void pass_begins() {
+    cudaGridDependencySynchronize();
+}
+
+__device__ __forceinline__ void next_pass_may_start(int early) {
+    if (early) cudaTriggerProgrammaticLaunchCompletion();
+}
+
 // u_e of the element's directions pk (signs applied): edges 0-2 and 3-5 summed apart
 template <typename TT>
 __device__ __forceinline__ void element_u(const TT (&pk)[6], const Chat<TT> &ch, TT &u0, TT &u1, TT &u2) {
@@ -204,20 +217,23 @@ __device__ __forceinline__ void apply_tensor(const TT (&t)[6], TT u0, TT u1, TT 
 //
 // In float64 (float32: k_epass1_pair).  Bound by the L1 data pipe (a slot per sector of the
 // scattered stores and gathers, 70-80% busy), at small sizes by the launch and its chain of
-// dependent loads.  Two lanes per element with shuffles were slower at every size: 28.3 against 25.4 us per iteration
-// at 287k tets, 17.0 against 15.7 at 100k, 70.7 against 69.9 at 1.16M.  Storing v_e instead of the
+// dependent loads.  Two lanes per element with shuffles were slower at every size (passes not
+// overlapping): 28.3 against 25.4 us per iteration at 287k tets, 17.0 against 15.7 at 100k, 70.7
+// against 69.9 at 1.16M.  In float32 one lane per element is no faster where it counts: 20.7 against
+// 20.9 us per iteration at 300k tets, 54.4 against 53.6 at 1.16M.  Storing v_e instead of the
 // terms halves this pass (20 us at 1.16M) and adds as much to the DoF pass, which then gathers.
 template <typename TT>
 __global__ void __launch_bounds__(kEBlock, 3)
     k_epass1(int64_t ne, const int32_t *__restrict__ edof, const int32_t *__restrict__ pos,
-             const TT *__restrict__ T, const Chat<TT> ch, const DofPair<TT> *__restrict__ G, TT *__restrict__ Y,
-             PcgState *st, double *part) {
+             const TT *__restrict__ T, const Chat<TT> ch, const DofPair<TT> *G, TT *Y,
+             PcgState *st, double *part, int early) {
     __shared__ double sh[32];
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     int32_t d[6];
 #pragma unroll
     for (int k = 0; k < 6; ++k) d[k] = e < ne ? __ldcs(edof + eslot(e, k)) : 0;
+    pass_begins();
     if (st->done) return;
     const TT beta = (TT)st->beta;
     double dot = 0.0;
@@ -250,6 +266,7 @@ __global__ void __launch_bounds__(kEBlock, 3)
 #pragma unroll
         for (int k = 0; k < 6; ++k) d[k] = nd[k];
     }
+    next_pass_may_start(early);
     dot = block_sum(dot, sh);
     if (threadIdx.x == 0) part[blockIdx.x] = dot;
     if (last_block(&st->counter)) {
@@ -275,8 +292,8 @@ __device__ __forceinline__ void load_chat(TT *sc, const TT *chat) {
 template <typename TT>
 __global__ void __launch_bounds__(kEBlock, 4)
     k_epass1_pair(int64_t ne, const int32_t *__restrict__ edof, const int32_t *__restrict__ pos,
-             const TT *__restrict__ T, const TT *__restrict__ chat, const DofPair<TT> *__restrict__ G,
-             TT *__restrict__ Y, PcgState *st, double *part) {
+             const TT *__restrict__ T, const TT *__restrict__ chat, const DofPair<TT> *G,
+             TT *Y, PcgState *st, double *part, int early) {
     __shared__ TT sc[18];
     __shared__ double sh[32];
     const int lane = threadIdx.x & 31;
@@ -305,6 +322,7 @@ __global__ void __launch_bounds__(kEBlock, 4)
         }
     };
     if (first < ne) stream_in(first, d, ps, th);
+    pass_begins();
     if (st->done) return;
     load_chat(sc, chat);
     const TT beta = (TT)st->beta;
@@ -369,6 +387,7 @@ __global__ void __launch_bounds__(kEBlock, 4)
         for (int j = 0; j < 3; ++j)
             Y[ps[j]] = edge_term(sc, 3 * h + j, d[j] < 0, v0, v1, v2);
     }
+    next_pass_may_start(early);
     dot = block_sum(dot, sh);
     if (threadIdx.x == 0) part[blockIdx.x] = dot;
     if (last_block(&st->counter)) {
@@ -422,9 +441,10 @@ __device__ __forceinline__ void close_dof_pass(double rz, double rr, double (*sh
 template <typename TT>
 __global__ void __launch_bounds__(kEBlock)
     k_epass2(int32_t n, const uint8_t *__restrict__ free_mask, const int32_t *__restrict__ inc_ptr,
-             const TT *__restrict__ Y, DofPair<TT> *__restrict__ G, DofPair<TT> *__restrict__ R,
-             const TT *__restrict__ D, PcgState *st, double *part, int use_cond, cudaGraphConditionalHandle cond) {
+             const TT *Y, DofPair<TT> *__restrict__ G, DofPair<TT> *__restrict__ R,
+             const TT *__restrict__ D, PcgState *st, double *part, int use_cond, cudaGraphConditionalHandle cond, int early) {
     __shared__ double sh2[2][32];
+    pass_begins();
     if (st->done) {
         if (use_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(cond, 0);
         return;
@@ -447,6 +467,7 @@ __global__ void __launch_bounds__(kEBlock)
         rz += (double)r * (double)z;
         rr += (double)r * (double)r;
     }
+    next_pass_may_start(early);
     close_dof_pass(rz, rr, sh2, part, st, use_cond, cond);
 }
 
@@ -454,9 +475,9 @@ __global__ void __launch_bounds__(kEBlock)
 template <typename TT>
 __global__ void __launch_bounds__(kEBlock)
     k_epass2_direct(int32_t n, const uint8_t *__restrict__ free_mask, const int32_t *__restrict__ inc_ptr,
-                const TT *__restrict__ Y, const uint16_t *__restrict__ meta, const float *__restrict__ binv,
+                const TT *Y, const uint16_t *__restrict__ meta, const float *__restrict__ binv,
                 DofPair<TT> *__restrict__ G, DofPair<TT> *__restrict__ R, PcgState *st, double *part, int use_cond,
-                cudaGraphConditionalHandle cond) {
+                cudaGraphConditionalHandle cond, int early) {
     __shared__ double sh2[2][32];
     // float64: r of the tile in two alternating buffers, so a tile needs one barrier: it writes
     // the buffer its predecessor's predecessor read, which every thread has finished with once
@@ -477,7 +498,10 @@ __global__ void __launch_bounds__(kEBlock)
         if (i0 < n) {
             nb0 = __ldcs(inc_ptr + i0);
             nb1 = __ldcs(inc_ptr + i0 + 1);
-            if constexpr (kStateAhead) {
+        }
+        pass_begins();
+        if constexpr (kStateAhead) {
+            if (i0 < n) {
                 ng = G[i0];
                 nrx = R[i0];
             }
@@ -536,6 +560,7 @@ __global__ void __launch_bounds__(kEBlock)
         }
         if constexpr (!kTwoBuffers) __syncthreads();
     }
+    next_pass_may_start(early);
     close_dof_pass(rz, rr, sh2, part, st, use_cond, cond);
 }
 
@@ -590,7 +615,7 @@ struct DofPassArgs {
 
 template <typename TT>
 __global__ void __launch_bounds__(kDofThreads, 4)
-    k_epass2_bj(const DofPassArgs<TT> a, PcgState *st, double *part, int use_cond, cudaGraphConditionalHandle cond) {
+    k_epass2_bj(const DofPassArgs<TT> a, PcgState *st, double *part, int use_cond, cudaGraphConditionalHandle cond, int early) {
     extern __shared__ __align__(128) unsigned char dof_smem[];
     DofStage<TT> *stage = reinterpret_cast<DofStage<TT> *>(dof_smem);
     __shared__ double sh2[2][32];
@@ -611,7 +636,7 @@ __global__ void __launch_bounds__(kDofThreads, 4)
     double rz = 0.0, rr = 0.0;
     if (producer) {
         if (threadIdx.x == kEBlock) {
-            auto issue = [&](int32_t tile, int s) {
+            auto issue = [&](int32_t tile, int s, bool before) {
                 DofStage<TT> &D = stage[s];
                 constexpr int kA = 16 / (int)sizeof(TT);  // values per 16 bytes
                 const int32_t i0 = __ldg(a.tile_inc + tile), i1 = __ldg(a.tile_inc + tile + 1);
@@ -622,13 +647,15 @@ __global__ void __launch_bounds__(kDofThreads, 4)
                 const uint32_t mb = (uint32_t)(m1 - m0) * 4u;
                 const uint32_t yb = staged && i1 > i0 ? (uint32_t)(cn * (int)sizeof(TT)) : 0u;
                 mbar_arrive_expect(full + s, kBjTile * 4u + mb + yb);
-                if (yb) bulk_load(D.y, a.Y + c0, yb, full + s);
                 bulk_load(D.word, a.word + (int64_t)tile * kBjTile, kBjTile * 4u, full + s);
                 if (mb) bulk_load(D.m, a.packed + m0, mb, full + s);
+                if (before) pass_begins();
+                if (yb) bulk_load(D.y, a.Y + c0, yb, full + s);
             };
             int issued = 0;
             int32_t tile = blockIdx.x;
-            for (; issued < kDofStages && tile < a.tiles; ++issued, tile += gridDim.x) issue(tile, issued);
+            for (; issued < kDofStages && tile < a.tiles; ++issued, tile += gridDim.x) issue(tile, issued, issued == 0);
+            if (issued == 0) pass_begins();
             if (*(volatile int *)&st->done) {
                 // a finished solve: the copies in flight end before the block does
                 for (int s = 0; s < issued; ++s) mbar_wait_bounded(full + s, 0);
@@ -641,12 +668,12 @@ __global__ void __launch_bounds__(kDofThreads, 4)
                             mbar_wait_bounded(full + q, (uint32_t)(((it - 1 - (it - 1 - q) % kDofStages) / kDofStages) & 1));
                         break;
                     }
-                    issue(tile, s);
+                    issue(tile, s, false);
                 }
             }
         }
         __syncwarp();
-    } else if (!st->done) {
+    } else if (pass_begins(), !st->done) {
         const TT alpha = (TT)st->alpha, beta = (TT)st->beta;
         const int tid = threadIdx.x;
         int it = 0;
@@ -674,7 +701,7 @@ __global__ void __launch_bounds__(kDofThreads, 4)
                 if (ti.shift >= 0)
                     for (int t = b0; t < b1; ++t) q += (double)D.y[ti.shift + t];
                 else
-                    for (int t = b0; t < b1; ++t) q += (double)__ldg(a.Y + ti.first + t);
+                    for (int t = b0; t < b1; ++t) q += (double)a.Y[ti.first + t];
                 r = rx.a - alpha * (TT)q;
             }
             s_r[tid] = r;
@@ -714,6 +741,7 @@ __global__ void __launch_bounds__(kDofThreads, 4)
         if (use_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(cond, 0);
         return;
     }
+    next_pass_may_start(early);
     close_dof_pass(rz, rr, sh2, part, st, use_cond, cond);
 }
 
@@ -1506,26 +1534,52 @@ int ElemPcg<TT>::reserve(int32_t n_, int64_t ne_) {
     return SNP_OK;
 }
 
+namespace {
+// Launch that may overlap the end of the previous kernel on the stream (pass_begins); errors are
+// left for the caller's launch check.
+template <typename... P, typename... A>
+void launch_pass(void (*kern)(P...), int grid, int block, size_t smem, cudaStream_t s, const A &...args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    (void)cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+}  // namespace
+
 template <typename TT>
 int ElemPcg<TT>::launch_iteration(const ElemTopology &top, const TT *T, const uint8_t *free_mask,
                                   const BlockPlan *plan, cudaStream_t s, int use_cond,
                                   cudaGraphConditionalHandle cond) {
     const Chat<TT> ch = chat_of<TT>(top);
-    if constexpr (sizeof(TT) == 4)
-        k_epass1_pair<TT><<<wave_grid(k_epass1_pair<TT>, 2 * ne, kEBlock), kEBlock, 0, s>>>(
-            ne, top.edof.p, top.pos.p, T, chat_ptr<TT>(top), G.p, Y.p, st.p, part.p);
-    else
-        k_epass1<TT><<<wave_grid(k_epass1<TT>, ne, kEBlock), kEBlock, 0, s>>>(ne, top.edof.p, top.pos.p, T, ch, G.p,
-                                                                            Y.p, st.p, part.p);
-    SNP_LAUNCH_CHECK();
     const int staged_grid =
         plan ? wave_grid(k_epass2_bj<TT>, (int64_t)plan->tiles * kDofThreads, kDofThreads, dof_pass_smem<TT>()) : 0;
+    const bool staged = plan && sizeof(TT) == 8 && plan->tiles >= 4 * staged_grid;
+    // Where a pass lets the next one start before its block sums: in float32 (per iteration at 38k,
+    // 150k and 300k tets 13.0, 16.3 and 21.7 us without, 12.3, 15.8 and 20.9 with; launches that do
+    // not overlap 13.6, 16.8 and 22.3) and in float64 around the staged DoF pass (69.2 against 67.8
+    // at 1.16M; 70.0 not overlapping).  In float64 below, the early blocks cost what they gain:
+    // 12.5, 18.5 and 24.7 without, 13.3, 19.2 and 25.5 with (12.7, 18.9 and 24.9 not overlapping).
+    const int early = sizeof(TT) == 4 || staged ? 1 : 0;
+    if constexpr (sizeof(TT) == 4)
+        launch_pass(k_epass1_pair<TT>, wave_grid(k_epass1_pair<TT>, 2 * ne, kEBlock), kEBlock, 0, s, ne, top.edof.p,
+                    top.pos.p, T, chat_ptr<TT>(top), G.p, Y.p, st.p, part.p, early);
+    else
+        launch_pass(k_epass1<TT>, wave_grid(k_epass1<TT>, ne, kEBlock), kEBlock, 0, s, ne, top.edof.p, top.pos.p, T, ch,
+                    G.p, Y.p, st.p, part.p, early);
+    SNP_LAUNCH_CHECK();
     // the staged DoF pass in float64 from four tiles per block on: 39.5 against 40.3 us per iteration
     // at 600k tets, 69.9 against 74.7 at 1.16M; below, 25.7 against 25.4 at 287k and 16.5 against
     // 15.7 at 100k (float32: 52.4 against 53.1 at 1.16M, 13.3 against 13.3 at 38k)
-    if (plan && (sizeof(TT) == 4 || plan->tiles < 4 * staged_grid)) {
-        k_epass2_direct<TT><<<wave_grid(k_epass2_direct<TT>, n, kEBlock), kEBlock, 0, s>>>(
-            n, free_mask, top.inc_ptr.p, Y.p, plan->meta, plan->binv, G.p, R.p, st.p, part.p, use_cond, cond);
+    if (plan && !staged) {
+        launch_pass(k_epass2_direct<TT>, wave_grid(k_epass2_direct<TT>, n, kEBlock), kEBlock, 0, s, n, free_mask,
+                    top.inc_ptr.p, Y.p, plan->meta, plan->binv, G.p, R.p, st.p, part.p, use_cond, cond, early);
         SNP_LAUNCH_CHECK();
         return SNP_OK;
     }
@@ -1542,10 +1596,10 @@ int ElemPcg<TT>::launch_iteration(const ElemTopology &top, const TT *T, const ui
         a.G = G.p;
         a.R = R.p;
         const size_t smem = dof_pass_smem<TT>();
-        k_epass2_bj<TT><<<staged_grid, kDofThreads, smem, s>>>(a, st.p, part.p, use_cond, cond);
+        launch_pass(k_epass2_bj<TT>, staged_grid, kDofThreads, smem, s, a, st.p, part.p, use_cond, cond, early);
     } else {
-        k_epass2<TT><<<wave_grid(k_epass2<TT>, n, kEBlock), kEBlock, 0, s>>>(
-            n, free_mask, top.inc_ptr.p, Y.p, G.p, R.p, D.p, st.p, part.p, use_cond, cond);
+        launch_pass(k_epass2<TT>, wave_grid(k_epass2<TT>, n, kEBlock), kEBlock, 0, s, n, free_mask, top.inc_ptr.p, Y.p,
+                    G.p, R.p, D.p, st.p, part.p, use_cond, cond, early);
     }
     SNP_LAUNCH_CHECK();
     return SNP_OK;
@@ -1628,7 +1682,7 @@ int ElemPcg<TT>::build_graph(const ElemTopology &top, const TT *T, const uint8_t
         cudaGraph_t body = cp.conditional.phGraph_out[0];
         ok = cudaStreamBeginCaptureToGraph(cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
         if (ok) {
-            const int unroll = pcg_body_unroll();
+            const int unroll = pcg_body_unroll(8);
             int rc = SNP_OK;
             for (int u = 0; u < unroll && rc == SNP_OK; ++u)
                 rc = launch_iteration(top, T, free_mask, plan, cs, 1, h);

@@ -12,13 +12,15 @@
 namespace snp {
 
 // CG iterations captured per execution of a Krylov graph's conditional WHILE body:
-// SNP_PCG_UNROLL (1-16), default 4.  Every execution of the body costs a few microseconds
-// beyond its kernels (about 3.5 us per float64 iteration of the 1.16M-tet benchmark with one
-// iteration per body); the passes of a solve that finished inside a body return at once, so
-// the body's remaining iterations cost only their launches.
-inline int pcg_body_unroll() {
+// SNP_PCG_UNROLL (1-16), else the engine's default.  Every execution of the body costs a few
+// microseconds beyond its kernels, and its first pass cannot start early; the passes of a solve that
+// finished inside a body return at once, so the body's remaining iterations cost only their
+// launches.  Element engine, 8: 12.3, 18.3 and 67.2 us per float64 iteration at 38k, 150k and 1.16M
+// tets, against 12.6, 18.6 and 67.8 with 4 and 13.3, 19.7 and 68.7 with 2; 12 measured as 8.
+// CSR engine, 4: its graph may be built for one solve.  Batch, 4: problems leave the body together.
+inline int pcg_body_unroll(int standard) {
     const char *e = getenv("SNP_PCG_UNROLL");
-    if (!e || !e[0]) return 4;
+    if (!e || !e[0]) return standard;
     const int u = atoi(e);
     return u < 1 ? 1 : (u > 16 ? 16 : u);
 }

@@ -334,3 +334,22 @@ def test_gradgrad_system_matches_material_by_material(sizes, wanted):
                   _lib.ptr(acc["K"]), _lib.ptr(acc["dK"]), None, _lib.stream_ptr())
         _assert_rows_close(acc["K"], ref["K"], pat.row_ptr, 1e-12)
         _assert_rows_close(acc["dK"], ref["dK"], pat.row_ptr, 1e-12)
+
+
+@pytest.mark.parametrize("tets,precision", [(900, "fp64"), (900, "mixed"), (60000, "mixed"), (620000, "fp64")])
+def test_overlapping_passes_give_one_answer(tets, precision, monkeypatch):
+    """CG passes that may start while the previous one drains, captured in the loop body and
+    launched one by one: bitwise the same solve, and the same again."""
+    import torch
+
+    s = _window_solver(tets)
+    out = []
+    for graph in ("1", "0", "1"):
+        monkeypatch.setenv("SNP_PCG_GRAPH", graph)
+        eng = s.newton_engine()
+        x, st = eng.solve(None, tol=1e-8, max_newton=2, precision={"fp64": 0, "mixed": 1}[precision],
+                          raise_on_failure=False)
+        out.append((x.clone(), st["cg_iterations"]))
+        s._newton = None
+    assert out[0][1] == out[1][1] == out[2][1] > 10
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][0], out[2][0])
