@@ -85,34 +85,130 @@ __device__ __forceinline__ void store_vectors(const CurlArgs &a, int64_t eo, con
 // and the element's node z coordinates Zn[4]
 template <bool DIL>
 __device__ __forceinline__ double nu_at(const CurlArgs &a, const double *relc, const double *relx, const double *ph,
-                                        const double (&Zn)[4], double bm, double &dnu) {
+                                        const double (&Zn)[4], double bm, double &dnu, int &near) {
     if constexpr (!DIL) {
-        return pchip_eval<double>(a.n_int, relc, relx, bm, dnu);
+        return pchip_eval<double>(a.n_int, relc, relx, bm, dnu, near);
     } else {
         double z = 0.0;
 #pragma unroll
         for (int i = 0; i < 4; ++i) z += ph[i] * Zn[i];
         const double sf = (a.dil[0] + z * a.dil[1]) / (a.dil[2] + z * a.dil[3]);
-        const double nu = sf * pchip_eval<double>(a.n_int, relc, relx, sf * bm, dnu);
+        const double nu = sf * pchip_eval<double>(a.n_int, relc, relx, sf * bm, dnu, near);
         dnu *= sf * sf;
         return nu;
     }
 }
 
-// One element's K and dK (upper triangle), residual terms Fj = (K x)_j - r_j and reduced-rhs terms
-// r_j.  emit(tri, j, k, kv, dv) is called for the 21 pairs j <= k row by row; r is set only with
-// HAS_BS (a source field at each quadrature point).  NQ: compile-time number of quadrature points
-// (0 = runtime count); DIL: diluted steel (with HAS_BS only).  The tables sit in shared memory.
-template <bool HAS_BS, int NQ, bool DIL, typename Emit>
-__device__ __forceinline__ void curl_element(const CurlArgs &a, int64_t e, const double *s_ctab, const double *s_dphi,
-                                             const double *s_w, const double *s_phi, const double *s_relc,
-                                             const double *s_relx, double wsum, int (&g)[6], double (&Fj)[6],
-                                             double (&r)[6], Emit emit) {
+// What the quadrature points of an element contribute: k = sum nu w, M = sum a B B^T (xx xy xz yy
+// yz zz) with a = [|B| >= 1e-14] nu' w / (det |B|), R = sum (nu0 - nu) w B_s.
+struct PointSums {
+    double k, M[6], R[3];
+    __device__ __forceinline__ void add(const PointSums &o) {
+        k += o.k;
+#pragma unroll
+        for (int t = 0; t < 6; ++t) M[t] += o.M[t];
+#pragma unroll
+        for (int t = 0; t < 3; ++t) R[t] += o.R[t];
+    }
+    __device__ __forceinline__ void load(const double *at) {
+        k = at[0];
+#pragma unroll
+        for (int t = 0; t < 6; ++t) M[t] = at[1 + t];
+#pragma unroll
+        for (int t = 0; t < 3; ++t) R[t] = at[7 + t];
+    }
+    __device__ __forceinline__ PointSums from_lane(int x) const {
+        PointSums o;
+        o.k = __shfl_xor_sync(0xffffffffu, k, x);
+#pragma unroll
+        for (int t = 0; t < 6; ++t) o.M[t] = __shfl_xor_sync(0xffffffffu, M[t], x);
+#pragma unroll
+        for (int t = 0; t < 3; ++t) o.R[t] = __shfl_xor_sync(0xffffffffu, R[t], x);
+        return o;
+    }
+};
+
+// the points first, first + step, ... of an element with B_s at bs and B of its own edges Bc
+template <int NQ, bool DIL>
+__device__ __forceinline__ PointSums point_sums(const CurlArgs &a, const double *bs, const double (&Bc)[3],
+                                                const double *s_w, const double *s_phi, const double *s_relc,
+                                                const double *s_relx, const double (&Zn)[4], double idet, int first,
+                                                int step) {
     const int nq = NQ > 0 ? NQ : a.nq;
+    PointSums p{};
+    int near = 0;
+    double n0 = 0.0, n1 = 0.0, n2 = 0.0;  // B_s of the next point
+    if (first < nq) {
+        n0 = __ldg(bs + 3 * first);
+        n1 = __ldg(bs + 3 * first + 1);
+        n2 = __ldg(bs + 3 * first + 2);
+    }
+#pragma unroll(NQ > 0 ? NQ : 1)
+    for (int q = first; q < nq; q += step) {
+        const double s0 = n0, s1 = n1, s2 = n2;
+        if (q + step < nq) {
+            n0 = __ldg(bs + 3 * (q + step));
+            n1 = __ldg(bs + 3 * (q + step) + 1);
+            n2 = __ldg(bs + 3 * (q + step) + 2);
+        }
+        const double B0 = s0 + Bc[0], B1 = s1 + Bc[1], B2 = s2 + Bc[2];
+        const double bm = sqrt(B0 * B0 + B1 * B1 + B2 * B2);
+        double dnu;
+        const double nu = nu_at<DIL>(a, s_relc, s_relx, s_phi + 4 * q, Zn, bm, dnu, near);
+        const double wq = s_w[q];
+        const double aq = (bm >= 1e-14) ? dnu * wq * idet / bm : 0.0;
+        const double rq = (kNu0 - nu) * wq;
+        p.k += nu * wq;
+        const double a0 = aq * B0, a1 = aq * B1, a2 = aq * B2;
+        p.M[0] += a0 * B0;
+        p.M[1] += a0 * B1;
+        p.M[2] += a0 * B2;
+        p.M[3] += a1 * B1;
+        p.M[4] += a1 * B2;
+        p.M[5] += a2 * B2;
+        p.R[0] += rq * s0;
+        p.R[1] += rq * s1;
+        p.R[2] += rq * s2;
+    }
+    return p;
+}
+
+// All points of an element.  A runtime number of points is summed in four interleaved classes,
+// (0 + 1) + (2 + 3): here, or by four lanes in k_point_sums with the same roundings.
+constexpr int kPointLanes = 4;
+constexpr int kPointBlock = 256;
+template <int NQ, bool DIL>
+__device__ __forceinline__ PointSums all_points(const CurlArgs &a, const double *bs, const double (&Bc)[3],
+                                                const double *s_w, const double *s_phi, const double *s_relc,
+                                                const double *s_relx, const double (&Zn)[4], double idet) {
+    auto part = [&](int first, int step) {
+        return point_sums<NQ, DIL>(a, bs, Bc, s_w, s_phi, s_relc, s_relx, Zn, idet, first, step);
+    };
+    if constexpr (NQ > 0) {
+        return part(0, 1);
+    } else {
+        PointSums p = part(0, kPointLanes);
+        p.add(part(1, kPointLanes));
+        PointSums o = part(2, kPointLanes);
+        o.add(part(3, kPointLanes));
+        p.add(o);
+        return p;
+    }
+}
+
+// Curls c_j = Jm chat_j, values x and DoFs g of an element's edges, B of the edges, 1 / det and the
+// nodes' z coordinates.
+struct ElemGeometry {
+    double c[6][3], xv[6], Bc[3], idet, Zn[4];
+    int g[6];
+};
+
+__device__ __forceinline__ void element_geometry(const CurlArgs &a, int64_t e, const double *s_ctab,
+                                                 const double *s_dphi, ElemGeometry &G) {
     const int4 cv = __ldg(reinterpret_cast<const int4 *>(a.cells) + e);
     const int cidx[4] = {cv.x, cv.y, cv.z, cv.w};
     // Jacobian J[k][l] = sum_i X[i][k] dphi[i][l]
-    double Jm[9], Zn[4];
+    double Jm[9];
 #pragma unroll
     for (int t = 0; t < 9; ++t) Jm[t] = 0.0;
 #pragma unroll
@@ -120,7 +216,7 @@ __device__ __forceinline__ void curl_element(const CurlArgs &a, int64_t e, const
         const double X0 = __ldg(a.nodes + 3 * (int64_t)cidx[i]);
         const double X1 = __ldg(a.nodes + 3 * (int64_t)cidx[i] + 1);
         const double X2 = __ldg(a.nodes + 3 * (int64_t)cidx[i] + 2);
-        Zn[i] = X2;
+        G.Zn[i] = X2;
 #pragma unroll
         for (int l = 0; l < 3; ++l) {
             const double d = s_dphi[3 * i + l];
@@ -131,41 +227,56 @@ __device__ __forceinline__ void curl_element(const CurlArgs &a, int64_t e, const
     }
     const double det = Jm[0] * (Jm[4] * Jm[8] - Jm[7] * Jm[5]) - Jm[1] * (Jm[3] * Jm[8] - Jm[5] * Jm[6]) +
                        Jm[2] * (Jm[3] * Jm[7] - Jm[4] * Jm[6]);
-    const double idet = 1.0 / det;
+    G.idet = 1.0 / det;
     const int o = __ldg(a.orient + e);
     const double *ct = s_ctab + o * 18;
     {
         const int2 *gp = reinterpret_cast<const int2 *>(a.gids + 6 * e);
         int2 g01 = __ldg(gp), g23 = __ldg(gp + 1), g45 = __ldg(gp + 2);
-        g[0] = g01.x; g[1] = g01.y; g[2] = g23.x; g[3] = g23.y; g[4] = g45.x; g[5] = g45.y;
+        G.g[0] = g01.x; G.g[1] = g01.y; G.g[2] = g23.x; G.g[3] = g23.y; G.g[4] = g45.x; G.g[5] = g45.y;
     }
-    double c[6][3], xv[6];
-    double Bc[3] = {0.0, 0.0, 0.0};
+    G.Bc[0] = G.Bc[1] = G.Bc[2] = 0.0;
 #pragma unroll
     for (int j = 0; j < 6; ++j) {
         const double h0 = ct[3 * j], h1 = ct[3 * j + 1], h2 = ct[3 * j + 2];
-        c[j][0] = Jm[0] * h0 + Jm[1] * h1 + Jm[2] * h2;
-        c[j][1] = Jm[3] * h0 + Jm[4] * h1 + Jm[5] * h2;
-        c[j][2] = Jm[6] * h0 + Jm[7] * h1 + Jm[8] * h2;
-        xv[j] = __ldg(a.x + g[j]);
-        Bc[0] += c[j][0] * xv[j];
-        Bc[1] += c[j][1] * xv[j];
-        Bc[2] += c[j][2] * xv[j];
+        G.c[j][0] = Jm[0] * h0 + Jm[1] * h1 + Jm[2] * h2;
+        G.c[j][1] = Jm[3] * h0 + Jm[4] * h1 + Jm[5] * h2;
+        G.c[j][2] = Jm[6] * h0 + Jm[7] * h1 + Jm[8] * h2;
+        G.xv[j] = __ldg(a.x + G.g[j]);
+        G.Bc[0] += G.c[j][0] * G.xv[j];
+        G.Bc[1] += G.c[j][1] * G.xv[j];
+        G.Bc[2] += G.c[j][2] * G.xv[j];
     }
-    Bc[0] *= idet;
-    Bc[1] *= idet;
-    Bc[2] *= idet;
+    G.Bc[0] *= G.idet;
+    G.Bc[1] *= G.idet;
+    G.Bc[2] *= G.idet;
+}
 
+// One element's K and dK (upper triangle), residual terms Fj = (K x)_j - r_j and reduced-rhs terms
+// r_j.  emit(tri, j, k, kv, dv) is called for the 21 pairs j <= k row by row; r is set only with
+// HAS_BS (a source field at each quadrature point).  NQ: compile-time number of quadrature points
+// (0 = runtime count); DIL: diluted steel (with HAS_BS only); pre: the element's point sums where
+// they are known, else NULL.  The tables sit in shared memory.
+template <bool HAS_BS, int NQ, bool DIL, bool PRE, typename Emit>
+__device__ __forceinline__ void curl_element(const CurlArgs &a, int64_t e, const double *s_ctab, const double *s_dphi,
+                                             const double *s_w, const double *s_phi, const double *s_relc,
+                                             const double *s_relx, double wsum, int (&g)[6], double (&Fj)[6],
+                                             double (&r)[6], const double *pre, Emit emit) {
+    ElemGeometry G;
+    element_geometry(a, e, s_ctab, s_dphi, G);
+    double(&c)[6][3] = G.c, (&xv)[6] = G.xv;
+#pragma unroll
+    for (int j = 0; j < 6; ++j) g[j] = G.g[j];
     double kfac;  // sum_q nu_q w_q / det
     if constexpr (!HAS_BS) {
-        const double bm = sqrt(Bc[0] * Bc[0] + Bc[1] * Bc[1] + Bc[2] * Bc[2]);
+        const double bm = sqrt(G.Bc[0] * G.Bc[0] + G.Bc[1] * G.Bc[1] + G.Bc[2] * G.Bc[2]);
         double dnu;
         const double nu = pchip_eval<double>(a.n_int, s_relc, s_relx, bm, dnu);
-        kfac = nu * wsum * idet;
-        const double af = (bm >= 1e-14) ? dnu * wsum * idet / bm : 0.0;
+        kfac = nu * wsum * G.idet;
+        const double af = (bm >= 1e-14) ? dnu * wsum * G.idet / bm : 0.0;
         double p[6];
 #pragma unroll
-        for (int j = 0; j < 6; ++j) p[j] = c[j][0] * Bc[0] + c[j][1] * Bc[1] + c[j][2] * Bc[2];
+        for (int j = 0; j < 6; ++j) p[j] = c[j][0] * G.Bc[0] + c[j][1] * G.Bc[1] + c[j][2] * G.Bc[2];
 #pragma unroll
         for (int j = 0; j < 6; ++j) Fj[j] = 0.0;
         int tri = 0;
@@ -181,41 +292,18 @@ __device__ __forceinline__ void curl_element(const CurlArgs &a, int64_t e, const
             }
         }
     } else {
-        // one pass over the quadrature points: accumulate sum_q nu w, the reduced rhs
-        // and the 21 dK pair sums (any number of points, fixed register footprint)
-        double dk[21];
+        PointSums ps;
+        if constexpr (PRE) ps.load(pre);
+        else ps = all_points<NQ, DIL>(a, a.Bs + (int64_t)e * a.nq * 3, G.Bc, s_w, s_phi, s_relc, s_relx, G.Zn, G.idet);
+        kfac = ps.k * G.idet;
+        double mc[6][3];  // M c_j
 #pragma unroll
-        for (int t = 0; t < 21; ++t) dk[t] = 0.0;
-#pragma unroll
-        for (int j = 0; j < 6; ++j) r[j] = 0.0;
-        kfac = 0.0;
-        const double *bs = a.Bs + (int64_t)e * nq * 3;
-#pragma unroll(NQ > 0 ? NQ : 1)
-        for (int q = 0; q < nq; ++q) {
-            const double s0 = __ldg(bs + 3 * q), s1 = __ldg(bs + 3 * q + 1), s2 = __ldg(bs + 3 * q + 2);
-            const double B0 = s0 + Bc[0], B1 = s1 + Bc[1], B2 = s2 + Bc[2];
-            const double bm = sqrt(B0 * B0 + B1 * B1 + B2 * B2);
-            double dnu;
-            const double nu = nu_at<DIL>(a, s_relc, s_relx, s_phi + 4 * q, Zn, bm, dnu);
-            const double wq = s_w[q];
-            kfac += nu * wq;
-            const double aq = (bm >= 1e-14) ? dnu * wq * idet / bm : 0.0;
-            const double rq = (kNu0 - nu) * wq;
-            double p[6];
-#pragma unroll
-            for (int j = 0; j < 6; ++j) {
-                p[j] = c[j][0] * B0 + c[j][1] * B1 + c[j][2] * B2;
-                r[j] += rq * (c[j][0] * s0 + c[j][1] * s1 + c[j][2] * s2);
-            }
-            int t = 0;
-#pragma unroll
-            for (int j = 0; j < 6; ++j) {
-                const double apj = aq * p[j];
-#pragma unroll
-                for (int k = j; k < 6; ++k) dk[t++] += apj * p[k];
-            }
+        for (int j = 0; j < 6; ++j) {
+            mc[j][0] = ps.M[0] * c[j][0] + ps.M[1] * c[j][1] + ps.M[2] * c[j][2];
+            mc[j][1] = ps.M[1] * c[j][0] + ps.M[3] * c[j][1] + ps.M[4] * c[j][2];
+            mc[j][2] = ps.M[2] * c[j][0] + ps.M[4] * c[j][1] + ps.M[5] * c[j][2];
+            r[j] = c[j][0] * ps.R[0] + c[j][1] * ps.R[1] + c[j][2] * ps.R[2];
         }
-        kfac *= idet;
 #pragma unroll
         for (int j = 0; j < 6; ++j) Fj[j] = -r[j];
         int tri = 0;
@@ -224,7 +312,7 @@ __device__ __forceinline__ void curl_element(const CurlArgs &a, int64_t e, const
 #pragma unroll
             for (int k = j; k < 6; ++k, ++tri) {
                 const double kv = kfac * (c[j][0] * c[k][0] + c[j][1] * c[k][1] + c[j][2] * c[k][2]);
-                emit(tri, j, k, kv, dk[tri]);
+                emit(tri, j, k, kv, c[j][0] * mc[k][0] + c[j][1] * mc[k][1] + c[j][2] * mc[k][2]);
                 Fj[j] = __fma_rn(kv, xv[k], Fj[j]);  // the same rounding in every kernel built on this
                 if (k != j) Fj[k] = __fma_rn(kv, xv[j], Fj[k]);
             }
@@ -272,7 +360,7 @@ __global__ void __launch_bounds__(kBlock)
         const int32_t *sl = want_mat ? a.slots + 36 * e : nullptr;
         int g[6];
         double Fj[6], r[6];
-        curl_element<HAS_BS, NQ, DIL>(a, e, T.ctab, T.dphi, T.w, T.phi, T.relc, T.relx, wsum, g, Fj, r,
+        curl_element<HAS_BS, NQ, DIL, false>(a, e, T.ctab, T.dphi, T.w, T.phi, T.relc, T.relx, wsum, g, Fj, r, nullptr,
                                       [&](int tri, int j, int k, double kv, double dv) {
             if (a.ET) store_pair(a, tri, eo, kv, dv);
             const int s1 = want_mat ? __ldg(sl + j * 6 + k) : 0;
@@ -302,12 +390,47 @@ __global__ void __launch_bounds__(kBlock)
     }
 }
 
+// Point sums of a material's elements, four lanes per element, into the first ten of each element's 21
+// values in `sums`.
+// An element's points are independent, and alone they need half the registers of the element kernel,
+// which kept the 21 sums of dK per point (now six of M) and a dozen warps an SM in flight.  Bound
+// by the latency of a point's chain (root, interval, two to four divisions) at the resident
+// warps.  64 points, with the element kernel that follows: 93 -> 53 us for the diluted steel of 150k
+// tets, 72 -> 27 of 20k; plain steel 160 -> 80 of 300k, 404 -> 235 of 1.1M (194 of them here, where B_s
+// alone is 0.7 GB).  Diluted steel runs better with two blocks an SM (42 against 47 us).
+template <bool DIL>
+__global__ void __launch_bounds__(kPointBlock, DIL ? 2 : 3)
+    k_point_sums(CurlArgs a, int quad_stride_ctab, double *sums) {
+    extern __shared__ double sm[];
+    const ElemTables T = stage_tables(a, quad_stride_ctab, sm);
+    constexpr int kElems = kPointBlock / kPointLanes;
+    const int sub = threadIdx.x % kPointLanes;
+    for (int64_t base = (int64_t)blockIdx.x * kElems; base < a.n_elems; base += (int64_t)gridDim.x * kElems) {
+        // lanes behind the last element repeat it, for the shuffles
+        const int64_t mine = base + threadIdx.x / kPointLanes, e = mine < a.n_elems ? mine : a.n_elems - 1;
+        PointSums p;
+        {
+            ElemGeometry G;
+            element_geometry(a, e, T.ctab, T.dphi, G);
+            p = point_sums<0, DIL>(a, a.Bs + e * a.nq * 3, G.Bc, T.w, T.phi, T.relc, T.relx, G.Zn, G.idet, sub,
+                                   kPointLanes);
+        }
+        p.add(p.from_lane(1));
+        p.add(p.from_lane(2));
+        const double v[10] = {p.k, p.M[0], p.M[1], p.M[2], p.M[3], p.M[4], p.M[5], p.R[0], p.R[1], p.R[2]};
+        double *at = sums + (a.t_offset + e) * kPackPairs;
+#pragma unroll
+        for (int t = 0; t < 10; ++t)
+            if (t % kPointLanes == sub && mine < a.n_elems) at[t] = v[t];
+    }
+}
+
 // Element values of the two-phase assembly with an element's values side by side (PackedTerms).
 // A CSR row takes up to six values of each of its elements, so phase 2 reads runs of neighbouring
 // doubles here, where blocks of equal-numbered values give it one useful double per 32-byte sector
 // (entry kernel, 1.16M tets: 571 us from the block layout, 2.7 GB through L2).  The values
 // leave through a shared tile so that the stores are whole lines.
-template <bool HAS_BS, int NQ, bool DIL>
+template <bool HAS_BS, int NQ, bool DIL, bool PRE>
 __global__ void __launch_bounds__(kBlock)
     k_curlcurl_packed(CurlArgs a, int quad_stride_ctab, int table_doubles, PackedTerms out) {
     extern __shared__ double sm[];
@@ -318,6 +441,8 @@ __global__ void __launch_bounds__(kBlock)
     double wsum = 0.0;
     for (int q = 0; q < nq; ++q) wsum += T.w[q];
     double *const first = out.J ? out.J : out.K;
+    // point sums of k_point_sums, in an array of which the block replaces the read elements later
+    const double *const sums = first ? first : out.D;
 
     for (int64_t base = (int64_t)blockIdx.x * kBlock; base < a.n_elems; base += (int64_t)gridDim.x * kBlock) {
         const int cnt = (int)(a.n_elems - base < kBlock ? a.n_elems - base : kBlock);
@@ -325,8 +450,9 @@ __global__ void __launch_bounds__(kBlock)
         int g[6];
         double Fj[6], r[6];
         if ((int)threadIdx.x < cnt)
-            curl_element<HAS_BS, NQ, DIL>(a, base + threadIdx.x, T.ctab, T.dphi, T.w, T.phi, T.relc, T.relx, wsum, g,
-                                          Fj, r, [&](int tri, int, int, double kv, double dv) {
+            curl_element<HAS_BS, NQ, DIL, PRE>(a, base + threadIdx.x, T.ctab, T.dphi, T.w, T.phi, T.relc, T.relx, wsum, g,
+                                               Fj, r, PRE ? sums + (eo + threadIdx.x) * kPackPairs : nullptr,
+                                               [&](int tri, int, int, double kv, double dv) {
                 if (first) tile[threadIdx.x * kPackPairs + tri] = out.J ? kv + dv : kv;
                 if (out.D) tile_d[threadIdx.x * kPackPairs + tri] = dv;
             });
@@ -517,30 +643,58 @@ __device__ __forceinline__ void elem_core(const CurlArgs &a, int64_t e, const do
         M[4] = af * Bc[1] * Bc[2];
         M[5] = af * Bc[2] * Bc[2];
     } else {
+        int near = 0;
         double kfac = 0.0;
 #pragma unroll
         for (int t = 0; t < 6; ++t) M[t] = 0.0;
+        // two points at a time, the next two requested ahead: every thread reads its own element's
+        // run, so a load instruction costs a slot of the L1 pipe per lane whatever its width
         const double *bs = a.Bs + (int64_t)e * nq * 3;
+        const bool wide = nq % 2 == 0 && ((uintptr_t)a.Bs & 15) == 0;
+        auto load2 = [&](int q, double (&v)[6]) {
+            if (wide) {
+#pragma unroll
+                for (int t = 0; t < 3; ++t) {
+                    const double2 d = __ldg(reinterpret_cast<const double2 *>(bs + 3 * q) + t);
+                    v[2 * t] = d.x;
+                    v[2 * t + 1] = d.y;
+                }
+            } else {
+#pragma unroll
+                for (int t = 0; t < 6; ++t) v[t] = q + t / 3 < nq ? __ldg(bs + 3 * q + t) : 0.0;
+            }
+        };
+        double nx[6];
+        load2(0, nx);
 #pragma unroll(NQ > 0 ? NQ : 1)
-        for (int q = 0; q < nq; ++q) {
-            const double s0 = __ldg(bs + 3 * q), s1 = __ldg(bs + 3 * q + 1), s2 = __ldg(bs + 3 * q + 2);
-            const double B0 = s0 + Bc[0], B1 = s1 + Bc[1], B2 = s2 + Bc[2];
-            const double bm = sqrt(B0 * B0 + B1 * B1 + B2 * B2);
-            double dnu;
-            const double nu = nu_at<DIL>(a, s_relc, s_relx, s_phi + 4 * q, Zn, bm, dnu);
-            const double wq = s_w[q];
-            kfac += nu * wq;
-            const double aq = (bm >= 1e-14) ? dnu * wq * idet / bm : 0.0;
-            const double rq = (kNu0 - nu) * wq;
-            M[0] += aq * B0 * B0;
-            M[1] += aq * B0 * B1;
-            M[2] += aq * B0 * B2;
-            M[3] += aq * B1 * B1;
-            M[4] += aq * B1 * B2;
-            M[5] += aq * B2 * B2;
-            Rs[0] += rq * s0;
-            Rs[1] += rq * s1;
-            Rs[2] += rq * s2;
+        for (int q0 = 0; q0 < nq; q0 += 2) {
+            double sv[6];
+#pragma unroll
+            for (int t = 0; t < 6; ++t) sv[t] = nx[t];
+            if (q0 + 2 < nq) load2(q0 + 2, nx);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int q = q0 + h;
+                if (q >= nq) break;
+                const double s0 = sv[3 * h], s1 = sv[3 * h + 1], s2 = sv[3 * h + 2];
+                const double B0 = s0 + Bc[0], B1 = s1 + Bc[1], B2 = s2 + Bc[2];
+                const double bm = sqrt(B0 * B0 + B1 * B1 + B2 * B2);
+                double dnu;
+                const double nu = nu_at<DIL>(a, s_relc, s_relx, s_phi + 4 * q, Zn, bm, dnu, near);
+                const double wq = s_w[q];
+                kfac += nu * wq;
+                const double aq = (bm >= 1e-14) ? dnu * wq * idet / bm : 0.0;
+                const double rq = (kNu0 - nu) * wq;
+                M[0] += aq * B0 * B0;
+                M[1] += aq * B0 * B1;
+                M[2] += aq * B0 * B2;
+                M[3] += aq * B1 * B1;
+                M[4] += aq * B1 * B2;
+                M[5] += aq * B2 * B2;
+                Rs[0] += rq * s0;
+                Rs[1] += rq * s1;
+                Rs[2] += rq * s2;
+            }
         }
         c.kfac = kfac * idet;
     }
@@ -726,17 +880,37 @@ int launch_t(const CurlArgs &a, cudaStream_t st, size_t smem, int qstride) {
     return SNP_OK;
 }
 
-template <bool HAS_BS, int NQ, bool DIL = false>
-int launch_packed_t(const CurlArgs &a, cudaStream_t st, int qstride, const PackedTerms &out) {
-    if (a.n_elems == 0) return SNP_OK;
-    auto kern = k_curlcurl_packed<HAS_BS, NQ, DIL>;
+template <bool HAS_BS, int NQ, bool DIL, bool PRE>
+int launch_packed_pre(const CurlArgs &a, cudaStream_t st, int qstride, const PackedTerms &out) {
+    auto kern = k_curlcurl_packed<HAS_BS, NQ, DIL, PRE>;
     const int tables = smem_layout(a.n_orient, a.nq, a.n_int).total;
     const size_t smem = sizeof(double) * ((size_t)tables + (out.D ? 2 : 1) * kBlock * kPackPairs);
     SNP_REQUIRE(smem <= 227 * 1024, "curl-curl assembly: tables need %zu bytes of shared memory", smem);
     if (smem > 48 * 1024) SNP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if constexpr (PRE) {
+        const size_t psmem = sizeof(double) * (size_t)tables;
+        auto points = k_point_sums<DIL>;
+        if (psmem > 48 * 1024)
+            SNP_CUDA_TRY(cudaFuncSetAttribute(points, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psmem));
+        double *sums = out.J ? out.J : out.K ? out.K : out.D;
+        points<<<wave_grid(points, a.n_elems * kPointLanes, kPointBlock, psmem), kPointBlock, psmem, st>>>(a, qstride, sums);
+        SNP_LAUNCH_CHECK();
+    }
     kern<<<wave_grid(kern, a.n_elems, kBlock, smem), kBlock, smem, st>>>(a, qstride, tables, out);
     SNP_LAUNCH_CHECK();
     return SNP_OK;
+}
+
+template <bool HAS_BS, int NQ, bool DIL = false>
+int launch_packed_t(const CurlArgs &a, cudaStream_t st, int qstride, const PackedTerms &out) {
+    if (a.n_elems == 0) return SNP_OK;
+    if constexpr (HAS_BS && NQ == 0) {
+        // 4 and 5 points have unrolled element kernels; the next rule has 27, where the separate
+        // launch already wins: 49 against 63 us (in the element kernel) at 300k tets, 18 against 31 at
+        // 20k, 144 against 160 at 1.1M; 64 points 80 against 123, 27 against 63, 235 against 321
+        if (a.nq >= 8 && (out.J || out.K || out.D)) return launch_packed_pre<HAS_BS, NQ, DIL, true>(a, st, qstride, out);
+    }
+    return launch_packed_pre<HAS_BS, NQ, DIL, false>(a, st, qstride, out);
 }
 
 }  // namespace

@@ -71,9 +71,12 @@ constexpr double kNu0 = 1.0 / 4.0 / 3.14159265358979323846 * 1e7;  // vacuum rel
 // PCHIP reluctance in piecewise-polynomial form (c[4][n_int] row-major, knots x[n_int+1]):
 // n_int == -1 is the constant c[0]; below x[0] (or NaN) 0; at/after x[n_int] the last
 // cubic extrapolates.  Binary search instead of the reference's linear scan
-// (fem_c/ctools.c:130-204); same interval choice.
+// (fem_c/ctools.c:130-204); same interval choice.  `near`: an interval to try first (in
+// [0, n_int)), then the one found: an element's quadrature points rarely differ in it, and a search
+// is five or six dependent reads.
 template <typename T>
-__device__ __forceinline__ T pchip_eval(int n_int, const T *__restrict__ c, const T *__restrict__ xk, T x, T &dval) {
+__device__ __forceinline__ T pchip_eval(int n_int, const T *__restrict__ c, const T *__restrict__ xk, T x, T &dval,
+                                        int &near) {
     if (n_int < 0) {
         dval = T(0);
         return c[0];
@@ -82,10 +85,10 @@ __device__ __forceinline__ T pchip_eval(int n_int, const T *__restrict__ c, cons
         dval = T(0);
         return T(0);
     }
-    int i;
+    int i = near;
     if (x >= xk[n_int]) {
         i = n_int - 1;
-    } else {
+    } else if (!(xk[i] <= x && x < xk[i + 1])) {
         int lo = 0, hi = n_int - 1;
         while (lo < hi) {
             int mid = (lo + hi + 1) >> 1;
@@ -93,10 +96,17 @@ __device__ __forceinline__ T pchip_eval(int n_int, const T *__restrict__ c, cons
         }
         i = lo;
     }
+    near = i;
     T d = x - xk[i];
     T c0 = c[i], c1 = c[n_int + i], c2 = c[2 * n_int + i], c3 = c[3 * n_int + i];
     dval = (T(3) * c0 * d + T(2) * c1) * d + c2;
     return ((c0 * d + c1) * d + c2) * d + c3;
+}
+
+template <typename T>
+__device__ __forceinline__ T pchip_eval(int n_int, const T *__restrict__ c, const T *__restrict__ xk, T x, T &dval) {
+    int near = 0;
+    return pchip_eval(n_int, c, xk, x, dval, near);
 }
 
 // mu(|H|) and dmu/d|H| of the B-spline permeability in x = log10|H| (fem_c/ctools.c:206-346).

@@ -353,3 +353,55 @@ def test_overlapping_passes_give_one_answer(tets, precision, monkeypatch):
         s._newton = None
     assert out[0][1] == out[1][1] == out[2][1] > 10
     assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][0], out[2][0])
+
+
+@pytest.mark.parametrize("diluted", [False, True])
+@pytest.mark.parametrize("n_iron", [1, 63, 65, 400])
+@pytest.mark.parametrize("order", [3, 4, 6])
+def test_point_sums_in_their_own_launch(order, n_iron, diluted):
+    """Many quadrature points: the launch that sums them, four lanes per element, behind every set of
+    wanted outputs, against the kernels that do it element by element and add into the CSR."""
+    msh = M.window_frame_mesh(2000, jitter=0.15, seed=3)
+    dom = np.full(msh.num_elements, M.TAG_AIR, dtype=np.int32)
+    dom[100:100 + n_iron] = M.TAG_IRON
+    msh.elem_domain = dom
+    tags, mats = [M.TAG_AIR, M.TAG_IRON], [S.ConstantReluctance(NU0), MAT.atan_reluctance()]
+    if diluted:
+        A = S.CurlCurlAssemblerDiluted(msh, tags, mats, [None, MAT.Dilution(0.0, 0.30, 0.35, 0.75, 0.02, 0.40, 0.45, 0.80,
+                                                                                z_pos=-0.25, z_len=0.5)])
+    else:
+        A = S.CurlCurlAssembler(msh, tags, mats)
+    rng = np.random.default_rng(order)
+    x = rng.normal(0, 2e-3, msh.num_dofs)
+    sf = [np.zeros((0, 3)), rng.normal(0, 0.5, (n_iron * A.tables(order).nq, 3))]
+    T = A.assemble_device(x, order, sf, method="atomic", K=True, J=True, dK=True, rhs=True, F=True)
+    for wanted in ("K,dK,J,rhs,F", "J,F", "dK", "K,rhs", "rhs,F"):
+        kw = {k: k in wanted.split(",") for k in ("K", "dK", "J", "rhs", "F")}
+        R = A.assemble_device(x, order, sf, method="rows", **kw)
+        for key in wanted.split(","):
+            if key in ("rhs", "F"):
+                assert rel_max(R[key].cpu().numpy(), T[key].cpu().numpy()) < 1e-12
+            else:
+                _assert_rows_close(R[key], T[key], A.pattern.row_ptr, 1e-12)
+
+
+@pytest.mark.parametrize("order", [1, 2, 3, 4, 6])
+def test_tensor_kernel_point_loads(order):
+    """Element tensors with points loaded in pairs (even counts), with a single one left over (odd
+    counts) and with one point only: F and J x against the CSR system's."""
+    import torch
+
+    s = _window_solver(900)
+    s.quad_order = order
+    eng = s.newton_engine()
+    x = torch.from_numpy(np.random.default_rng(order).normal(0, 1e-3, eng.n)).cuda()
+    v = torch.from_numpy(np.random.default_rng(9).normal(0, 1.0, eng.n)).cuda()
+    free = eng.free_mask.bool()
+    v[~free] = 0.0
+    F = eng.assemble_tensors(x, "fp64", torch.empty_like(x))
+    Jv = eng.jacobian_apply(v, torch.zeros_like(v))
+    out = s.curl_curl_factory.assemble_device(x, order, s.compute_source_fields(), K=False, J=True, rhs=False, F=True)
+    ref = out["pattern"].to_torch(out["J"]).matmul(v)
+    # sums of a few tens of element terms of the same magnitude in another order
+    for a, b in ((F[free], out["F"][:eng.n][free]), (Jv[free], ref[free])):
+        assert float((a - b).abs().max()) <= 1e-12 * float(b.abs().max())
