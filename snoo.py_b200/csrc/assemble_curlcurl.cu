@@ -26,6 +26,7 @@
 // gathered coordinates and x (mostly cache hits for a locality-ordered mesh).
 #include "snp_common.cuh"
 #include "snp_internal.cuh"
+#include "snp_overlap.cuh"
 
 namespace snp {
 
@@ -402,6 +403,7 @@ template <bool DIL>
 __global__ void __launch_bounds__(kPointBlock, DIL ? 2 : 3)
     k_point_sums(CurlArgs a, int quad_stride_ctab, double *sums) {
     extern __shared__ double sm[];
+    allow_next_kernel();
     const ElemTables T = stage_tables(a, quad_stride_ctab, sm);
     constexpr int kElems = kPointBlock / kPointLanes;
     const int sub = threadIdx.x % kPointLanes;
@@ -423,6 +425,7 @@ __global__ void __launch_bounds__(kPointBlock, DIL ? 2 : 3)
         for (int t = 0; t < 10; ++t)
             if (t % kPointLanes == sub && mine < a.n_elems) at[t] = v[t];
     }
+    wait_for_previous_kernel();
 }
 
 // Element values of the two-phase assembly with an element's values side by side (PackedTerms).
@@ -434,7 +437,9 @@ template <bool HAS_BS, int NQ, bool DIL, bool PRE>
 __global__ void __launch_bounds__(kBlock)
     k_curlcurl_packed(CurlArgs a, int quad_stride_ctab, int table_doubles, PackedTerms out) {
     extern __shared__ double sm[];
+    allow_next_kernel();
     const ElemTables T = stage_tables(a, quad_stride_ctab, sm);
+    if constexpr (PRE) wait_for_previous_kernel();
     double *tile = sm + table_doubles;                              // K or J, then F and r
     double *tile_d = tile + kBlock * kPackPairs;                    // dK
     const int nq = NQ > 0 ? NQ : a.nq;
@@ -481,6 +486,7 @@ __global__ void __launch_bounds__(kBlock)
             __syncthreads();
         }
     }
+    if constexpr (!PRE) wait_for_previous_kernel();
 }
 
 // Reduced rhs only (compute_rhs_Hcurl_red, fem_c/ctools.c:1390-1497).
@@ -754,6 +760,7 @@ template <bool HAS_BS, int NQ, typename TT, bool DIL>
 __global__ void __launch_bounds__(kBlock)
     k_curlcurl_tensor(CurlArgs a, int quad_stride_ctab, TT *__restrict__ T) {
     extern __shared__ double sm[];
+    allow_next_kernel();
     const SmemLayout L = smem_layout(a.n_orient, a.nq, a.n_int);
     double *s_ctab = sm + L.off_ctab;
     double *s_dphi = sm + L.off_dphi;
@@ -781,6 +788,7 @@ __global__ void __launch_bounds__(kBlock)
 
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < a.n_elems; e += (int64_t)gridDim.x * blockDim.x)
         tensor_element<HAS_BS, NQ, TT, DIL>(a, e, s_ctab, s_dphi, s_w, s_phi, s_relc, s_relx, wsum, T);
+    wait_for_previous_kernel();
 }
 
 // Batched element tensors: a grid of resident blocks walks the work items (runs of one
@@ -847,7 +855,9 @@ int launch_tensor_t(const CurlArgs &a, TT *T, cudaStream_t st, size_t smem, int 
     if (a.n_elems == 0) return SNP_OK;
     auto kern = k_curlcurl_tensor<HAS_BS, NQ, TT, DIL>;
     if (smem > 48 * 1024) SNP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<wave_grid(kern, a.n_elems, kBlock, smem), kBlock, smem, st>>>(a, qstride, T);
+    // materials write disjoint elements, so the next one's blocks fill the SMs behind this one's
+    // last ones: Newton steps of 35k tets 1630 -> 1511 us, of 290k (mixed) 4515 -> 4436
+    launch_overlapping(a.beside, kern, wave_grid(kern, a.n_elems, kBlock, smem), kBlock, smem, st, a, qstride, T);
     SNP_LAUNCH_CHECK();
     return SNP_OK;
 }
@@ -893,10 +903,12 @@ int launch_packed_pre(const CurlArgs &a, cudaStream_t st, int qstride, const Pac
         if (psmem > 48 * 1024)
             SNP_CUDA_TRY(cudaFuncSetAttribute(points, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psmem));
         double *sums = out.J ? out.J : out.K ? out.K : out.D;
-        points<<<wave_grid(points, a.n_elems * kPointLanes, kPointBlock, psmem), kPointBlock, psmem, st>>>(a, qstride, sums);
+        launch_overlapping(a.beside, points, wave_grid(points, a.n_elems * kPointLanes, kPointBlock, psmem), kPointBlock,
+                           psmem, st, a, qstride, sums);
         SNP_LAUNCH_CHECK();
     }
-    kern<<<wave_grid(kern, a.n_elems, kBlock, smem), kBlock, smem, st>>>(a, qstride, tables, out);
+    launch_overlapping(PRE || a.beside, kern, wave_grid(kern, a.n_elems, kBlock, smem), kBlock, smem, st, a, qstride,
+                       tables, out);
     SNP_LAUNCH_CHECK();
     return SNP_OK;
 }
@@ -908,7 +920,7 @@ int launch_packed_t(const CurlArgs &a, cudaStream_t st, int qstride, const Packe
         // 4 and 5 points have unrolled element kernels; the next rule has 27, where the separate
         // launch already wins: 49 against 63 us (in the element kernel) at 300k tets, 18 against 31 at
         // 20k, 144 against 160 at 1.1M; 64 points 80 against 123, 27 against 63, 235 against 321
-        if (a.nq >= 8 && (out.J || out.K || out.D)) return launch_packed_pre<HAS_BS, NQ, DIL, true>(a, st, qstride, out);
+        if (a.nq >= kManyPoints && (out.J || out.K || out.D)) return launch_packed_pre<HAS_BS, NQ, DIL, true>(a, st, qstride, out);
     }
     return launch_packed_pre<HAS_BS, NQ, DIL, false>(a, st, qstride, out);
 }

@@ -387,14 +387,22 @@ int launch_curlcurl_system(const snp_pattern *pat, const CurlArgs *mats, int n_m
     all.J = take(nd.j, kPackPairs);
     all.F = take(o.F != nullptr, 6);
     all.R = take(o.rhs != nullptr, 6);
+    bool beside = false;
     for (int m = 0; m < n_mats; ++m) {
-        const CurlArgs &a = mats[m];
+        CurlArgs a = mats[m];
         if (a.n_elems == 0) continue;
+        a.beside = beside;
         PackedTerms out = all;
         // constant reluctance: dK = 0 (nu' = 0)
         if (out.D && a.n_int < 0 && zero_dk.n < 2 && zero_dk.add(a.t_offset, a.t_offset + a.n_elems)) out.D = nullptr;
         if (a.Bs == nullptr) out.R = nullptr;
-        if (out.K || out.D || out.J || out.F || out.R) SNP_TRY(launch_curlcurl_packed(a, out, st));
+        if (out.K || out.D || out.J || out.F || out.R) {
+            SNP_TRY(launch_curlcurl_packed(a, out, st));
+            // the next material's element kernel starts while this one's points are bound by
+            // latency (183 -> 175 us a call at 150k tets diluted, 250 -> 235 at 300k); beside a kernel
+            // bound by its streams it gains nothing (485 -> 485-510 us at 1.16M tets, 4 points)
+            beside = a.Bs != nullptr && a.nq >= kManyPoints;
+        }
     }
     r.nnz = pat->nnz;
     r.cptr = pat->cptr.p;

@@ -28,6 +28,7 @@
 #include "snp_elem.cuh"
 #include "snp_internal.cuh"
 #include "snp_krylov.cuh"
+#include "snp_overlap.cuh"
 #include "snp_reduce.cuh"
 
 namespace snp {
@@ -177,11 +178,11 @@ Chat<TT> chat_of(const ElemTopology &top) {
 // may be read before, nothing may be written; what the other passes write (G, R, Y, the CG state) is
 // read with plain loads, since a read-only path's data may not change while the kernel is resident.
 __device__ __forceinline__ void pass_begins() {
-    cudaGridDependencySynchronize();
+    wait_for_previous_kernel();
 }
 
 __device__ __forceinline__ void next_pass_may_start(int early) {
-    if (early) cudaTriggerProgrammaticLaunchCompletion();
+    if (early) allow_next_kernel();
 }
 
 // u_e of the element's directions pk (signs applied): edges 0-2 and 3-5 summed apart
@@ -1534,25 +1535,6 @@ int ElemPcg<TT>::reserve(int32_t n_, int64_t ne_) {
     return SNP_OK;
 }
 
-namespace {
-// Launch that may overlap the end of the previous kernel on the stream (pass_begins); errors are
-// left for the caller's launch check.
-template <typename... P, typename... A>
-void launch_pass(void (*kern)(P...), int grid, int block, size_t smem, cudaStream_t s, const A &...args) {
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3((unsigned)block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    (void)cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
-}
-}  // namespace
-
 template <typename TT>
 int ElemPcg<TT>::launch_iteration(const ElemTopology &top, const TT *T, const uint8_t *free_mask,
                                   const BlockPlan *plan, cudaStream_t s, int use_cond,
@@ -1568,18 +1550,19 @@ int ElemPcg<TT>::launch_iteration(const ElemTopology &top, const TT *T, const ui
     // 12.5, 18.5 and 24.7 without, 13.3, 19.2 and 25.5 with (12.7, 18.9 and 24.9 not overlapping).
     const int early = sizeof(TT) == 4 || staged ? 1 : 0;
     if constexpr (sizeof(TT) == 4)
-        launch_pass(k_epass1_pair<TT>, wave_grid(k_epass1_pair<TT>, 2 * ne, kEBlock), kEBlock, 0, s, ne, top.edof.p,
-                    top.pos.p, T, chat_ptr<TT>(top), G.p, Y.p, st.p, part.p, early);
+        launch_overlapping(true, k_epass1_pair<TT>, wave_grid(k_epass1_pair<TT>, 2 * ne, kEBlock), kEBlock, 0, s, ne,
+                           top.edof.p, top.pos.p, T, chat_ptr<TT>(top), G.p, Y.p, st.p, part.p, early);
     else
-        launch_pass(k_epass1<TT>, wave_grid(k_epass1<TT>, ne, kEBlock), kEBlock, 0, s, ne, top.edof.p, top.pos.p, T, ch,
-                    G.p, Y.p, st.p, part.p, early);
+        launch_overlapping(true, k_epass1<TT>, wave_grid(k_epass1<TT>, ne, kEBlock), kEBlock, 0, s, ne, top.edof.p,
+                           top.pos.p, T, ch, G.p, Y.p, st.p, part.p, early);
     SNP_LAUNCH_CHECK();
     // the staged DoF pass in float64 from four tiles per block on: 39.5 against 40.3 us per iteration
     // at 600k tets, 69.9 against 74.7 at 1.16M; below, 25.7 against 25.4 at 287k and 16.5 against
     // 15.7 at 100k (float32: 52.4 against 53.1 at 1.16M, 13.3 against 13.3 at 38k)
     if (plan && !staged) {
-        launch_pass(k_epass2_direct<TT>, wave_grid(k_epass2_direct<TT>, n, kEBlock), kEBlock, 0, s, n, free_mask,
-                    top.inc_ptr.p, Y.p, plan->meta, plan->binv, G.p, R.p, st.p, part.p, use_cond, cond, early);
+        launch_overlapping(true, k_epass2_direct<TT>, wave_grid(k_epass2_direct<TT>, n, kEBlock), kEBlock, 0, s, n,
+                           free_mask, top.inc_ptr.p, Y.p, plan->meta, plan->binv, G.p, R.p, st.p, part.p, use_cond,
+                           cond, early);
         SNP_LAUNCH_CHECK();
         return SNP_OK;
     }
@@ -1596,10 +1579,11 @@ int ElemPcg<TT>::launch_iteration(const ElemTopology &top, const TT *T, const ui
         a.G = G.p;
         a.R = R.p;
         const size_t smem = dof_pass_smem<TT>();
-        launch_pass(k_epass2_bj<TT>, staged_grid, kDofThreads, smem, s, a, st.p, part.p, use_cond, cond, early);
+        launch_overlapping(true, k_epass2_bj<TT>, staged_grid, kDofThreads, smem, s, a, st.p, part.p, use_cond, cond,
+                           early);
     } else {
-        launch_pass(k_epass2<TT>, wave_grid(k_epass2<TT>, n, kEBlock), kEBlock, 0, s, n, free_mask, top.inc_ptr.p, Y.p,
-                    G.p, R.p, D.p, st.p, part.p, use_cond, cond, early);
+        launch_overlapping(true, k_epass2<TT>, wave_grid(k_epass2<TT>, n, kEBlock), kEBlock, 0, s, n, free_mask,
+                           top.inc_ptr.p, Y.p, G.p, R.p, D.p, st.p, part.p, use_cond, cond, early);
     }
     SNP_LAUNCH_CHECK();
     return SNP_OK;

@@ -94,6 +94,7 @@ struct CurlArgs {
     const double *w;      // [Q]
     int32_t nq;
     const double *x;
+    bool beside;          // may run beside the launch right before it (another material of the system)
     const double *Bs;     // [n_elems][Q][3] or null
     int32_t n_int;
     const double *rel_c;
@@ -198,6 +199,7 @@ int launch_curlcurl_rows(const snp_pattern *pat, const double *terms, const Term
 // Element values side by side (the assembly of whole systems, launch_curlcurl_system): value q of
 // element e at X[e * 21 + q] for the upper triangles of K, dK and J = K + dK, at X[e * 6 + k] for
 // the residual and reduced-rhs terms; null: not wanted.
+constexpr int kManyPoints = 8;  // from here on the points of an element have a launch of their own
 constexpr int kPackPairs = 21;
 constexpr int kPackPairs4 = 10;  // of an element with 4 DoFs
 struct PackedTerms {

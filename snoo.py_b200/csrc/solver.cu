@@ -354,6 +354,7 @@ struct snp_solver {
     // Element tensors (float64 or float32), diag(J) and F = K x - rhs - rhs_extra at x.
     int assemble_elem(const double *x, bool f32, double *Fv) {
         j_valid[f32 ? 1 : 0] = 1;
+        bool beside = false;  // an element kernel of this system is the last launch
         for (auto &m : mats) {
             snp::CurlArgs a{};
             a.n_elems = m->count;
@@ -380,8 +381,12 @@ struct snp_solver {
             a.t_offset = m->offset;
             a.Fe = Fe.p;
             a.De = De.p;
+            a.beside = beside;
             SNP_TRY(snp::launch_curlcurl_tensor(a, stream));
-            if (m->count) ++launches;
+            if (m->count) {
+                ++launches;
+                beside = true;
+            }
         }
         SNP_TRY(snp::elem_sum_to_dofs(etop, Fe.p, De.p, has_extra ? rhs_extra.p : nullptr, Fv, Jdiag.p, stream));
         ++launches;
