@@ -279,6 +279,111 @@ __global__ void __launch_bounds__(kEBlock, 3)
     }
 }
 
+constexpr int kTileElems = 256, kTilePairs = 3;
+
+// The same pass over tiles of consecutive elements (TilePlan): a tile's distinct DoFs are gathered
+// once, its terms meet in shared memory and each DoF's sum leaves as one slot value, so an element
+// costs 2.3 gathers and 2.3 scattered stores instead of six and six, and the DoF pass reads 2.3
+// slot values per element instead of six.  Bound by the latency of a tile's two barriers and by
+// its streams (T 48 B, places and lists 24 B, pairs 28 B an element) at 32 warps an SM; all words of
+// a tile are requested at its start.  Per iteration at 1.16M tets 67.2 -> 60.1 us, 600k 38.7 -> 34.9,
+// 450k 31.1 -> 29.5; with the pairs' words requested where they are used 81.5 (1.16M), with three
+// blocks an SM 68.4, tiles of 128 elements 62.0.
+__global__ void __launch_bounds__(kTileElems, 4)
+    k_epass1_tile(int64_t ne, int32_t tiles, const int32_t *__restrict__ tile_ptr, const int32_t *__restrict__ dof,
+                  const int32_t *__restrict__ slot, const uint32_t *__restrict__ terms,
+                  const uint16_t *__restrict__ list, const uint16_t *__restrict__ place, const double *__restrict__ T,
+                  const Chat<double> ch, const DofPair<double> *G, double *Y, PcgState *st, double *part, int early) {
+    constexpr int TE = kTileElems, kJ = kTilePairs;  // kJ pairs per thread, their words requested ahead
+    __shared__ double s_p[6 * TE], s_t[6 * TE], sh[32];
+    __shared__ __align__(16) uint32_t s_l[3 * TE];
+    const uint16_t *const s_list = reinterpret_cast<const uint16_t *>(s_l);
+    const int tid = threadIdx.x;
+    int32_t tile = blockIdx.x;
+    int32_t p0 = 0, n = 0, d[kJ];
+    auto open_tile = [&](int32_t at) {
+        p0 = __ldg(tile_ptr + at);
+        n = __ldg(tile_ptr + at + 1) - p0;
+#pragma unroll
+        for (int i = 0; i < kJ; ++i) d[i] = tid + i * TE < n ? __ldcs(dof + p0 + tid + i * TE) : 0;
+    };
+    if (tile < tiles) open_tile(tile);
+    pass_begins();
+    if (st->done) return;
+    const double beta = st->beta;
+    double dot = 0.0;
+#pragma unroll 1
+    for (; tile < tiles; tile += gridDim.x) {
+        const int64_t e = (int64_t)tile * TE + tid;
+        const bool here = e < ne;
+        DofPair<double> w[kJ];
+#pragma unroll
+        for (int i = 0; i < kJ; ++i)
+            if (tid + i * TE < n) w[i] = G[d[i]];
+        double t[6];
+        uint32_t at[6], ls[3], tw[kJ];
+        int32_t ys[kJ];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            t[k] = here ? __ldcs(T + eslot(e, k)) : 0.0;
+            at[k] = here ? __ldcs(place + ((int64_t)tile * 6 + k) * TE + tid) : 0u;
+        }
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+            ls[i] = __ldcs(reinterpret_cast<const uint32_t *>(list) + (int64_t)tile * (3 * TE) + i * TE + tid);
+#pragma unroll
+        for (int i = 0; i < kJ; ++i) {
+            const bool in = tid + i * TE < n;
+            tw[i] = in ? __ldcs(terms + p0 + tid + i * TE) : 0u;
+            ys[i] = in ? __ldcs(slot + p0 + tid + i * TE) : 0;
+        }
+#pragma unroll
+        for (int i = 0; i < kJ; ++i)
+            if (tid + i * TE < n) s_p[tid + i * TE] = pnext(beta, w[i].b, w[i].a);
+        for (int j = tid + kJ * TE; j < n; j += TE) {
+            const DofPair<double> g = G[__ldcs(dof + p0 + j)];
+            s_p[j] = pnext(beta, g.b, g.a);
+        }
+        __syncthreads();
+        double pk[6], u0, u1, u2, v0, v1, v2;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            pk[k] = s_p[at[k] & 0x7fffu];
+            if (at[k] & 0x8000u) pk[k] = -pk[k];
+        }
+        element_u(pk, ch, u0, u1, u2);
+        apply_tensor(t, u0, u1, u2, v0, v1, v2);
+        if (here) dot += u0 * v0 + u1 * v1 + u2 * v2;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) s_t[k * TE + tid] = edge_term(ch.c, k, (at[k] & 0x8000u) != 0, v0, v1, v2);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) s_l[i * TE + tid] = ls[i];
+        const int32_t q0 = p0, m = n;
+        if (tile + (int32_t)gridDim.x < tiles) open_tile(tile + gridDim.x);
+        __syncthreads();
+        auto leave = [&](uint32_t word, int32_t y) {
+            const int f = (int)(word & 0xffffu), c = (int)(word >> 16);
+            double sum = 0.0;
+            for (int i = 0; i < c; ++i) sum += s_t[s_list[f + i]];
+            Y[y] = sum;
+        };
+#pragma unroll
+        for (int i = 0; i < kJ; ++i)
+            if (tid + i * TE < m) leave(tw[i], ys[i]);
+        for (int j = tid + kJ * TE; j < m; j += TE) leave(__ldcs(terms + q0 + j), __ldcs(slot + q0 + j));
+    }
+    next_pass_may_start(early);
+    dot = block_sum(dot, sh);
+    if (tid == 0) part[blockIdx.x] = dot;
+    if (last_block(&st->counter)) {
+        const double pq = reduce_parts(part, gridDim.x, 1, 0, sh);
+        if (tid == 0) {
+            st->pq = pq;
+            st->alpha = st->rz / pq;
+        }
+    }
+}
+
 template <typename TT>
 __device__ __forceinline__ void load_chat(TT *sc, const TT *chat) {
     if (threadIdx.x < 18) sc[threadIdx.x] = chat[threadIdx.x];
@@ -1367,6 +1472,139 @@ const float *chat_ptr<float>(const ElemTopology &top) {
 
 }  // namespace
 
+// ---------------------------------------------------------------- tile plan
+
+namespace {
+
+constexpr int64_t kTileMinElems = 300000;
+
+// head[t] = 1 where entry t of the DoF-ordered incidence list starts a DoF's entries in a tile
+__global__ void k_tile_heads(int64_t m, int te, const int32_t *__restrict__ inc, const int32_t *__restrict__ edof,
+                             int32_t *__restrict__ head) {
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < m; t += (int64_t)gridDim.x * blockDim.x) {
+        const uint32_t u = (uint32_t)inc[t] & ~kSignBit, v = t ? (uint32_t)inc[t - 1] & ~kSignBit : 0u;
+        const bool same = t && (u >> 3) / te == (v >> 3) / te &&
+                          ((edof[eslot(u >> 3, (int)(u & 7u))] ^ edof[eslot(v >> 3, (int)(v & 7u))]) & ~kSignBit) == 0;
+        head[t] = same ? 0 : 1;
+    }
+}
+
+// slot s: its tile and first entry; first slot of every DoF (scan: inclusive sum of head)
+__global__ void k_tile_slots(int64_t m, int te, int32_t n, const int32_t *__restrict__ inc,
+                             const int32_t *__restrict__ inc_ptr, const int32_t *__restrict__ head,
+                             const int32_t *__restrict__ scan, int32_t *__restrict__ key, int32_t *__restrict__ val,
+                             int32_t *__restrict__ first, int32_t *__restrict__ slot_ptr) {
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x, t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    for (int64_t t = t0; t < m; t += stride)
+        if (head[t]) {
+            const int32_t s = scan[t] - 1;
+            key[s] = (int32_t)((((uint32_t)inc[t] & ~kSignBit) >> 3) / te);
+            val[s] = s;
+            first[s] = (int32_t)t;
+        }
+    for (int64_t i = t0; i <= n; i += stride) {
+        const int32_t t = inc_ptr[i];
+        slot_ptr[i] = t < m ? scan[t] - head[t] : scan[m - 1];
+    }
+    if (t0 == 0) first[scan[m - 1]] = (int32_t)m;
+}
+
+// pairs in tile order: number of terms, first pair of every tile
+__global__ void k_tile_lengths(int32_t pairs, int32_t tiles, const int32_t *__restrict__ key,
+                               const int32_t *__restrict__ slot, const int32_t *__restrict__ first,
+                               int32_t *__restrict__ len, int32_t *__restrict__ tile_ptr) {
+    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < pairs; p += (int64_t)gridDim.x * blockDim.x) {
+        const int32_t s = slot[p];
+        len[p] = first[s + 1] - first[s];
+        if (p == 0 || key[p] != key[p - 1]) tile_ptr[key[p]] = (int32_t)p;
+        if (p == 0) tile_ptr[tiles] = pairs;
+    }
+}
+
+__global__ void k_tile_fill(int32_t pairs, int te, const int32_t *__restrict__ key, const int32_t *__restrict__ slot,
+                            const int32_t *__restrict__ first, const int32_t *__restrict__ tile_ptr,
+                            const int32_t *__restrict__ at, const int32_t *__restrict__ inc,
+                            const int32_t *__restrict__ edof, int32_t *__restrict__ dof, uint32_t *__restrict__ terms,
+                            uint16_t *__restrict__ list, uint16_t *__restrict__ place) {
+    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < pairs; p += (int64_t)gridDim.x * blockDim.x) {
+        const int32_t s = slot[p], tile = key[p], j = (int32_t)p - tile_ptr[tile];
+        const int32_t t0 = first[s], c = first[s + 1] - t0;
+        const int64_t base = (int64_t)tile * 6 * te;  // every tile before it is full
+        const int32_t rel = (int32_t)(at[p] - base);
+        for (int i = 0; i < c; ++i) {
+            const uint32_t w = (uint32_t)inc[t0 + i], u = w & ~kSignBit;
+            const int k = (int)(u & 7u), l = (int)((u >> 3) % (uint32_t)te);
+            list[base + rel + i] = (uint16_t)(k * te + l);
+            place[base + (int64_t)k * te + l] = (uint16_t)((uint32_t)j | ((w & kSignBit) ? 0x8000u : 0u));
+            if (i == 0) dof[p] = (int32_t)((uint32_t)edof[eslot(u >> 3, k)] & ~kSignBit);
+        }
+        terms[p] = (uint32_t)rel | (uint32_t)c << 16;
+    }
+}
+
+int build_tile_plan(ElemTopology &top, cudaStream_t s) {
+    TilePlan &P = top.tile;
+    P.te = 0;
+    // below, the chain of a tile's phases costs what it saves: 300k tets 23.3 against 23.6 us per
+    // iteration, 100k 16.4 against 15.7, 38k 13.7 against 12.4
+    if (top.n_elems < kTileMinElems) return SNP_OK;
+    const int64_t m = 6 * top.n_elems;
+    const int te = kTileElems;
+    P.tiles = (int32_t)((top.n_elems + te - 1) / te);
+    DevBuf<int32_t> head, scan;
+    SNP_TRY(head.alloc(m));
+    SNP_TRY(scan.alloc(m));
+    const int g = stride_grid(m, 256, 8);
+    k_tile_heads<<<g, 256, 0, s>>>(m, te, top.inc.p, top.edof.p, head.p);
+    SNP_LAUNCH_CHECK();
+    DevBuf<unsigned char> temp;
+    size_t tb = 0;
+    SNP_CUDA_TRY(cub::DeviceScan::InclusiveSum(nullptr, tb, head.p, scan.p, (int)m, s));
+    SNP_TRY(temp.alloc(tb));
+    SNP_CUDA_TRY(cub::DeviceScan::InclusiveSum(temp.p, tb, head.p, scan.p, (int)m, s));
+    int32_t pairs = 0;
+    SNP_CUDA_TRY(cudaMemcpyAsync(&pairs, scan.p + (m - 1), sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+    SNP_CUDA_TRY(cudaStreamSynchronize(s));
+    // an element order with few shared edges inside a tile (meshes in arbitrary order) gains
+    // nothing; up to here a tile's pairs fit kTilePairs per thread (2.3 per element, 0.39 of the
+    // terms, in the window frame's order)
+    if (pairs > kTilePairs * top.n_elems) return SNP_OK;
+    DevBuf<int32_t> key, key2, val, first, len, at;
+    for (DevBuf<int32_t> *b : {&key, &key2, &val, &P.slot, &len, &at, &P.dof}) SNP_TRY(b->alloc(pairs));
+    SNP_TRY(first.alloc((size_t)pairs + 1));
+    SNP_TRY(P.terms.alloc(pairs));
+    SNP_TRY(P.tile_ptr.alloc((size_t)P.tiles + 1));
+    SNP_TRY(P.list.alloc((size_t)P.tiles * 6 * te));
+    SNP_TRY(P.place.alloc((size_t)P.tiles * 6 * te));
+    SNP_TRY(P.slot_ptr.alloc((size_t)top.n + 1));
+    k_tile_slots<<<g, 256, 0, s>>>(m, te, top.n, top.inc.p, top.inc_ptr.p, head.p, scan.p, key.p, val.p, first.p,
+                                   P.slot_ptr.p);
+    SNP_LAUNCH_CHECK();
+    int bits = 1;
+    while (bits < 31 && ((int64_t)1 << bits) < P.tiles) ++bits;
+    cub::DoubleBuffer<int32_t> dk(key.p, key2.p), dv(val.p, P.slot.p);
+    size_t ts = 0, tx = 0;
+    SNP_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, ts, dk, dv, pairs, 0, bits, s));
+    SNP_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tx, len.p, at.p, pairs, s));
+    if (ts > tb || tx > tb) SNP_TRY(temp.alloc(ts > tx ? ts : tx));
+    SNP_CUDA_TRY(cub::DeviceRadixSort::SortPairs(temp.p, ts, dk, dv, pairs, 0, bits, s));
+    if (dv.Current() != P.slot.p)
+        SNP_CUDA_TRY(cudaMemcpyAsync(P.slot.p, dv.Current(), sizeof(int32_t) * (size_t)pairs, cudaMemcpyDeviceToDevice, s));
+    const int gp = stride_grid(pairs, 256, 8);
+    k_tile_lengths<<<gp, 256, 0, s>>>(pairs, P.tiles, dk.Current(), P.slot.p, first.p, len.p, P.tile_ptr.p);
+    SNP_LAUNCH_CHECK();
+    SNP_CUDA_TRY(cub::DeviceScan::ExclusiveSum(temp.p, tx, len.p, at.p, pairs, s));
+    k_tile_fill<<<gp, 256, 0, s>>>(pairs, te, dk.Current(), P.slot.p, first.p, P.tile_ptr.p, at.p, top.inc.p, top.edof.p,
+                                   P.dof.p, P.terms.p, P.list.p, P.place.p);
+    SNP_LAUNCH_CHECK();
+    SNP_CUDA_TRY(cudaStreamSynchronize(s));
+    P.pairs = pairs;
+    P.te = te;
+    return SNP_OK;
+}
+
+}  // namespace
+
 // ---------------------------------------------------------------- topology
 
 int build_elem_topology(ElemTopology &top, int32_t n, const ElemBlock *blocks, int n_blocks, const double *ctab_host,
@@ -1451,6 +1689,7 @@ int build_elem_topology(ElemTopology &top, int32_t n, const ElemBlock *blocks, i
     SNP_REQUIRE(hbad == 0, "element topology: a DoF index or orientation is out of range");
     top.n_elems = ne;
     top.n = n;
+    SNP_TRY(build_tile_plan(top, s));
     *usable = true;
     return SNP_OK;
 }
@@ -1468,13 +1707,13 @@ int build_block_plan(BlockPlan &plan, const ElemTopology &top, const uint8_t *fr
     SNP_TRY(plan.tile_inc.alloc((size_t)tiles + 1));
     SNP_TRY(plan.tile_m.alloc((size_t)tiles + 1));
     SNP_CUDA_TRY(cudaMemsetAsync(wide.p, 0, sizeof(int), s));
-    k_plan_tiles<<<tiles, kBjTile, 0, s>>>(n, tiles, meta, top.inc_ptr.p, cnt.p, plan.tile_inc.p);
+    k_plan_tiles<<<tiles, kBjTile, 0, s>>>(n, tiles, meta, top.slot_ptr64(), cnt.p, plan.tile_inc.p);
     SNP_LAUNCH_CHECK();
     size_t tb = 0;
     SNP_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb, cnt.p, plan.tile_m.p, tiles + 1, s));
     SNP_TRY(temp.alloc(tb));
     SNP_CUDA_TRY(cub::DeviceScan::ExclusiveSum(temp.p, tb, cnt.p, plan.tile_m.p, tiles + 1, s));
-    k_plan_words<<<tiles, kBjTile, 0, s>>>(n, meta, free_mask, top.inc_ptr.p, plan.word.p, wide.p);
+    k_plan_words<<<tiles, kBjTile, 0, s>>>(n, meta, free_mask, top.slot_ptr64(), plan.word.p, wide.p);
     SNP_LAUNCH_CHECK();
     int32_t total = 0;
     int hw = 0;
@@ -1536,10 +1775,22 @@ int ElemPcg<TT>::reserve(int32_t n_, int64_t ne_) {
 }
 
 template <typename TT>
+void ElemPcg<TT>::launch_tile_pass(const ElemTopology &top, const double *T, int early, cudaStream_t s) {
+    if constexpr (sizeof(TT) == 8) {
+        const TilePlan &P = top.tile;
+        const Chat<double> ch = chat_of<double>(top);
+        launch_overlapping(true, k_epass1_tile, wave_grid(k_epass1_tile, (int64_t)P.tiles * kTileElems, kTileElems),
+                           kTileElems, 0, s, ne, P.tiles, P.tile_ptr.p, P.dof.p, P.slot.p, P.terms.p, P.list.p, P.place.p,
+                           T, ch, G.p, Y.p, st.p, part.p, early);
+    }
+}
+
+template <typename TT>
 int ElemPcg<TT>::launch_iteration(const ElemTopology &top, const TT *T, const uint8_t *free_mask,
                                   const BlockPlan *plan, cudaStream_t s, int use_cond,
                                   cudaGraphConditionalHandle cond) {
     const Chat<TT> ch = chat_of<TT>(top);
+    const int32_t *slot_ptr = sizeof(TT) == 8 ? top.slot_ptr64() : top.inc_ptr.p;
     const int staged_grid =
         plan ? wave_grid(k_epass2_bj<TT>, (int64_t)plan->tiles * kDofThreads, kDofThreads, dof_pass_smem<TT>()) : 0;
     const bool staged = plan && sizeof(TT) == 8 && plan->tiles >= 4 * staged_grid;
@@ -1552,6 +1803,8 @@ int ElemPcg<TT>::launch_iteration(const ElemTopology &top, const TT *T, const ui
     if constexpr (sizeof(TT) == 4)
         launch_overlapping(true, k_epass1_pair<TT>, wave_grid(k_epass1_pair<TT>, 2 * ne, kEBlock), kEBlock, 0, s, ne,
                            top.edof.p, top.pos.p, T, chat_ptr<TT>(top), G.p, Y.p, st.p, part.p, early);
+    else if (top.tile.te)
+        launch_tile_pass(top, T, early, s);
     else
         launch_overlapping(true, k_epass1<TT>, wave_grid(k_epass1<TT>, ne, kEBlock), kEBlock, 0, s, ne, top.edof.p,
                            top.pos.p, T, ch, G.p, Y.p, st.p, part.p, early);
@@ -1561,7 +1814,7 @@ int ElemPcg<TT>::launch_iteration(const ElemTopology &top, const TT *T, const ui
     // 15.7 at 100k (float32: 52.4 against 53.1 at 1.16M, 13.3 against 13.3 at 38k)
     if (plan && !staged) {
         launch_overlapping(true, k_epass2_direct<TT>, wave_grid(k_epass2_direct<TT>, n, kEBlock), kEBlock, 0, s, n,
-                           free_mask, top.inc_ptr.p, Y.p, plan->meta, plan->binv, G.p, R.p, st.p, part.p, use_cond,
+                           free_mask, slot_ptr, Y.p, plan->meta, plan->binv, G.p, R.p, st.p, part.p, use_cond,
                            cond, early);
         SNP_LAUNCH_CHECK();
         return SNP_OK;
@@ -1573,7 +1826,7 @@ int ElemPcg<TT>::launch_iteration(const ElemTopology &top, const TT *T, const ui
         a.word = plan->word.p;
         a.tile_inc = plan->tile_inc.p;
         a.tile_m = plan->tile_m.p;
-        a.inc_ptr = plan->wide ? top.inc_ptr.p : nullptr;
+        a.inc_ptr = plan->wide ? slot_ptr : nullptr;
         a.packed = plan->packed.p;
         a.Y = Y.p;
         a.G = G.p;
@@ -1583,7 +1836,7 @@ int ElemPcg<TT>::launch_iteration(const ElemTopology &top, const TT *T, const ui
                            early);
     } else {
         launch_overlapping(true, k_epass2<TT>, wave_grid(k_epass2<TT>, n, kEBlock), kEBlock, 0, s, n, free_mask,
-                           top.inc_ptr.p, Y.p, G.p, R.p, D.p, st.p, part.p, use_cond, cond, early);
+                           slot_ptr, Y.p, G.p, R.p, D.p, st.p, part.p, use_cond, cond, early);
     }
     SNP_LAUNCH_CHECK();
     return SNP_OK;

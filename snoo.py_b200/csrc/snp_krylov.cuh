@@ -129,6 +129,20 @@ struct Pcg {
 
 // Element topology of the operator: DoFs with edge signs and the DoF -> (element, local
 // edge) incidence, built once per mesh.
+// Tiles of consecutive elements for the float64 element pass: the distinct DoFs of a tile ("pairs"
+// of tile and DoF), tile by tile, DoFs ascending.  A pair's terms are summed inside the tile and
+// leave as one slot value; slots are numbered by DoF, then tile.
+struct TilePlan {
+    int32_t te = 0;             // elements of a tile; 0: no plan
+    int32_t tiles = 0, pairs = 0;
+    DevBuf<int32_t> tile_ptr;   // [tiles + 1] first pair of each tile
+    DevBuf<int32_t> dof, slot;  // [pairs]
+    DevBuf<uint32_t> terms;     // [pairs] first of the pair's terms in the tile's list | number << 16
+    DevBuf<uint16_t> list;      // [tiles][6 te] the pairs' terms k * te + element, element order
+    DevBuf<uint16_t> place;     // [tiles][6][te] pair of (element, k) within the tile, bit 15 = sign
+    DevBuf<int32_t> slot_ptr;   // [n + 1] first slot of each DoF
+};
+
 struct ElemTopology {
     int64_t n_elems = 0;
     int32_t n = 0;
@@ -139,6 +153,9 @@ struct ElemTopology {
     DevBuf<double> chat64;    // [18] reference curls of orientation 0
     DevBuf<float> chat32;
     double chat_h[18];        // the same on the host (kernel parameters)
+    TilePlan tile;
+    // first slot value of every DoF in the float64 passes
+    const int32_t *slot_ptr64() const { return tile.te ? tile.slot_ptr.p : inc_ptr.p; }
 };
 
 // What the block-Jacobi DoF pass reads per 256-DoF tile besides the CG state, laid out so that a
@@ -279,6 +296,7 @@ struct ElemPcg {
     int apply(const ElemTopology &top, const TT *T, const uint8_t *free_mask, const TT *x, TT *y, cudaStream_t s);
 
    private:
+    void launch_tile_pass(const ElemTopology &top, const double *T, int early, cudaStream_t s);
     int launch_iteration(const ElemTopology &top, const TT *T, const uint8_t *free_mask, const BlockPlan *plan,
                          cudaStream_t s, int use_cond, cudaGraphConditionalHandle cond);
     int build_graph(const ElemTopology &top, const TT *T, const uint8_t *free_mask, const BlockPlan *plan);
