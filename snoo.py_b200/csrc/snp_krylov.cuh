@@ -258,10 +258,15 @@ template <typename TT>
 struct ElemPcg {
     int32_t n = 0;
     int64_t ne = 0;
-    DevBuf<DofPair<TT>> G;  // {z, p}, padded to whole 256-DoF tiles
-    DevBuf<DofPair<TT>> R;  // {r, x}, likewise
+    template <typename T>
+    struct Part {
+        T *p = nullptr;
+    };
+    DevBuf<DofPair<TT>> state;  // R, G and Y one after another: one L2 window reaches all of them
+    Part<DofPair<TT>> R;    // {r, x}, padded to whole 256-DoF tiles
+    Part<DofPair<TT>> G;    // {z, p}, likewise
     DevBuf<TT> D;           // 1 / diag(J)
-    DevBuf<TT> Y;           // [6 n_elems] element-edge terms in DoF-ordered slots, padded by 8
+    Part<TT> Y;             // [6 n_elems] element-edge terms in DoF-ordered slots, padded by 8
     DevBuf<double> part;
     DevBuf<PcgState> st;
     HostBuf<PcgState> hst;
@@ -272,7 +277,7 @@ struct ElemPcg {
     const TT *key_T = nullptr;
     const uint8_t *key_fm = nullptr;
     const BlockPlan *key_plan = nullptr;
-    bool l2_window = false;  // the graph's kernels carry the L2 window over Y
+    bool l2_window = false;  // the graph's kernels carry an L2 window (over Y, G and R as they fit)
     size_t l2_bytes = 0;     // its size, the set-aside raised while a solve runs
     // raise and release the context's persisting-L2 set-aside around each solve (a device-wide
     // setting: off while several solvers run at once, snp_solver_solve_many)
