@@ -1722,6 +1722,7 @@ int build_block_plan(BlockPlan &plan, const ElemTopology &top, const uint8_t *fr
     SNP_CUDA_TRY(cudaStreamSynchronize(s));
     SNP_TRY(plan.packed.alloc((size_t)total));
     SNP_CUDA_TRY(cudaMemsetAsync(plan.packed.p, 0, sizeof(float) * (size_t)(total > 0 ? total : 1), s));
+    SNP_CUDA_TRY(cudaStreamSynchronize(s));  // solves may run on other streams
     plan.wide = hw != 0;
     plan.tiles = tiles;
     return SNP_OK;
@@ -1752,7 +1753,7 @@ void ElemPcg<TT>::drop_graph() {
 }
 
 template <typename TT>
-int ElemPcg<TT>::reserve(int32_t n_, int64_t ne_) {
+int ElemPcg<TT>::reserve(int32_t n_, int64_t ne_, cudaStream_t s) {
     if (n_ == n && ne_ == ne && G.p) return SNP_OK;
     drop_graph();
     n = n_;
@@ -1761,7 +1762,9 @@ int ElemPcg<TT>::reserve(int32_t n_, int64_t ne_) {
     // whole 16-byte words of Y are copied: 8 values of padding
     const size_t slots = ((6 * (size_t)ne + 8) * sizeof(TT) + sizeof(DofPair<TT>) - 1) / sizeof(DofPair<TT>);
     SNP_TRY(state.alloc(2 * padded + slots));
-    SNP_CUDA_TRY(cudaMemset(state.p, 0, sizeof(DofPair<TT>) * (2 * padded + slots)));
+    // on the solve's stream: a memset on the default stream is not ordered with it, and behind the
+    // kernels of other solves it may run after this solve has started
+    SNP_CUDA_TRY(cudaMemsetAsync(state.p, 0, sizeof(DofPair<TT>) * (2 * padded + slots), s));
     R.p = state.p;
     G.p = R.p + padded;
     Y.p = reinterpret_cast<TT *>(G.p + padded);
@@ -1771,7 +1774,7 @@ int ElemPcg<TT>::reserve(int32_t n_, int64_t ne_) {
     SNP_TRY(st.alloc(1));
     SNP_TRY(hst.alloc(1));
     SNP_TRY(bad.alloc(1));
-    SNP_CUDA_TRY(cudaMemset(st.p, 0, sizeof(PcgState)));
+    SNP_CUDA_TRY(cudaMemsetAsync(st.p, 0, sizeof(PcgState), s));
     return SNP_OK;
 }
 
@@ -2019,7 +2022,7 @@ int ElemPcg<TT>::solve(const ElemTopology &top, const TT *T, const double *diag,
                        cudaStream_t s, int64_t *its, double *res, int *status, const BlockPlan *plan) {
     bool hold = false;  // this solve raised the L2 set-aside
     SNP_REQUIRE(top.n > 0 && top.n_elems > 0, "element PCG: topology not built");
-    SNP_TRY(reserve(top.n, top.n_elems));
+    SNP_TRY(reserve(top.n, top.n_elems, s));
     if (maxit < 0) maxit = 10 * (int64_t)n;
     SNP_CUDA_TRY(cudaMemsetAsync(bad.p, 0, sizeof(int), s));
     if (plan)
@@ -2083,7 +2086,7 @@ extract:
     }
     const PcgState &H = *hst.p;
     if (H.done == 5) {
-        SNP_CUDA_TRY(cudaMemset(st.p, 0, sizeof(PcgState)));
+        SNP_CUDA_TRY(cudaMemsetAsync(st.p, 0, sizeof(PcgState), s));
         return fail(SNP_CUDA_ERROR, "element PCG: a wait inside the Krylov loop timed out");
     }
     launches += 1 + (chunk_launches >= 0 ? chunk_launches : 2 * (H.iter > 0 ? H.iter : 1));
@@ -2100,7 +2103,7 @@ template <typename TT>
 int ElemPcg<TT>::apply(const ElemTopology &top, const TT *T, const uint8_t *free_mask, const TT *x, TT *y,
                        cudaStream_t s) {
     SNP_REQUIRE(top.n > 0 && top.n_elems > 0, "element operator: topology not built");
-    SNP_TRY(reserve(top.n, top.n_elems));
+    SNP_TRY(reserve(top.n, top.n_elems, s));
     const Chat<TT> ch = chat_of<TT>(top);
     k_eapply1<TT><<<wave_grid(k_eapply1<TT>, ne, kEBlock), kEBlock, 0, s>>>(ne, top.edof.p, top.pos.p, T, ch,
                                                                            free_mask, x, Y.p);

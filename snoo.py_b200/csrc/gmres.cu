@@ -105,7 +105,7 @@ int point_jacobi_apply(int32_t n, const uint8_t *free_mask, const double *diag, 
     return SNP_OK;
 }
 
-int Gmres::reserve(int64_t n_, int m_) {
+int Gmres::reserve(int64_t n_, int m_, cudaStream_t s) {
     if (n_ == n && m_ == m) return SNP_OK;
     n = n_;
     m = m_;
@@ -117,7 +117,7 @@ int Gmres::reserve(int64_t n_, int m_) {
     SNP_TRY(hdev.alloc(2 * (size_t)(m + 1) + 2));
     SNP_TRY(counter.alloc(1));
     SNP_TRY(hhost.alloc(2 * (size_t)(m + 1) + 2));
-    SNP_CUDA_TRY(cudaMemset(counter.p, 0, sizeof(unsigned int)));
+    SNP_CUDA_TRY(cudaMemsetAsync(counter.p, 0, sizeof(unsigned int), s));
     return SNP_OK;
 }
 

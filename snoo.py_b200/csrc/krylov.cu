@@ -428,7 +428,7 @@ Pcg<VT, XT>::~Pcg() {
 }
 
 template <typename VT, typename XT>
-int Pcg<VT, XT>::reserve(int32_t n_) {
+int Pcg<VT, XT>::reserve(int32_t n_, cudaStream_t s) {
     if (n_ <= cap) {
         n = n_;
         return SNP_OK;
@@ -445,7 +445,7 @@ int Pcg<VT, XT>::reserve(int32_t n_) {
     SNP_TRY(st.alloc(1));
     SNP_TRY(hst.alloc(1));
     SNP_TRY(bad.alloc(1));
-    SNP_CUDA_TRY(cudaMemset(st.p, 0, sizeof(PcgState)));
+    SNP_CUDA_TRY(cudaMemsetAsync(st.p, 0, sizeof(PcgState), s));
     return SNP_OK;
 }
 
@@ -543,7 +543,7 @@ int Pcg<VT, XT>::build_graph(const CsrView<VT> &A, const uint8_t *free_mask, XT 
 template <typename VT, typename XT>
 int Pcg<VT, XT>::solve(const CsrView<VT> &A, const uint8_t *free_mask, const XT *b, XT *x, double rtol, double atol,
                        int64_t maxit, bool zero_x, cudaStream_t s, int64_t *its, double *res, int *status) {
-    SNP_TRY(reserve(A.n));
+    SNP_TRY(reserve(A.n, s));
     if (maxit < 0) maxit = 10 * (int64_t)A.n;  // scipy's default uses n_free; A.n bounds it
     // initial residual
     const int g = stride_grid(A.n, kVecBlock, 8);
@@ -702,7 +702,7 @@ int snp_pcg(int32_t n_rows, const int32_t *row_ptr, const int32_t *col_idx, cons
     SNP_CUDA_TRY(cudaStreamSynchronize(s));
     snp::CsrView<double> A{n_rows, nnz_last, row_ptr, col_idx, vals};
     snp::Pcg<double, double> pcg;
-    SNP_TRY(pcg.reserve(n_rows));
+    SNP_TRY(pcg.reserve(n_rows, s));
     bool zp = false;
     SNP_TRY(pcg.set_jacobi(A, diag.p, free_mask, s, &zp));
     if (zp) return snp::fail(SNP_ZERO_PIVOT, "snp_pcg: zero or missing diagonal entry on a free row");

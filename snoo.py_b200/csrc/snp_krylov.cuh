@@ -103,7 +103,7 @@ struct Pcg {
     Pcg(const Pcg &) = delete;
     Pcg &operator=(const Pcg &) = delete;
     ~Pcg();
-    int reserve(int32_t n);
+    int reserve(int32_t n, cudaStream_t s);
     void drop_graph();
     int set_jacobi(const CsrView<VT> &A, const int32_t *diag_pos, const uint8_t *free_mask, cudaStream_t s,
                    bool *zero_pivot);
@@ -288,7 +288,7 @@ struct ElemPcg {
     ElemPcg(const ElemPcg &) = delete;
     ElemPcg &operator=(const ElemPcg &) = delete;
     ~ElemPcg();
-    int reserve(int32_t n, int64_t ne);
+    int reserve(int32_t n, int64_t ne, cudaStream_t s);
     void drop_graph();
     // Solve J h = b_scale * b on the free DoFs from h = 0 with Jacobi from diag, or block
     // Jacobi when a plan is given (block_jacobi_build); h (float64) gets the
@@ -324,7 +324,7 @@ struct Gmres {
     DevBuf<double> V, w, z, part, hdev;
     DevBuf<unsigned int> counter;
     HostBuf<double> hhost;
-    int reserve(int64_t n, int m);
+    int reserve(int64_t n, int m, cudaStream_t s);
     int solve(const Op &apply_J, const Op &apply_M, const uint8_t *free_mask, const double *b, double b_scale,
               double *x, double rtol, double atol, int64_t maxit, cudaStream_t s, int64_t *its, double *res,
               int *status);

@@ -689,7 +689,7 @@ struct snp_solver {
                     int rc;
                     if (krylov == 1) {
                         if (f32) return snp::fail(SNP_BAD_ARG, "GMRES runs in float64 (solve with precision 0)");
-                        SNP_TRY(gmres.reserve(n, krylov_restart));
+                        SNP_TRY(gmres.reserve(n, krylov_restart, stream));
                         gmres.launches = 0;
                         const snp::Gmres::Op opJ = [&](const double *xx, double *yy) {
                             launches += 2;
@@ -989,8 +989,9 @@ int snp_solver_finalize(snp_solver *s) {
     SNP_CUDA_TRY(cudaMemcpyAsync(&hc, cnt.p, sizeof(hc), cudaMemcpyDeviceToHost, st));
     SNP_CUDA_TRY(cudaStreamSynchronize(st));
     s->n_free = (int64_t)hc;
-    SNP_TRY(s->pcg64.reserve(s->n));
-    SNP_TRY(s->pcg32.reserve(s->n));
+    SNP_TRY(s->pcg64.reserve(s->n, st));
+    SNP_TRY(s->pcg32.reserve(s->n, st));
+    SNP_CUDA_TRY(cudaStreamSynchronize(st));  // solves may run on other streams
     s->finalized = true;
     return SNP_OK;
 }
@@ -1127,8 +1128,8 @@ int snp_solver_set_block_jacobi(snp_solver *s, const uint16_t *meta) {
     SNP_TRY(s->bj_mat.alloc((size_t)n * snp::kBlockJacobiMax));
     SNP_TRY(s->bj_inv.alloc((size_t)n * snp::kBlockJacobiMax));
     SNP_TRY(s->bj_fallback.alloc(1));
-    SNP_CUDA_TRY(cudaMemcpy(s->bj_meta.p, meta, sizeof(uint16_t) * n, cudaMemcpyHostToDevice));
-    SNP_CUDA_TRY(cudaMemset(s->bj_fallback.p, 0, sizeof(int)));
+    SNP_CUDA_TRY(cudaMemcpyAsync(s->bj_meta.p, meta, sizeof(uint16_t) * n, cudaMemcpyHostToDevice, s->stream));
+    SNP_CUDA_TRY(cudaMemsetAsync(s->bj_fallback.p, 0, sizeof(int), s->stream));
     // the Krylov graphs hold the previous partition's arrays
     s->epcg64.drop_graph();
     s->epcg32.drop_graph();

@@ -433,3 +433,33 @@ def test_tile_pass_and_its_fallback(order):
     Jh = eng.jacobian_apply(h, torch.zeros_like(h), "fp64")
     rel = float(torch.linalg.vector_norm((Jh + F)[free]) / torch.linalg.vector_norm(F[free]))
     assert rel <= 1.0001e-3  # the recursive residual met 1e-3; the true one differs by rounding
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_first_solves_are_ordered_without_the_default_stream(precision):
+    """A solver's first Krylov solve clears its state on its own stream: two solvers at once, with the
+    default stream busy meanwhile, answer as they do the second time, bit by bit."""
+    import torch
+
+    from snoopy_b200 import _lib
+
+    solvers = [_window_solver(20000) for _ in range(2)]
+    for s in solvers:
+        s.stream = torch.cuda.Stream()
+    engs = [s.newton_engine() for s in solvers]
+    opts = (_lib.SolveOpts * 2)(*[_lib.SolveOpts(1, 1e-6, 50000, 60, 0.1, precision, 0, 1, 0.0)] * 2)
+    out = []
+    for busy in (True, False):
+        xs = [torch.zeros(e.n, dtype=torch.float64, device="cuda") for e in engs]
+        torch.cuda.synchronize()
+        if busy:
+            torch.cuda._sleep(400_000_000)  # about 0.2 s
+        stats, status = (_lib.SolveStats * 2)(), (ctypes.c_int32 * 2)()
+        rc = _lib.load().snp_solver_solve_many((ctypes.c_void_p * 2)(*[e.handle.value for e in engs]), 2,
+                                               (ctypes.c_void_p * 2)(*[x.data_ptr() for x in xs]), opts, stats, 2,
+                                               status)
+        torch.cuda.synchronize()
+        assert rc == 0, _lib.load().snp_last_error()
+        out.append(xs)
+    for a, b in zip(*out):
+        assert torch.equal(a, b)
