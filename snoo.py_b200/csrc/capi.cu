@@ -6,6 +6,7 @@
 #include <tuple>
 
 #include "snp_common.cuh"
+#include "snp_internal.cuh"
 
 namespace snp {
 
@@ -20,6 +21,15 @@ int fail(int code, const char *fmt, ...) {
 }
 
 void clear_error() { g_err[0] = '\0'; }
+
+static thread_local int64_t g_alloc_made = 0, g_alloc_left = -1;
+
+bool alloc_refused() {
+    ++g_alloc_made;
+    if (g_alloc_left == 0) return true;
+    if (g_alloc_left > 0) --g_alloc_left;
+    return false;
+}
 
 int sm_count() {
     static std::mutex mu;
@@ -70,5 +80,12 @@ extern "C" {
 const char *snp_last_error(void) { return snp::g_err; }
 
 int snp_version(void) { return 1; }
+
+int snp_alloc_probe(int64_t allowed, int64_t *made) {
+    snp::clear_error();
+    if (made) *made = snp::g_alloc_made;
+    snp::g_alloc_left = allowed < 0 ? -1 : allowed;
+    return SNP_OK;
+}
 
 }  // extern "C"

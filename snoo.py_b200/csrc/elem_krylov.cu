@@ -1754,27 +1754,31 @@ void ElemPcg<TT>::drop_graph() {
 
 template <typename TT>
 int ElemPcg<TT>::reserve(int32_t n_, int64_t ne_, cudaStream_t s) {
-    if (n_ == n && ne_ == ne && G.p) return SNP_OK;
+    if (n_ == n && ne_ == ne) return SNP_OK;
     drop_graph();
-    n = n_;
-    ne = ne_;
-    const size_t padded = ((size_t)n + kBjTile - 1) / kBjTile * kBjTile;
+    n = 0;  // the sizes stand once everything behind them does: launches take the pointers unchecked
+    ne = 0;
+    R.p = G.p = nullptr;
+    Y.p = nullptr;
+    const size_t padded = ((size_t)n_ + kBjTile - 1) / kBjTile * kBjTile;
     // whole 16-byte words of Y are copied: 8 values of padding
-    const size_t slots = ((6 * (size_t)ne + 8) * sizeof(TT) + sizeof(DofPair<TT>) - 1) / sizeof(DofPair<TT>);
+    const size_t slots = ((6 * (size_t)ne_ + 8) * sizeof(TT) + sizeof(DofPair<TT>) - 1) / sizeof(DofPair<TT>);
     SNP_TRY(state.alloc(2 * padded + slots));
     // on the solve's stream: a memset on the default stream is not ordered with it, and behind the
     // kernels of other solves it may run after this solve has started
     SNP_CUDA_TRY(cudaMemsetAsync(state.p, 0, sizeof(DofPair<TT>) * (2 * padded + slots), s));
-    R.p = state.p;
-    G.p = R.p + padded;
-    Y.p = reinterpret_cast<TT *>(G.p + padded);
-    SNP_TRY(D.alloc(n));
+    SNP_TRY(D.alloc(n_));
     const int gmax = sm_count() * 8 + 1;
     SNP_TRY(part.alloc(3 * (size_t)gmax));
     SNP_TRY(st.alloc(1));
     SNP_TRY(hst.alloc(1));
     SNP_TRY(bad.alloc(1));
     SNP_CUDA_TRY(cudaMemsetAsync(st.p, 0, sizeof(PcgState), s));
+    R.p = state.p;
+    G.p = R.p + padded;
+    Y.p = reinterpret_cast<TT *>(G.p + padded);
+    n = n_;
+    ne = ne_;
     return SNP_OK;
 }
 

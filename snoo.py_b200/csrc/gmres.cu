@@ -107,17 +107,19 @@ int point_jacobi_apply(int32_t n, const uint8_t *free_mask, const double *diag, 
 
 int Gmres::reserve(int64_t n_, int m_, cudaStream_t s) {
     if (n_ == n && m_ == m) return SNP_OK;
+    n = 0;  // the sizes stand once everything behind them does
+    m = 0;
+    blocks = stride_grid(n_, kGB, 4);
+    SNP_TRY(V.alloc((size_t)(m_ + 1) * (size_t)n_));
+    SNP_TRY(w.alloc(n_));
+    SNP_TRY(z.alloc(n_));
+    SNP_TRY(part.alloc((size_t)(m_ + 1) * blocks));
+    SNP_TRY(hdev.alloc(2 * (size_t)(m_ + 1) + 2));
+    SNP_TRY(counter.alloc(1));
+    SNP_TRY(hhost.alloc(2 * (size_t)(m_ + 1) + 2));
+    SNP_CUDA_TRY(cudaMemsetAsync(counter.p, 0, sizeof(unsigned int), s));
     n = n_;
     m = m_;
-    blocks = stride_grid(n, kGB, 4);
-    SNP_TRY(V.alloc((size_t)(m + 1) * (size_t)n));
-    SNP_TRY(w.alloc(n));
-    SNP_TRY(z.alloc(n));
-    SNP_TRY(part.alloc((size_t)(m + 1) * blocks));
-    SNP_TRY(hdev.alloc(2 * (size_t)(m + 1) + 2));
-    SNP_TRY(counter.alloc(1));
-    SNP_TRY(hhost.alloc(2 * (size_t)(m + 1) + 2));
-    SNP_CUDA_TRY(cudaMemsetAsync(counter.p, 0, sizeof(unsigned int), s));
     return SNP_OK;
 }
 

@@ -434,18 +434,19 @@ int Pcg<VT, XT>::reserve(int32_t n_, cudaStream_t s) {
         return SNP_OK;
     }
     drop_graph();
-    n = cap = n_;
-    SNP_TRY(r.alloc(n));
-    SNP_TRY(z.alloc(n));
-    SNP_TRY(p.alloc(n));
-    SNP_TRY(q.alloc(n));
-    SNP_TRY(dinv.alloc(n));
+    n = cap = 0;  // the sizes stand once everything behind them does
+    SNP_TRY(r.alloc(n_));
+    SNP_TRY(z.alloc(n_));
+    SNP_TRY(p.alloc(n_));
+    SNP_TRY(q.alloc(n_));
+    SNP_TRY(dinv.alloc(n_));
     const int gmax = sm_count() * 8 + 1;
     SNP_TRY(part.alloc(3 * (size_t)gmax));
     SNP_TRY(st.alloc(1));
     SNP_TRY(hst.alloc(1));
     SNP_TRY(bad.alloc(1));
     SNP_CUDA_TRY(cudaMemsetAsync(st.p, 0, sizeof(PcgState), s));
+    n = cap = n_;
     return SNP_OK;
 }
 

@@ -15,6 +15,10 @@ namespace snp {
 __host__ __device__ __forceinline__ int64_t eslot(int64_t e, int k) { return ((e >> 5) * 6 + k) * 32 + (e & 31); }
 __host__ __device__ __forceinline__ int64_t eslots_size(int64_t n_elems) { return ((n_elems + 31) >> 5) * 192; }
 
+// Counts an allocation of the calling thread; true when snp_alloc_probe has it refused, as if memory
+// were exhausted.
+bool alloc_refused();
+
 // Owning device allocation (cudaMalloc'd; freed on destruction).
 template <typename T>
 struct DevBuf {
@@ -39,7 +43,8 @@ struct DevBuf {
     int alloc(size_t count) {
         release();
         if (count == 0) count = 1;
-        cudaError_t e = cudaMalloc(reinterpret_cast<void **>(&p), count * sizeof(T));
+        cudaError_t e = alloc_refused() ? cudaErrorMemoryAllocation
+                                        : cudaMalloc(reinterpret_cast<void **>(&p), count * sizeof(T));
         if (e != cudaSuccess) {
             p = nullptr;
             cudaGetLastError();
@@ -68,7 +73,9 @@ struct HostBuf {
     int alloc(size_t count) {
         if (p) cudaFreeHost(p);
         p = nullptr;
-        cudaError_t e = cudaMallocHost(reinterpret_cast<void **>(&p), (count ? count : 1) * sizeof(T));
+        cudaError_t e = alloc_refused()
+                            ? cudaErrorMemoryAllocation
+                            : cudaMallocHost(reinterpret_cast<void **>(&p), (count ? count : 1) * sizeof(T));
         if (e != cudaSuccess) {
             p = nullptr;
             cudaGetLastError();
