@@ -729,9 +729,10 @@ __global__ void __launch_bounds__(kDofThreads, 4)
     __shared__ uint64_t full[kDofStages], empty[kDofStages];
     __shared__ TileInfo info[kDofStages];
     __shared__ volatile int s_fail;
+    __shared__ volatile int s_done;
     const bool producer = threadIdx.x >= kEBlock;
     if (threadIdx.x == 0) {
-        s_fail = 0;
+        s_fail = s_done = 0;
         for (int s = 0; s < kDofStages; ++s) {
             mbar_init(full + s, 1);
             mbar_init(empty + s, kEBlock / 32);
@@ -779,7 +780,14 @@ __global__ void __launch_bounds__(kDofThreads, 4)
             }
         }
         __syncwarp();
-    } else if (pass_begins(), !st->done) {
+    } else {
+        pass_begins();
+        // A block whose wait ran out sets done while others of the launch are still starting, so two
+        // threads may read it differently.  None leaves by its own reading: the barrier of the first
+        // tile, which counts all eight warps, votes on it before anything is written.  The first
+        // tile's loads no longer wait for done: 34.8 -> 34.4 and 56.4 -> 56.0 us per iteration at
+        // 600k and 1.16M tets (55.9 -> 57.0 with a volatile read).
+        const bool finished = st->done != 0;
         const TT alpha = (TT)st->alpha, beta = (TT)st->beta;
         const int tid = threadIdx.x;
         int it = 0;
@@ -813,8 +821,9 @@ __global__ void __launch_bounds__(kDofThreads, 4)
             s_r[tid] = r;
             // r alternates between two buffers: a tile writes the one whose readers of two tiles ago
             // have passed the barrier in between
-            if (consumer_sync_any(!here)) {
-                s_fail = 1;
+            if (consumer_sync_any(!here || finished)) {
+                if (finished) s_done = 1;
+                else if (!here) s_fail = 1;
                 break;
             }
             if (fr) {
@@ -843,7 +852,7 @@ __global__ void __launch_bounds__(kDofThreads, 4)
         }
         return;
     }
-    if (st->done) {
+    if (s_done) {
         if (use_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(cond, 0);
         return;
     }
