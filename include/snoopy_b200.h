@@ -503,7 +503,8 @@ int snp_solver_reduced_system(snp_solver *s, int precision, const float *V, int3
  * edge DoFs numbered by their lower node, blocks of the edges that share that node halve the CG
  * iterations of the window-frame yoke.  meta = NULL goes back to point Jacobi.  The
  * reference-semantics mode keeps point Jacobi (red_mvp_solver.py:199 builds
- * M = diags(1 / diag(J))).  Synchronises (meta is checked and uploaded). */
+ * M = diags(1 / diag(J))).  Synchronises (meta is checked and uploaded).  A partition that does not
+ * pass the check leaves the previous one; a failure behind it (SNP_NO_MEMORY) leaves point Jacobi. */
 int snp_solver_set_block_jacobi(snp_solver *s, const uint16_t *meta);
 
 /* Krylov method of the residual-mode Newton steps (the reference's scipy cg in each Newton step,

@@ -1124,15 +1124,16 @@ int snp_solver_set_block_jacobi(snp_solver *s, const uint16_t *meta) {
         }
         i += size;
     }
+    // off until everything of the new partition stands; the Krylov graphs hold the previous one's arrays
+    s->bj_on = false;
+    s->epcg64.drop_graph();
+    s->epcg32.drop_graph();
     SNP_TRY(s->bj_meta.alloc(n));
     SNP_TRY(s->bj_mat.alloc((size_t)n * snp::kBlockJacobiMax));
     SNP_TRY(s->bj_inv.alloc((size_t)n * snp::kBlockJacobiMax));
     SNP_TRY(s->bj_fallback.alloc(1));
     SNP_CUDA_TRY(cudaMemcpyAsync(s->bj_meta.p, meta, sizeof(uint16_t) * n, cudaMemcpyHostToDevice, s->stream));
     SNP_CUDA_TRY(cudaMemsetAsync(s->bj_fallback.p, 0, sizeof(int), s->stream));
-    // the Krylov graphs hold the previous partition's arrays
-    s->epcg64.drop_graph();
-    s->epcg32.drop_graph();
     SNP_TRY(snp::build_block_plan(s->bj_plan, s->etop, s->free_mask.p, s->bj_meta.p, s->stream));
     s->bj_plan.meta = s->bj_meta.p;
     s->bj_plan.binv = s->bj_inv.p;

@@ -220,7 +220,12 @@ class DeviceNewton:
             return
         meta = np.ascontiguousarray(meta, dtype=np.uint16)
         assert meta.shape == (self.n,)
-        _lib.call("snp_solver_set_block_jacobi", self.handle, meta.ctypes.data_as(ctypes.c_void_p))
+        try:
+            _lib.call("snp_solver_set_block_jacobi", self.handle, meta.ctypes.data_as(ctypes.c_void_p))
+        except _lib.SnpError as err:
+            if _lib.STATUS.get(err.status) != "SNP_BAD_ARG":  # a bad partition leaves the previous one
+                self.block_jacobi = False
+            raise
         self.block_jacobi = True
 
     def set_preconditioner(self, kind="block", meta=None):

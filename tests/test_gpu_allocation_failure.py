@@ -66,3 +66,37 @@ def test_krylov_work_space_refused_in_the_middle(method, precision, allowed):
             allowed(-1)
             assert err.value.status == NO_MEMORY
         assert torch.equal(solve(eng), want), k
+
+
+def test_block_partition_refused_in_the_middle(allowed):
+    """A refused new partition leaves point Jacobi; the next one takes over completely."""
+    import numpy as np
+    import torch
+    from snoopy_b200.newton import dof_blocks
+
+    eng = _solver(900).newton_engine()
+    free = eng.free_mask.cpu().numpy().astype(bool)
+    other = dof_blocks(np.arange(eng.n) // 3, free)
+
+    def solve():
+        return eng.solve(None, tol=1e-8, max_newton=2, raise_on_failure=False)[0].clone()
+
+    lower_node = solve()
+    before = allowed(-1)
+    eng.set_preconditioner("block", meta=other)
+    need = allowed(-1) - before
+    threes = solve()
+    eng.set_preconditioner("jacobi")
+    point = solve()
+    assert not torch.equal(point, threes) and not torch.equal(lower_node, threes)
+    for k in range(need):
+        eng.set_preconditioner("block")
+        assert torch.equal(solve(), lower_node)
+        allowed(k)
+        with pytest.raises(_lib.SnpError) as err:
+            eng.set_preconditioner("block", meta=other)
+        allowed(-1)
+        assert err.value.status == NO_MEMORY and not eng.block_jacobi
+        assert torch.equal(solve(), point), k
+        eng.set_preconditioner("block", meta=other)
+        assert torch.equal(solve(), threes), k
