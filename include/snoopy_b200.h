@@ -54,9 +54,10 @@ int snp_version(void);
 
 /* For tests of memory exhaustion.  *made (may be NULL): buffers the calling thread has asked this
  * library's allocator for so far (refused ones included).  From now on `allowed` further ones of
- * this thread are served and the ones behind them refused (SNP_NO_MEMORY) without asking the
- * driver; negative: no refusals, the default. */
-int snp_alloc_probe(int64_t allowed, int64_t *made);
+ * this thread are served, the `refused` ones behind them refused (SNP_NO_MEMORY) without asking
+ * the driver, and all later ones served; allowed < 0: no refusals, the default; refused < 0: all
+ * later ones are refused. */
+int snp_alloc_probe(int64_t allowed, int64_t refused, int64_t *made);
 
 /* ------------------------------------------------------------------ CSR pattern
  * Replaces the COO->CSR conversion of fem_c/interface_c.pyx:154-155,367-368

@@ -80,7 +80,7 @@ class GradGradMaterial(ctypes.Structure):
 # name -> argtypes (every function returns int32 status unless listed in _RESTYPES)
 _SIGS = {
     "snp_last_error": [],
-    "snp_alloc_probe": [_c_i64, ctypes.POINTER(_c_i64)],
+    "snp_alloc_probe": [_c_i64, _c_i64, ctypes.POINTER(_c_i64)],
     "snp_version": [],
     "snp_pattern_create": [_vp, _c_i64, _c_i32, _c_i32, _vp, _pp],
     "snp_pattern_info": [_vp, ctypes.POINTER(_c_i32), ctypes.POINTER(_c_i64), ctypes.POINTER(_c_i64),

@@ -22,12 +22,15 @@ int fail(int code, const char *fmt, ...) {
 
 void clear_error() { g_err[0] = '\0'; }
 
-static thread_local int64_t g_alloc_made = 0, g_alloc_left = -1;
+static thread_local int64_t g_alloc_made = 0, g_alloc_left = -1, g_alloc_refusals = 0;
 
 bool alloc_refused() {
     ++g_alloc_made;
-    if (g_alloc_left == 0) return true;
     if (g_alloc_left > 0) --g_alloc_left;
+    else if (g_alloc_left == 0 && g_alloc_refusals != 0) {
+        if (g_alloc_refusals > 0) --g_alloc_refusals;
+        return true;
+    }
     return false;
 }
 
@@ -81,10 +84,11 @@ const char *snp_last_error(void) { return snp::g_err; }
 
 int snp_version(void) { return 1; }
 
-int snp_alloc_probe(int64_t allowed, int64_t *made) {
+int snp_alloc_probe(int64_t allowed, int64_t refused, int64_t *made) {
     snp::clear_error();
     if (made) *made = snp::g_alloc_made;
     snp::g_alloc_left = allowed < 0 ? -1 : allowed;
+    snp::g_alloc_refusals = refused;
     return SNP_OK;
 }
 

@@ -1698,7 +1698,15 @@ int build_elem_topology(ElemTopology &top, int32_t n, const ElemBlock *blocks, i
     SNP_REQUIRE(hbad == 0, "element topology: a DoF index or orientation is out of range");
     top.n_elems = ne;
     top.n = n;
-    SNP_TRY(build_tile_plan(top, s));
+    // the plan is an option: without memory for it the float64 passes keep a slot per element edge
+    const int plan_rc = build_tile_plan(top, s);
+    if (plan_rc == SNP_NO_MEMORY) {
+        SNP_CUDA_TRY(cudaStreamSynchronize(s));
+        top.tile = TilePlan{};
+        clear_error();
+    } else {
+        SNP_TRY(plan_rc);
+    }
     *usable = true;
     return SNP_OK;
 }

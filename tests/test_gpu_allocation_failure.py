@@ -18,11 +18,12 @@ NO_MEMORY = 6
 
 @pytest.fixture
 def allowed():
-    """Sets how many allocations are served from now on (negative: all); returns those made so far."""
+    """Sets how many allocations are served from now on (negative: all) and how many are refused
+    behind them (negative: all); returns those made so far."""
 
-    def probe(n):
+    def probe(n, refused=-1):
         made = ctypes.c_int64()
-        _lib.call("snp_alloc_probe", n, ctypes.byref(made))
+        _lib.call("snp_alloc_probe", n, refused, ctypes.byref(made))
         return made.value
 
     yield probe
@@ -100,3 +101,64 @@ def test_block_partition_refused_in_the_middle(allowed):
         assert torch.equal(solve(), point), k
         eng.set_preconditioner("block", meta=other)
         assert torch.equal(solve(), threes), k
+
+
+def _frame(n_tets, order):
+    import numpy as np
+
+    msh = M.window_frame_mesh(n_tets, jitter=0.15, seed=11)
+    if order == "mesh":
+        return msh
+    perm = np.random.default_rng(3).permutation(msh.num_elements)
+    return M.TetMesh(msh.nodes, msh.cells[perm], msh.elem_domain[perm], grid=msh.grid,
+                     boundary_node_mask=msh._boundary_node_mask)
+
+
+def test_tile_plan_refused_in_the_middle(allowed):
+    """The tiles of the float64 element pass are an option: a solver for which one of their arrays could
+    not be had keeps a slot per element edge, and every other refusal ends the set-up."""
+    import torch
+
+    meshes = {o: _frame(330000, o) for o in ("mesh", "shuffled")}
+    coils = _frame(900, "mesh").geometry.coils()
+
+    def engine(order, *probe):
+        s = S.RedMVPSolver(meshes[order], coils, [M.TAG_IRON], [M.TAG_AIR], [MAT.atan_reluctance()],
+                           max_newton_iterations=60, quad_order=2)
+        s.verbose = False
+        s.curl_curl_factory.pattern  # the assembler's own allocations come first
+        s.compute_source_fields()
+        before = allowed(*(probe or (-1,)))
+        try:
+            eng = s.newton_engine()
+        finally:
+            made = allowed(-1) - before
+        return eng, made
+
+    def step(eng):  # twelve CG iterations
+        x, st = eng.solve(None, tol=1e-8, max_newton=1, cg_rtol=1e-12, cg_maxiter=12, raise_on_failure=False,
+                          line_search=False)
+        assert st["cg_iterations"] == 12
+        return x.clone()
+
+    eng, total = engine("mesh")
+    tiles = step(eng)
+    # a mesh order whose tiles share too few edges stops after three of the plan's allocations
+    plan = total - engine("shuffled")[1] + 3
+    assert plan >= 15
+    # behind the plan: 18 arrays of the solver, 9 of each assembled-matrix CG, 11 of the block partition
+    end = total - (18 + 2 * 9 + 11)
+    first = None
+    for k in range(end - plan, end):
+        eng, _ = engine("mesh", k, 1)
+        x = step(eng)
+        first = x if first is None else first
+        assert torch.equal(x, first), k
+    assert not torch.equal(first, tiles)  # the other sums
+    # the same iterate to rounding: a few 1e-16 per iteration, and room for twelve iterations to carry
+    # them on by a factor of three each
+    assert float((first - tiles).abs().max()) <= 1e-10 * float(tiles.abs().max())
+    for k in (end - plan - 1, end):
+        with pytest.raises(_lib.SnpError) as err:
+            engine("mesh", k, 1)
+        assert err.value.status == NO_MEMORY
