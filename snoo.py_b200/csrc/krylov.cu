@@ -680,13 +680,17 @@ int snp_pcg(int32_t n_rows, const int32_t *row_ptr, const int32_t *col_idx, cons
     SNP_REQUIRE(row_ptr && col_idx && vals && b && x, "snp_pcg: NULL argument");
     SNP_REQUIRE(rtol >= 0 && atol >= 0, "snp_pcg: tolerances must be non-negative");
     cudaStream_t s = snp::as_stream(stream);
-    if (n_rows <= snp::kPcgSmallMaxN) {
-        snp::DevBuf<unsigned char> scratch;
-        SNP_TRY(scratch.alloc(snp::pcg_small_scratch(n_rows)));
+    // one array for the cluster solve's lists, then for the diagonal positions: a system that turns
+    // out not to fit pays the list and no allocation of its own
+    snp::DevBuf<unsigned char> scratch;
+    const bool small = snp::pcg_small_may_fit(n_rows, free_mask);
+    SNP_TRY(scratch.alloc(small ? snp::pcg_small_scratch(n_rows) : sizeof(int32_t) * (size_t)n_rows));
+    int32_t nnz_last = 0;
+    if (small) {
         bool ran = false;
         int st = SNP_OK;
         SNP_TRY(snp::pcg_small(n_rows, row_ptr, col_idx, vals, free_mask, b, x, rtol, atol, maxiter, scratch.p, s, &ran,
-                               iterations, res_norm, &st));
+                               &nnz_last, iterations, res_norm, &st));
         if (ran) {
             if (st == SNP_ZERO_PIVOT) return snp::fail(st, "snp_pcg: zero or missing diagonal entry on a free row");
             if (st == SNP_NOT_CONVERGED) return snp::fail(st, "snp_pcg: maxiter reached");
@@ -695,17 +699,17 @@ int snp_pcg(int32_t n_rows, const int32_t *row_ptr, const int32_t *col_idx, cons
         }
     }
     // diagonal positions (rows are sorted; found by a search kernel)
-    snp::DevBuf<int32_t> diag;
-    SNP_TRY(diag.alloc(n_rows));
-    SNP_TRY(snp::find_diag(n_rows, row_ptr, col_idx, diag.p, s));
-    int32_t nnz_last = 0;
-    SNP_CUDA_TRY(cudaMemcpyAsync(&nnz_last, row_ptr + n_rows, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-    SNP_CUDA_TRY(cudaStreamSynchronize(s));
+    int32_t *diag = reinterpret_cast<int32_t *>(scratch.p);
+    SNP_TRY(snp::find_diag(n_rows, row_ptr, col_idx, diag, s));
+    if (!small) {
+        SNP_CUDA_TRY(cudaMemcpyAsync(&nnz_last, row_ptr + n_rows, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+        SNP_CUDA_TRY(cudaStreamSynchronize(s));
+    }
     snp::CsrView<double> A{n_rows, nnz_last, row_ptr, col_idx, vals};
     snp::Pcg<double, double> pcg;
     SNP_TRY(pcg.reserve(n_rows, s));
     bool zp = false;
-    SNP_TRY(pcg.set_jacobi(A, diag.p, free_mask, s, &zp));
+    SNP_TRY(pcg.set_jacobi(A, diag, free_mask, s, &zp));
     if (zp) return snp::fail(SNP_ZERO_PIVOT, "snp_pcg: zero or missing diagonal entry on a free row");
     int status = SNP_OK;
     SNP_TRY(pcg.solve(A, free_mask, b, x, rtol, atol, maxiter, false, s, iterations, res_norm, &status));

@@ -84,11 +84,13 @@ extern "C" int snp_pcg_noalloc(int32_t n_rows, const int32_t *row_ptr, const int
     B.st = reinterpret_cast<snp::PcgState *>(base + snp::kOffState);
     B.bad = reinterpret_cast<int *>(base + snp::kOffBad);
     B.max_blocks = snp::kMaxBlocks;
-    {
+    int32_t nnz = 0;
+    const bool small = snp::pcg_small_may_fit(n_rows, free_mask);
+    if (small) {
         bool ran = false;
         int st = SNP_OK;
         SNP_TRY(snp::pcg_small(n_rows, row_ptr, col_idx, vals, free_mask, b, x, rtol, atol, maxiter,
-                               base + snp::kOffR, s, &ran, iterations, res_norm, &st));
+                               base + snp::kOffR, s, &ran, &nnz, iterations, res_norm, &st));
         if (ran) {
             if (st == SNP_ZERO_PIVOT) return snp::fail(st, "pcg: zero or missing diagonal entry on a free row");
             if (st == SNP_NOT_CONVERGED) return snp::fail(st, "snp_pcg_noalloc: maxiter reached");
@@ -96,9 +98,10 @@ extern "C" int snp_pcg_noalloc(int32_t n_rows, const int32_t *row_ptr, const int
             return SNP_OK;
         }
     }
-    int32_t nnz = 0;
-    SNP_CUDA_TRY(cudaMemcpyAsync(&nnz, row_ptr + n_rows, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-    SNP_CUDA_TRY(cudaStreamSynchronize(s));
+    if (!small) {
+        SNP_CUDA_TRY(cudaMemcpyAsync(&nnz, row_ptr + n_rows, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+        SNP_CUDA_TRY(cudaStreamSynchronize(s));
+    }
     snp::CsrView<double> A{n_rows, nnz, row_ptr, col_idx, vals};
     int status = SNP_OK;
     SNP_TRY(snp::pcg_on_buffers(A, free_mask, b, x, rtol, atol, maxiter, B, s, iterations, res_norm, &status));

@@ -17,7 +17,10 @@
 // The path is taken where the vectors (at most 8192 free rows) and every block's entries fit into
 // shared memory: 5700 rows of 15 entries.  8192 rows of 4 entries take 14 us per iteration here and
 // 19 us in the general path over 36k rows; a matrix that had to be streamed from L2 took 20 us.
-// The list is one block's work, so meshes above 262144 rows go to the general path unasked.
+// The list is one block's work, so meshes above 262144 rows go to the general path unasked.  A masked
+// system below that whose free rows turn out not to fit pays the list and an empty launch: 3.2 ms
+// per call of 40k rows as before there was this path (3.8 ms while the list had an allocation and a
+// synchronisation of its own).
 #include <cooperative_groups.h>
 
 #include "snp_common.cuh"
@@ -38,7 +41,7 @@ constexpr int kListBlock = 1024;
 constexpr size_t kSmem = 222 * 1024;  // what a block can have beside its slots
 
 struct SmallHead {
-    int32_t run, bad, nf, done;
+    int32_t run, bad, nf, done, nnz;  // nnz: entries of the whole matrix
     long long iter;
     double rr;
 };
@@ -61,6 +64,7 @@ __global__ void __launch_bounds__(kListBlock)
     __shared__ int32_t s_rows[kListWarps];
     __shared__ int64_t s_nnz[kListWarps];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if (threadIdx.x == 0) head->nnz = rp[n];
     const int32_t span = (n + kListBlock - 1) / kListBlock * 32;
     const int32_t i0 = min(wid * span, n), i1 = min(i0 + span, n);
     int32_t cnt = 0;
@@ -323,9 +327,8 @@ size_t pcg_small_scratch(int32_t n) {
 
 int pcg_small(int32_t n, const int32_t *rp, const int32_t *ci, const double *v, const uint8_t *fm, const double *b,
               double *x, double rtol, double atol, int64_t maxit, void *scratch, cudaStream_t s, bool *ran,
-              int64_t *its, double *res, int *status) {
+              int32_t *nnz, int64_t *its, double *res, int *status) {
     *ran = false;
-    if (n > kPcgSmallMaxN || (!fm && n > kPcgSmallRows)) return SNP_OK;
     unsigned char *at = static_cast<unsigned char *>(scratch);
     auto take = [&](size_t count) {
         int32_t *p = reinterpret_cast<int32_t *>(at);
@@ -347,6 +350,7 @@ int pcg_small(int32_t n, const int32_t *rp, const int32_t *ci, const double *v, 
     SmallHead h;
     SNP_CUDA_TRY(cudaMemcpyAsync(&h, head, sizeof(h), cudaMemcpyDeviceToHost, s));
     SNP_CUDA_TRY(cudaStreamSynchronize(s));
+    *nnz = h.nnz;
     if (!h.run) return SNP_OK;
     *ran = true;
     if (h.bad) {

@@ -59,14 +59,16 @@ struct PcgBuffers {
 
 // The same CG for systems of at most kPcgSmallMaxN rows with few free ones, in one thread-block
 // cluster (pcg_small.cu); *ran = false when the system does not fit (then nothing was written to
-// x).  scratch: pcg_small_scratch(n) bytes of device memory, 16-byte aligned.  *status is
-// SNP_ZERO_PIVOT for a zero, missing or NaN diagonal entry on a free row (x untouched).
+// x, and *nnz is the matrix's number of entries).  scratch: pcg_small_scratch(n) bytes of device
+// memory, 16-byte aligned, at least 4 n.  *status is SNP_ZERO_PIVOT for a zero, missing or NaN
+// diagonal entry on a free row (x untouched).  Only where pcg_small_may_fit.
 constexpr int32_t kPcgSmallMaxN = 262144;
 constexpr int32_t kPcgSmallRows = 8192;
+inline bool pcg_small_may_fit(int32_t n, const uint8_t *fm) { return n <= (fm ? kPcgSmallMaxN : kPcgSmallRows); }
 size_t pcg_small_scratch(int32_t n);
 int pcg_small(int32_t n, const int32_t *rp, const int32_t *ci, const double *v, const uint8_t *fm, const double *b,
               double *x, double rtol, double atol, int64_t maxit, void *scratch, cudaStream_t s, bool *ran,
-              int64_t *its, double *res, int *status);
+              int32_t *nnz, int64_t *its, double *res, int *status);
 
 // Jacobi-PCG (float64) with scipy cg's stopping rule on the given buffers; launches only
 // kernels, async copies of scalars and stream synchronisations.

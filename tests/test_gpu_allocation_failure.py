@@ -162,3 +162,19 @@ def test_tile_plan_refused_in_the_middle(allowed):
         with pytest.raises(_lib.SnpError) as err:
             engine("mesh", k, 1)
         assert err.value.status == NO_MEMORY
+
+
+@pytest.mark.parametrize("n,nf", [(9000, 9000), (9000, 8193), (40000, 20000)])
+def test_pcg_too_large_for_the_cluster_allocates_as_any_other(n, nf, allowed):
+    """snp_pcg on systems that the cluster solve does not take: the buffers of the general path, which
+    the same system padded beyond the cluster's limit takes unasked, and no more."""
+    from test_gpu_kernel_edges import _masked_system, _pcg
+
+    A, free, rng = _masked_system(n, nf, 5)
+    b, x0 = rng.normal(size=n), rng.normal(size=n)
+    made = []
+    for pad in (0, 262145 - n):
+        before = allowed(-1)
+        rc, _, its = _pcg(A, None if nf == n else free, b, x0, pad)
+        made.append((allowed(-1) - before, rc))
+    assert made[0] == made[1] == (10, 0)  # diagonal positions; nine of the Krylov work space
