@@ -10,9 +10,28 @@ import numpy as np
 
 from . import _lib
 from . import finite_element as fe
+from .curl_curl_assembler import CurlCurlAssembler
 from .device import torch, upload, zeros
 from .fem_c import biot_savart_device
 from .racetrack_coil import RacetrackCoil
+
+
+# the methods that have a form on the device
+_RACETRACK_B = RacetrackCoil.compute_B
+_NODAL_FIELDS = CurlCurlAssembler.compute_nodal_fields
+
+
+def _method_of(obj, name):
+    """The plain function behind a method bound to ``obj`` itself, else None."""
+    method = getattr(obj, name)
+    return getattr(method, "__func__", None) if getattr(method, "__self__", None) is obj else None
+
+
+def _nodal_fields(assembler, x, tag):
+    """``assembler.compute_nodal_fields(x, [tag])`` as a CUDA tensor [N, 3]."""
+    if _method_of(assembler, "compute_nodal_fields") is _NODAL_FIELDS:
+        return assembler.nodal_fields_device(x, [tag])
+    return upload(assembler.compute_nodal_fields(x, [tag]), np.float64).view(-1, 3)
 
 
 def _located(mesh, positions, vol_tags):
@@ -77,16 +96,15 @@ def evaluate_interpolation(positions, gmsh_model, vol_tags, nodal_values):
 def evaluate_fem_solution_node_interpolation(gmsh_model, points, solver, coil_list, x, domain_list):
     """B at ``points`` by interpolating nodal averages (``evaluators.py:413-454``): per domain of
     ``domain_list`` the element fields averaged at the nodes plus the coils' field at the nodes."""
-    t = torch()
     asm = solver.curl_curl_factory
     nodes_d = upload(asm.nodes, np.float64)
-    b_coil = t.zeros_like(nodes_d)
+    b_coil = torch().zeros_like(nodes_d)
     for coil in coil_list:
-        if type(coil) is RacetrackCoil:  # its compute_B, without the copies to the host and back
+        if _method_of(coil, "compute_B") is _RACETRACK_B:  # the same without the copies to the host and back
             b = biot_savart_device(upload(coil.get_segments(), np.float64), nodes_d, coil.current, coil.rad)
-        else:
-            b = upload(coil.compute_B(asm.nodes), np.float64)
+        else:  # any value that broadcasts over the nodes
+            b = upload(np.broadcast_to(coil.compute_B(asm.nodes), asm.nodes.shape), np.float64)
         b_coil = b_coil + b[: nodes_d.numel()]
     b_coil = b_coil.view(-1, 3)
-    b_node_list = [asm.nodal_fields_device(x, [indx]) + b_coil for indx in domain_list]
+    b_node_list = [_nodal_fields(asm, x, indx) + b_coil for indx in domain_list]
     return evaluate_interpolation(points, gmsh_model, domain_list, b_node_list)
