@@ -303,6 +303,10 @@ int snp_rhs_grad_potential(int64_t n_elems, const double *nodes, const int32_t *
 int snp_biot_savart(const double *src, int64_t n_src, const double *tar, int64_t n_tar, double current,
                     double radius, double *B, void *stream);
 
+/* root[i] = sqrt(a[i]) and quotient[i] = a[i] / b[i] for i < n, as snp_biot_savart evaluates them for
+ * its pairs (for tests of their rounding): positive operands, a from 2^-900 to 2^1000. */
+int snp_biot_savart_roots(int64_t n, const double *a, const double *b, double *root, double *quotient, void *stream);
+
 /* ------------------------------------------------------------------ sparse linear algebra
  * y = A x on the rows/cols with free[i] != 0 (free == NULL: all).  Rows with free[i] == 0
  * give y[i] = 0, and their columns are skipped.  (scipy `J @ x`, `J[mask,:][:,mask]`,

@@ -113,6 +113,7 @@ _SIGS = {
     "snp_b_at_elements": [_c_i64, _vp, _vp, _vp, _vp, _vp, _vp, _c_i32, _vp, _c_i32, _vp, _vp, _vp],
     "snp_rhs_grad_potential": [_c_i64, _vp, _vp, _vp, _vp, _vp, _c_i32, _vp, _vp, _c_i32, _vp, _vp, _vp],
     "snp_biot_savart": [_vp, _c_i64, _vp, _c_i64, _c_f64, _c_f64, _vp, _vp],
+    "snp_biot_savart_roots": [_c_i64, _vp, _vp, _vp, _vp, _vp],
     "snp_spmv": [_c_i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp],
     "snp_pcg": [_c_i32, _vp, _vp, _vp, _vp, _vp, _vp, _c_f64, _c_f64, _c_i64, ctypes.POINTER(_c_i64),
                 ctypes.POINTER(_c_f64), _vp],
