@@ -94,8 +94,10 @@ __device__ __forceinline__ double nu_at(const CurlArgs &a, const double *relc, c
 #pragma unroll
         for (int i = 0; i < 4; ++i) z += ph[i] * Zn[i];
         const double sf = (a.dil[0] + z * a.dil[1]) / (a.dil[2] + z * a.dil[3]);
-        const double nu = sf * pchip_eval<double>(a.n_int, relc, relx, sf * bm, dnu, near);
-        dnu *= sf * sf;
+        // the products' roundings are written out: a kernel that fused one into the next sum would
+        // give other last bits than the kernels it shares this with
+        const double nu = __dmul_rn(sf, pchip_eval<double>(a.n_int, relc, relx, __dmul_rn(sf, bm), dnu, near));
+        dnu = __dmul_rn(dnu, __dmul_rn(sf, sf));
         return nu;
     }
 }
