@@ -181,7 +181,7 @@ int snp_curlcurl_rows(const snp_pattern *pat, const double *terms, int32_t parts
  * of its own in `work` (snp_curlcurl_system_work doubles; contents are not an output): the
  * materials' elements together are the pattern's, in order.  Every requested output is
  * overwritten; J = K + dK per entry; results are bitwise repeatable and equal those of
- * snp_curlcurl_terms + snp_curlcurl_rows. */
+ * snp_curlcurl_terms + snp_curlcurl_rows, also where x holds infinities or NaNs. */
 typedef struct {
     int64_t elem_offset, n_elems;   /* the pattern's elements [elem_offset, elem_offset + n_elems) */
     const int32_t *cells, *glob_ids, *orientations;

@@ -435,7 +435,9 @@ __global__ void __launch_bounds__(kPointBlock, DIL ? 2 : 3)
 // doubles here, where blocks of equal-numbered values give it one useful double per 32-byte sector
 // (entry kernel, 1.16M tets: 571 us from the block layout, 2.7 GB through L2).  The values
 // leave through a shared tile so that the stores are whole lines.
-template <bool HAS_BS, int NQ, bool DIL, bool PRE>
+//
+// ZERO_DK: a material with constant reluctance, whose dK is not stored where it is zero (PackedTerms).
+template <bool HAS_BS, int NQ, bool DIL, bool PRE, bool ZERO_DK>
 __global__ void __launch_bounds__(kBlock)
     k_curlcurl_packed(CurlArgs a, int quad_stride_ctab, int table_doubles, PackedTerms out) {
     extern __shared__ double sm[];
@@ -450,19 +452,37 @@ __global__ void __launch_bounds__(kBlock)
     double *const first = out.J ? out.J : out.K;
     // point sums of k_point_sums, in an array of which the block replaces the read elements later
     const double *const sums = first ? first : out.D;
+    bool any = false;
+    // the values of an element that are not all zero, evaluated again; behind the loop where the point
+    // sums are not replaced by then: inside it costs every call 9 of 435 us at 1.16M tets
+    auto keep_dk = [&](const double *pre, int64_t base) {
+        int g[6];
+        double Fj[6], r[6], *at = out.Dz + (a.t_offset + base + threadIdx.x) * kPackPairs;
+        curl_element<HAS_BS, NQ, DIL, PRE>(a, base + threadIdx.x, T.ctab, T.dphi, T.w, T.phi, T.relc, T.relx, wsum, g, Fj,
+                                           r, pre, [&](int tri, int, int, double, double dv) { at[tri] = dv; });
+    };
 
     for (int64_t base = (int64_t)blockIdx.x * kBlock; base < a.n_elems; base += (int64_t)gridDim.x * kBlock) {
         const int cnt = (int)(a.n_elems - base < kBlock ? a.n_elems - base : kBlock);
         const int64_t eo = a.t_offset + base;
         int g[6];
         double Fj[6], r[6];
+        bool kept = false;
         if ((int)threadIdx.x < cnt)
             curl_element<HAS_BS, NQ, DIL, PRE>(a, base + threadIdx.x, T.ctab, T.dphi, T.w, T.phi, T.relc, T.relx, wsum, g,
                                                Fj, r, PRE ? sums + (eo + threadIdx.x) * kPackPairs : nullptr,
                                                [&](int tri, int, int, double kv, double dv) {
                 if (first) tile[threadIdx.x * kPackPairs + tri] = out.J ? kv + dv : kv;
                 if (out.D) tile_d[threadIdx.x * kPackPairs + tri] = dv;
+                if constexpr (ZERO_DK) kept |= !(dv == 0.0);
             });
+        if constexpr (ZERO_DK) {
+            if constexpr (PRE) {
+                if (kept) keep_dk(sums + (eo + threadIdx.x) * kPackPairs, base);
+            }
+            if ((int)threadIdx.x < cnt) out.kept[eo + threadIdx.x] = kept;
+            any |= kept;
+        }
         __syncthreads();
         if (first)
             for (int t = threadIdx.x; t < cnt * kPackPairs; t += kBlock) first[eo * kPackPairs + t] = tile[t];
@@ -487,6 +507,18 @@ __global__ void __launch_bounds__(kBlock)
             }
             __syncthreads();
         }
+    }
+    if constexpr (ZERO_DK) {
+        any = __syncthreads_or(any);
+        if constexpr (!PRE) {
+            if (any)
+                for (int64_t base = (int64_t)blockIdx.x * kBlock; base < a.n_elems; base += (int64_t)gridDim.x * kBlock)
+                    if (base + threadIdx.x < a.n_elems && out.kept[a.t_offset + base + threadIdx.x])
+                        keep_dk(nullptr, base);
+        }
+        const int at = (int)blockIdx.x + (int)threadIdx.x;
+        if (threadIdx.x == 0 || (blockIdx.x + 1 == gridDim.x && at < ((int)gridDim.x + 15) / 16 * 16))
+            out.any[at] = threadIdx.x == 0 && any;
     }
     if constexpr (!PRE) wait_for_previous_kernel();
 }
@@ -892,9 +924,9 @@ int launch_t(const CurlArgs &a, cudaStream_t st, size_t smem, int qstride) {
     return SNP_OK;
 }
 
-template <bool HAS_BS, int NQ, bool DIL, bool PRE>
-int launch_packed_pre(const CurlArgs &a, cudaStream_t st, int qstride, const PackedTerms &out) {
-    auto kern = k_curlcurl_packed<HAS_BS, NQ, DIL, PRE>;
+template <bool HAS_BS, int NQ, bool DIL, bool PRE, bool ZERO_DK>
+int launch_packed_pre(const CurlArgs &a, cudaStream_t st, int qstride, const PackedTerms &out, int *blocks) {
+    auto kern = k_curlcurl_packed<HAS_BS, NQ, DIL, PRE, ZERO_DK>;
     const int tables = smem_layout(a.n_orient, a.nq, a.n_int).total;
     const size_t smem = sizeof(double) * ((size_t)tables + (out.D ? 2 : 1) * kBlock * kPackPairs);
     SNP_REQUIRE(smem <= 227 * 1024, "curl-curl assembly: tables need %zu bytes of shared memory", smem);
@@ -909,41 +941,45 @@ int launch_packed_pre(const CurlArgs &a, cudaStream_t st, int qstride, const Pac
                            psmem, st, a, qstride, sums);
         SNP_LAUNCH_CHECK();
     }
-    launch_overlapping(PRE || a.beside, kern, wave_grid(kern, a.n_elems, kBlock, smem), kBlock, smem, st, a, qstride,
-                       tables, out);
+    *blocks = wave_grid(kern, a.n_elems, kBlock, smem);
+    launch_overlapping(PRE || a.beside, kern, *blocks, kBlock, smem, st, a, qstride, tables, out);
     SNP_LAUNCH_CHECK();
     return SNP_OK;
 }
 
 template <bool HAS_BS, int NQ, bool DIL = false>
-int launch_packed_t(const CurlArgs &a, cudaStream_t st, int qstride, const PackedTerms &out) {
+int launch_packed_t(const CurlArgs &a, cudaStream_t st, int qstride, const PackedTerms &out, int *blocks) {
+    *blocks = 0;
     if (a.n_elems == 0) return SNP_OK;
     if constexpr (HAS_BS && NQ == 0) {
         // 4 and 5 points have unrolled element kernels; the next rule has 27, where the separate
         // launch already wins: 49 against 63 us (in the element kernel) at 300k tets, 18 against 31 at
         // 20k, 144 against 160 at 1.1M; 64 points 80 against 123, 27 against 63, 235 against 321
-        if (a.nq >= kManyPoints && (out.J || out.K || out.D)) return launch_packed_pre<HAS_BS, NQ, DIL, true>(a, st, qstride, out);
+        if (a.nq >= kManyPoints && (out.J || out.K || out.D))
+            return out.any ? launch_packed_pre<HAS_BS, NQ, DIL, true, true>(a, st, qstride, out, blocks)
+                           : launch_packed_pre<HAS_BS, NQ, DIL, true, false>(a, st, qstride, out, blocks);
     }
-    return launch_packed_pre<HAS_BS, NQ, DIL, false>(a, st, qstride, out);
+    return out.any ? launch_packed_pre<HAS_BS, NQ, DIL, false, true>(a, st, qstride, out, blocks)
+                   : launch_packed_pre<HAS_BS, NQ, DIL, false, false>(a, st, qstride, out, blocks);
 }
 
 }  // namespace
 
-int launch_curlcurl_packed(const CurlArgs &a, const PackedTerms &out, cudaStream_t st) {
+int launch_curlcurl_packed(const CurlArgs &a, const PackedTerms &out, cudaStream_t st, int *blocks) {
     const int qstride = a.nq * 18;
     if (a.Bs == nullptr) {
-        if (a.nq == 1) return launch_packed_t<false, 1>(a, st, qstride, out);
-        if (a.nq == 4) return launch_packed_t<false, 4>(a, st, qstride, out);
-        return launch_packed_t<false, 0>(a, st, qstride, out);
+        if (a.nq == 1) return launch_packed_t<false, 1>(a, st, qstride, out, blocks);
+        if (a.nq == 4) return launch_packed_t<false, 4>(a, st, qstride, out, blocks);
+        return launch_packed_t<false, 0>(a, st, qstride, out, blocks);
     }
     if (a.phi) {
-        if (a.nq == 4) return launch_packed_t<true, 4, true>(a, st, qstride, out);
-        return launch_packed_t<true, 0, true>(a, st, qstride, out);
+        if (a.nq == 4) return launch_packed_t<true, 4, true>(a, st, qstride, out, blocks);
+        return launch_packed_t<true, 0, true>(a, st, qstride, out, blocks);
     }
-    if (a.nq == 1) return launch_packed_t<true, 1>(a, st, qstride, out);
-    if (a.nq == 4) return launch_packed_t<true, 4>(a, st, qstride, out);
-    if (a.nq == 5) return launch_packed_t<true, 5>(a, st, qstride, out);
-    return launch_packed_t<true, 0>(a, st, qstride, out);
+    if (a.nq == 1) return launch_packed_t<true, 1>(a, st, qstride, out, blocks);
+    if (a.nq == 4) return launch_packed_t<true, 4>(a, st, qstride, out, blocks);
+    if (a.nq == 5) return launch_packed_t<true, 5>(a, st, qstride, out, blocks);
+    return launch_packed_t<true, 0>(a, st, qstride, out, blocks);
 }
 
 bool packed_fits(int32_t n_orient, int32_t nq, int32_t n_int) {

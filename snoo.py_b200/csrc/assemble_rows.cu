@@ -135,8 +135,9 @@ __global__ void __launch_bounds__(kEntryBlock)
 
 // ---------------------------------------------------------------- packed element values
 
-// Element ranges whose dK (constant reluctance) or reduced-rhs terms (no source field) are zero:
-// phase 1 does not store them and phase 2 does not read them.
+// Element ranges whose reduced-rhs terms (no source field) are zero, or whose dK is unless x holds an
+// infinity or a NaN (constant reluctance): phase 1 does not store the zeros and phase 2 does not read
+// them.
 constexpr int kMaxRanges = 16;
 struct ZeroRanges {
     int n = 0;
@@ -166,8 +167,11 @@ struct PackedEntryArgs {
     const double *m0, *m1;  // K (or J) and dK values
     double *K, *dK, *J;
     float *J32;
-    // value indices [lo, hi) whose dK is zero and not stored (up to two ranges)
+    // value indices [lo, hi) whose dK is zero and not stored (up to two ranges), but for the elements
+    // that kept[] lists where one of any[] is set
     uint32_t lo[2], hi[2];
+    const uint8_t *kept, *any;
+    int32_t n_any;  // a multiple of 16
 };
 
 // One thread per CSR entry: its contributions' values (the pattern's coupling words are the value
@@ -177,13 +181,19 @@ struct PackedEntryArgs {
 // elements' values are runs of doubles, so most of each sector is used.  Decoding element and
 // pair from a coupling id and four entries a thread took 1600 instructions per 128 entries
 // (422 us at 1.16M tets); from the block layout the sums took 571 us, this way 205 us.
-template <int MODE>
-__global__ void __launch_bounds__(kEntryBlock) k_cc_entries_packed(PackedEntryArgs r) {
+//
+// KEPT: elements of the ranges may have values (an infinity or a NaN in x).  The ordinary call's loop does
+// not look at kept[]: with one loop for both a call at 1.16M tets took 457 us instead of 445.
+template <int MODE, bool KEPT>
+__device__ __forceinline__ void packed_entries(const PackedEntryArgs &r) {
     auto stored = [&](uint32_t t) {
-        if constexpr (MODE == kEntKD || MODE == kEntD)
-            return !((t >= r.lo[0] && t < r.hi[0]) || (t >= r.lo[1] && t < r.hi[1]));
-        else
+        if constexpr (MODE == kEntKD || MODE == kEntD) {
+            const bool zero = (t >= r.lo[0] && t < r.hi[0]) || (t >= r.lo[1] && t < r.hi[1]);
+            if constexpr (KEPT) return !zero || __ldg(r.kept + t / (uint32_t)kPackPairs) != 0;
+            else return !zero;
+        } else {
             return true;
+        }
     };
     for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < r.nnz; p += (int64_t)gridDim.x * blockDim.x) {
         const int c0 = __ldcs(r.cptr + p), c1 = __ldg(r.cptr + p + 1);
@@ -231,6 +241,19 @@ __global__ void __launch_bounds__(kEntryBlock) k_cc_entries_packed(PackedEntryAr
             __stcs(r.dK + p, s0);
         }
     }
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kEntryBlock) k_cc_entries_packed(PackedEntryArgs r) {
+    if constexpr (MODE == kEntKD || MODE == kEntD) {
+        bool any = false;
+        for (int i = threadIdx.x & 31; i < r.n_any / 16; i += 32) {
+            const uint4 v = __ldg(reinterpret_cast<const uint4 *>(r.any) + i);
+            any |= (v.x | v.y | v.z | v.w) != 0u;
+        }
+        if (__any_sync(0xffffffffu, any)) return packed_entries<MODE, true>(r);
+    }
+    packed_entries<MODE, false>(r);
 }
 
 // F_i and rhs_i from the packed six-term values over DoF i's incidences, in element order
@@ -343,9 +366,13 @@ int launch_curlcurl_rows(const snp_pattern *pat, const double *terms, const Term
     return SNP_OK;
 }
 
+// PackedTerms::any of all launches; a material that finds no room left stores its dK
+static size_t any_bytes(const snp_pattern *pat) { return ((size_t)pat->n_elems / kPackBlock + 256) / 16 * 16; }
+
 size_t curlcurl_system_work(const snp_pattern *pat, const SystemOut &o) {
     const PackedNeeds nd = packed_needs(o);
-    return (size_t)pat->n_elems * ((nd.k + nd.d + nd.j) * kPackPairs + (o.F ? 6 : 0) + (o.rhs ? 6 : 0));
+    const size_t zeros = nd.d ? (any_bytes(pat) + (size_t)pat->n_elems + 15) / 16 * 2 + 2 : 0;
+    return (size_t)pat->n_elems * ((nd.k + nd.d + nd.j) * kPackPairs + (o.F ? 6 : 0) + (o.rhs ? 6 : 0)) + zeros;
 }
 
 int launch_curlcurl_system(const snp_pattern *pat, const CurlArgs *mats, int n_mats, double *work, const SystemOut &o,
@@ -387,17 +414,29 @@ int launch_curlcurl_system(const snp_pattern *pat, const CurlArgs *mats, int n_m
     all.J = take(nd.j, kPackPairs);
     all.F = take(o.F != nullptr, 6);
     all.R = take(o.rhs != nullptr, 6);
+    // read 16 bytes at a time
+    uint8_t *const any = nd.d ? reinterpret_cast<uint8_t *>(((uintptr_t)p + 15) / 16 * 16) : nullptr;
+    uint8_t *const kept = nd.d ? any + any_bytes(pat) : nullptr;
     bool beside = false;
     for (int m = 0; m < n_mats; ++m) {
         CurlArgs a = mats[m];
         if (a.n_elems == 0) continue;
         a.beside = beside;
         PackedTerms out = all;
-        // constant reluctance: dK = 0 (nu' = 0)
-        if (out.D && a.n_int < 0 && zero_dk.n < 2 && zero_dk.add(a.t_offset, a.t_offset + a.n_elems)) out.D = nullptr;
+        // constant reluctance: nu' = 0, and with it dK unless B is not finite
+        const size_t most = (size_t)(a.n_elems / kPackBlock) + 16;
+        if (out.D && a.n_int < 0 && (size_t)r.n_any + most <= any_bytes(pat) && zero_dk.n < 2 &&
+            zero_dk.add(a.t_offset, a.t_offset + a.n_elems)) {
+            out.D = nullptr;
+            out.Dz = all.D;
+            out.kept = kept;
+            out.any = any + r.n_any;
+        }
         if (a.Bs == nullptr) out.R = nullptr;
-        if (out.K || out.D || out.J || out.F || out.R) {
-            SNP_TRY(launch_curlcurl_packed(a, out, st));
+        if (out.K || out.D || out.J || out.F || out.R || out.any) {
+            int blocks = 0;
+            SNP_TRY(launch_curlcurl_packed(a, out, st, &blocks));
+            if (out.any) r.n_any += (blocks + 15) / 16 * 16;
             // the next material's element kernel starts while this one's points are bound by
             // latency (183 -> 175 us a call at 150k tets diluted, 250 -> 235 at 300k); beside a kernel
             // bound by its streams it gains nothing (485 -> 485-510 us at 1.16M tets, 4 points)
@@ -415,6 +454,8 @@ int launch_curlcurl_system(const snp_pattern *pat, const CurlArgs *mats, int n_m
         r.lo[i] = (uint32_t)zero_dk.lo[i] * kPackPairs;
         r.hi[i] = (uint32_t)zero_dk.hi[i] * kPackPairs;
     }
+    r.kept = kept;
+    r.any = any;
     if (r.nnz > 0) {
         if (nd.j) {
             r.m0 = all.J;

@@ -211,8 +211,15 @@ constexpr int kPackPairs = 21;
 constexpr int kPackPairs4 = 10;  // of an element with 4 DoFs
 struct PackedTerms {
     double *K = nullptr, *D = nullptr, *J = nullptr, *F = nullptr, *R = nullptr;
+    // of a material whose dK is zero unless x holds an infinity or a NaN (constant reluctance; D is null):
+    // kept[e] says that the values of element e are not all zero and stand in Dz, any[i] that block i of
+    // the launch met such an element (the last block fills any[] up to a multiple of 16)
+    double *Dz = nullptr;
+    uint8_t *kept = nullptr, *any = nullptr;
 };
-int launch_curlcurl_packed(const CurlArgs &a, const PackedTerms &out, cudaStream_t st);
+constexpr int kPackBlock = 128;  // elements of a block's tile: a launch has at most n_elems / 128 + 1 blocks
+// *blocks: of the launch of the element kernel
+int launch_curlcurl_packed(const CurlArgs &a, const PackedTerms &out, cudaStream_t st, int *blocks);
 // Whether the packed element kernel's tables and tiles fit in shared memory.
 bool packed_fits(int32_t n_orient, int32_t nq, int32_t n_int);
 

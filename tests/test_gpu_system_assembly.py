@@ -62,3 +62,29 @@ def test_system_has_the_bits_of_terms_and_rows(order, diluted):
         T = _two_calls(A, x, order, sf, parts, keys, R)
         for k in keys:
             assert torch.equal(T[k], R[k]), (keys, k)
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf, 1e200])
+@pytest.mark.parametrize("order,air_field", [(2, False), (2, True), (4, True)])
+def test_constant_reluctance_keeps_what_is_not_finite(order, air_field, value):
+    """dK of a material with constant reluctance is nu' times something: 0 for a finite B, else what the
+    products give.  An infinity, a NaN or a large number in x shows in dK and J as in the two-call form."""
+    import torch
+
+    msh = M.window_frame_mesh(3000, jitter=0.15, seed=9)
+    A = S.CurlCurlAssembler(msh, [M.TAG_IRON, M.TAG_AIR], [MAT.atan_reluctance(), S.ConstantReluctance(NU0)])
+    rng = np.random.default_rng(order)
+    x = torch.from_numpy(rng.normal(0, 2e-3, msh.num_dofs)).cuda()
+    gids = A._device_state()["mats"][1]["gids"].view(-1, 6)
+    x[gids[[0, 200, 201], [0, 3, 5]].long()] = value
+    nq = A.tables(order).nq
+    sf = [rng.normal(0, 0.5, (len(A._elems[0]) * nq, 3)),
+          rng.normal(0, 0.5, (len(A._elems[1]) * nq, 3)) if air_field else np.zeros((0, 3))]
+    K, DK, F, RHS = _lib.TERMS_K, _lib.TERMS_DK, _lib.TERMS_F, _lib.TERMS_RHS
+    for parts, keys in ((K | DK | F | RHS, ("K", "dK", "J", "rhs", "F")), (K | DK, ("J",)), (DK, ("dK",))):
+        R = A.assemble_device(x, order, sf, method="rows", **{k: k in keys for k in ("K", "dK", "J", "rhs", "F")})
+        T = _two_calls(A, x, order, sf, parts, keys, R)
+        for k in keys:
+            assert torch.equal(T[k].isnan(), R[k].isnan()) and torch.equal(T[k].nan_to_num(), R[k].nan_to_num()), (keys, k)
+        matrix = "dK" if "dK" in keys else "J"
+        assert bool(T[matrix].isfinite().all()) == np.isfinite(value)  # 0 times a large B is 0
