@@ -759,25 +759,23 @@ __global__ void __launch_bounds__(kDofThreads, 4)
                 if (before) pass_begins();
                 if (yb) bulk_load(D.y, a.Y + c0, yb, full + s);
             };
-            int issued = 0;
+            int it = 0;
             int32_t tile = blockIdx.x;
-            for (; issued < kDofStages && tile < a.tiles; ++issued, tile += gridDim.x) issue(tile, issued, issued == 0);
-            if (issued == 0) pass_begins();
-            if (*(volatile int *)&st->done) {
-                // a finished solve: the copies in flight end before the block does
-                for (int s = 0; s < issued; ++s) mbar_wait_bounded(full + s, 0);
-            } else {
-                for (int it = issued; tile < a.tiles; ++it, tile += gridDim.x) {
+            for (; it < kDofStages && tile < a.tiles; ++it, tile += gridDim.x) issue(tile, it, it == 0);
+            if (it == 0) pass_begins();
+            if (!*(volatile int *)&st->done)
+                for (; tile < a.tiles; ++it, tile += gridDim.x) {
                     const int s = it % kDofStages;
                     if (!mbar_wait_bounded(empty + s, (uint32_t)((it / kDofStages - 1) & 1), &s_fail)) {
                         s_fail = 1;
-                        for (int q = 0; q < kDofStages; ++q)
-                            mbar_wait_bounded(full + q, (uint32_t)(((it - 1 - (it - 1 - q) % kDofStages) / kDofStages) & 1));
                         break;
                     }
                     issue(tile, s, false);
                 }
-            }
+            // However its threads leave, the copies in flight end before the block does: its consumers may
+            // go by a done that this thread did not see yet.
+            for (int q = it > kDofStages ? it - kDofStages : 0; q < it; ++q)
+                mbar_wait_bounded(full + q % kDofStages, (uint32_t)((q / kDofStages) & 1));
         }
         __syncwarp();
     } else {

@@ -39,3 +39,20 @@ def test_staged_dof_pass_leaves_together():
     assert not re.search(r"\b(return|break|continue|goto)\b", between)
     waits = re.findall(r"\bmbar_\w*wait\w*|__syncthreads|consumer_sync\w*|mbar_try", producer)
     assert waits and set(waits) == {"mbar_wait_bounded"}
+
+
+def test_staged_dof_pass_waits_for_its_copies():
+    """The consumer warps may leave by a ``done`` that the producer thread did not see.  The thread that
+    issued the copies waits for the last of every stage on each way out."""
+    body = _kernel("k_epass2_bj")
+    producer = body[body.index("if (producer)"):re.search(r"}\s*else\s*{?[^{]*pass_begins\(\)", body).start()]
+    tail = producer[producer.rindex("for ("):]
+    assert re.match(r"for \(int q = it > kDofStages \? it - kDofStages : 0; q < it; \+\+q\)\s*"
+                    r"mbar_wait_bounded\(full \+ q % kDofStages, \(uint32_t\)\(\(q / kDofStages\) & 1\)\);\s*}\s*"
+                    r"__syncwarp\(\);\s*$", tail)
+    # the loop stands behind every branch and loop of the thread's own block, and nothing returns before it
+    before = producer[producer.index("int it = 0;"):producer.rindex("for (")]
+    assert before.count("{") == before.count("}") and "return" not in before and "goto" not in before
+    # each copy counts once: the stage and phase waited for are those of the issue
+    assert len(re.findall(r"\bissue\(tile, it, it == 0\)", before)) == 1
+    assert re.search(r"const int s = it % kDofStages;.*issue\(tile, s, false\);", before, re.S)
