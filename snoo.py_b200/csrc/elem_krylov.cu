@@ -384,8 +384,7 @@ __global__ void __launch_bounds__(kTileElems, 4)
     }
 }
 
-template <typename TT>
-__device__ __forceinline__ void load_chat(TT *sc, const TT *chat) {
+__device__ __forceinline__ void load_chat(float *sc, const float *chat) {
     if (threadIdx.x < 18) sc[threadIdx.x] = chat[threadIdx.x];
     __syncthreads();
 }
@@ -395,28 +394,23 @@ __device__ __forceinline__ void load_chat(TT *sc, const TT *chat) {
 // each lane gathers three DoF states, the halves of u_e meet through one shuffle, and each
 // lane stores its three edge terms (half the registers of one lane per element, so twice
 // the resident warps keep the same number of gathers in flight).
-template <typename TT>
 __global__ void __launch_bounds__(kEBlock, 4)
     k_epass1_pair(int64_t ne, const int32_t *__restrict__ edof, const int32_t *__restrict__ pos,
-             const TT *__restrict__ T, const TT *__restrict__ chat, const DofPair<TT> *G,
-             TT *Y, PcgState *st, double *part, int early) {
-    __shared__ TT sc[18];
+                  const float *__restrict__ T, const float *__restrict__ chat, const DofPair<float> *G, float *Y,
+                  PcgState *st, double *part, int early) {
+    __shared__ float sc[18];
     __shared__ double sh[32];
     const int lane = threadIdx.x & 31;
     const int h = lane & 1;  // edges 3h .. 3h+2
     // a warp takes 16 consecutive elements per pass; the loop bound is uniform across the warp
     const int64_t wstride = (int64_t)gridDim.x * (blockDim.x >> 5) * 16;
     const int64_t first = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 16;
-    // every streamed word of a pass is requested before its gathers: the lane's three DoF words,
-    // slots and tensor components (the partner lane holds the other three); the first pass's
-    // words before the CG state is read
-    // In float32 the words of the warp's next pass are requested while this pass gathers, one
-    // pass ahead (in float64 their registers need a lower occupancy target, which cost more:
-    // 78.1 -> 79-82 us per iteration at 1.16M tets with three blocks per SM).
-    constexpr bool kAhead = sizeof(TT) == 4;
+    // every streamed word of a pass is requested one pass ahead, while the one before gathers: the
+    // lane's three DoF words, slots and tensor components (the partner lane holds the other three); the
+    // first pass's words before the CG state is read
     int32_t d[3], ps[3], nd[3], nps[3];
-    TT th[3], nth[3];
-    auto stream_in = [&](int64_t e0, int32_t(&od)[3], int32_t(&ops)[3], TT(&oth)[3]) {
+    float th[3], nth[3];
+    auto stream_in = [&](int64_t e0, int32_t(&od)[3], int32_t(&ops)[3], float(&oth)[3]) {
         const int64_t e = e0 + (lane >> 1);
         const bool valid = e < ne;
         const int64_t eb = eslot(valid ? e : 0, 0);
@@ -424,50 +418,46 @@ __global__ void __launch_bounds__(kEBlock, 4)
         for (int j = 0; j < 3; ++j) {
             od[j] = valid ? __ldcs(edof + eb + 32 * (3 * h + j)) : 0;
             ops[j] = valid ? __ldcs(pos + eb + 32 * (3 * h + j)) : 0;
-            oth[j] = valid ? __ldcs(T + eb + 32 * (3 * h + j)) : TT(0);
+            oth[j] = valid ? __ldcs(T + eb + 32 * (3 * h + j)) : 0.0f;
         }
     };
     if (first < ne) stream_in(first, d, ps, th);
     pass_begins();
     if (st->done) return;
     load_chat(sc, chat);
-    const TT beta = (TT)st->beta;
+    const float beta = (float)st->beta;
     double dot = 0.0;
 #pragma unroll 1
     for (int64_t e0 = first; e0 < ne; e0 += wstride) {
         const int64_t e = e0 + (lane >> 1);
         const bool valid = e < ne;
-        if constexpr (kAhead) {
-            if (e0 != first) {
+        if (e0 != first) {
 #pragma unroll
-                for (int j = 0; j < 3; ++j) {
-                    d[j] = nd[j];
-                    ps[j] = nps[j];
-                    th[j] = nth[j];
-                }
+            for (int j = 0; j < 3; ++j) {
+                d[j] = nd[j];
+                ps[j] = nps[j];
+                th[j] = nth[j];
             }
-            if (e0 + wstride < ne) stream_in(e0 + wstride, nd, nps, nth);
-        } else {
-            if (e0 != first) stream_in(e0, d, ps, th);
         }
-        DofPair<TT> w[3];
+        if (e0 + wstride < ne) stream_in(e0 + wstride, nd, nps, nth);
+        DofPair<float> w[3];
 #pragma unroll
         for (int j = 0; j < 3; ++j) w[j] = G[(uint32_t)d[j] & ~kSignBit];
-        TT u0 = TT(0), u1 = TT(0), u2 = TT(0);
+        float u0 = 0.0f, u1 = 0.0f, u2 = 0.0f;
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
-            TT pk = pnext(beta, w[j].b, w[j].a);
+            float pk = pnext(beta, w[j].b, w[j].a);
             if (d[j] < 0) pk = -pk;
-            const TT *c = sc + 3 * (3 * h + j);
+            const float *c = sc + 3 * (3 * h + j);
             u0 += pk * c[0];
             u1 += pk * c[1];
             u2 += pk * c[2];
         }
-        if (!valid) u0 = u1 = u2 = TT(0);
+        if (!valid) u0 = u1 = u2 = 0.0f;
         // u_e = (edges 0-2) + (edges 3-5), added in that order on both lanes
-        const TT o0 = __shfl_xor_sync(0xffffffffu, u0, 1);
-        const TT o1 = __shfl_xor_sync(0xffffffffu, u1, 1);
-        const TT o2 = __shfl_xor_sync(0xffffffffu, u2, 1);
+        const float o0 = __shfl_xor_sync(0xffffffffu, u0, 1);
+        const float o1 = __shfl_xor_sync(0xffffffffu, u1, 1);
+        const float o2 = __shfl_xor_sync(0xffffffffu, u2, 1);
         if (h) {
             u0 = o0 + u0;
             u1 = o1 + u1;
@@ -477,17 +467,17 @@ __global__ void __launch_bounds__(kEBlock, 4)
             u1 = u1 + o1;
             u2 = u2 + o2;
         }
-        TT t[6];
+        float t[6];
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
-            const TT other = __shfl_xor_sync(0xffffffffu, th[j], 1);
+            const float other = __shfl_xor_sync(0xffffffffu, th[j], 1);
             t[j] = h ? other : th[j];
             t[3 + j] = h ? th[j] : other;
         }
         if (!valid) continue;
-        const TT v0 = t[0] * u0 + t[1] * u1 + t[2] * u2;
-        const TT v1 = t[1] * u0 + t[3] * u1 + t[4] * u2;
-        const TT v2 = t[2] * u0 + t[4] * u1 + t[5] * u2;
+        const float v0 = t[0] * u0 + t[1] * u1 + t[2] * u2;
+        const float v1 = t[1] * u0 + t[3] * u1 + t[4] * u2;
+        const float v2 = t[2] * u0 + t[4] * u1 + t[5] * u2;
         if (!h) dot += (double)u0 * (double)v0 + (double)u1 * (double)v1 + (double)u2 * (double)v2;
 #pragma unroll
         for (int j = 0; j < 3; ++j)
@@ -683,9 +673,8 @@ constexpr int kDofStages = 2;
 constexpr int kIncCap = 1536;  // slots of a tile staged in shared memory (1290 on average)
 constexpr int kPackMax = kBjTile / kBjMax * (kBjMax * (kBjMax + 1) / 2);  // packed entries of a tile, at most
 
-template <typename TT>
 struct __align__(128) DofStage {
-    TT y[kIncCap + 8];
+    double y[kIncCap + 8];
     float m[kPackMax];
     uint32_t word[kBjTile];
 };
@@ -708,24 +697,23 @@ __device__ __forceinline__ bool consumer_sync_any(bool fail) {
         : "memory");
     return any != 0;
 }
-template <typename TT>
 struct DofPassArgs {
-    int32_t n, tiles;
+    int32_t tiles;
     const uint32_t *word;
     const int32_t *tile_inc, *tile_m;
     const int32_t *inc_ptr;  // only for plans whose words do not hold the starts
     const float *packed;
-    const TT *Y;
-    DofPair<TT> *G, *R;
+    const double *Y;
+    DofPair<double> *G, *R;
 };
 
-template <typename TT>
 __global__ void __launch_bounds__(kDofThreads, 4)
-    k_epass2_bj(const DofPassArgs<TT> a, PcgState *st, double *part, int use_cond, cudaGraphConditionalHandle cond, int early) {
+    k_epass2_bj(const DofPassArgs a, PcgState *st, double *part, int use_cond, cudaGraphConditionalHandle cond,
+                int early) {
     extern __shared__ __align__(128) unsigned char dof_smem[];
-    DofStage<TT> *stage = reinterpret_cast<DofStage<TT> *>(dof_smem);
+    DofStage *stage = reinterpret_cast<DofStage *>(dof_smem);
     __shared__ double sh2[2][32];
-    __shared__ TT s_r2[2][kBjTile];
+    __shared__ double s_r2[2][kBjTile];
     __shared__ uint64_t full[kDofStages], empty[kDofStages];
     __shared__ TileInfo info[kDofStages];
     __shared__ volatile int s_fail;
@@ -744,15 +732,15 @@ __global__ void __launch_bounds__(kDofThreads, 4)
     if (producer) {
         if (threadIdx.x == kEBlock) {
             auto issue = [&](int32_t tile, int s, bool before) {
-                DofStage<TT> &D = stage[s];
-                constexpr int kA = 16 / (int)sizeof(TT);  // values per 16 bytes
+                DofStage &D = stage[s];
+                constexpr int kA = 2;  // values per 16 bytes
                 const int32_t i0 = __ldg(a.tile_inc + tile), i1 = __ldg(a.tile_inc + tile + 1);
                 const int32_t m0 = __ldg(a.tile_m + tile), m1 = __ldg(a.tile_m + tile + 1);
                 const int32_t c0 = i0 & ~(kA - 1), cn = (i1 - c0 + kA - 1) & ~(kA - 1);
                 const bool staged = i1 - i0 <= kIncCap;
                 info[s] = TileInfo{i0, i1 - i0, staged ? i0 - c0 : -1};
                 const uint32_t mb = (uint32_t)(m1 - m0) * 4u;
-                const uint32_t yb = staged && i1 > i0 ? (uint32_t)(cn * (int)sizeof(TT)) : 0u;
+                const uint32_t yb = staged && i1 > i0 ? (uint32_t)(cn * (int)sizeof(double)) : 0u;
                 mbar_arrive_expect(full + s, kBjTile * 4u + mb + yb);
                 bulk_load(D.word, a.word + (int64_t)tile * kBjTile, kBjTile * 4u, full + s);
                 if (mb) bulk_load(D.m, a.packed + m0, mb, full + s);
@@ -786,20 +774,20 @@ __global__ void __launch_bounds__(kDofThreads, 4)
         // tile's loads no longer wait for done: 34.8 -> 34.4 and 56.4 -> 56.0 us per iteration at
         // 600k and 1.16M tets (55.9 -> 57.0 with a volatile read).
         const bool finished = st->done != 0;
-        const TT alpha = (TT)st->alpha, beta = (TT)st->beta;
+        const double alpha = st->alpha, beta = st->beta;
         const int tid = threadIdx.x;
         int it = 0;
         for (int32_t tile = blockIdx.x; tile < a.tiles; tile += gridDim.x, ++it) {
             const int s = it % kDofStages;
-            const DofStage<TT> &D = stage[s];
-            TT *s_r = s_r2[it & 1];
+            const DofStage &D = stage[s];
+            double *s_r = s_r2[it & 1];
             const int64_t i = (int64_t)tile * kBjTile + tid;  // the states are padded to whole tiles
-            const DofPair<TT> g = a.G[i], rx = a.R[i];
+            const DofPair<double> g = a.G[i], rx = a.R[i];
             const bool here = mbar_wait_bounded(full + s, (uint32_t)((it / kDofStages) & 1));
             const TileInfo ti = info[s];
             const uint32_t w = D.word[tid];
             const bool fr = here && ((w >> 6) & 1u);
-            TT r = TT(0);
+            double r = 0.0;
             if (fr) {
                 int b0, b1;
                 if (a.inc_ptr == nullptr) {
@@ -811,10 +799,10 @@ __global__ void __launch_bounds__(kDofThreads, 4)
                 }
                 double q = 0.0;
                 if (ti.shift >= 0)
-                    for (int t = b0; t < b1; ++t) q += (double)D.y[ti.shift + t];
+                    for (int t = b0; t < b1; ++t) q += D.y[ti.shift + t];
                 else
-                    for (int t = b0; t < b1; ++t) q += (double)a.Y[ti.first + t];
-                r = rx.a - alpha * (TT)q;
+                    for (int t = b0; t < b1; ++t) q += a.Y[ti.first + t];
+                r = rx.a - alpha * q;
             }
             s_r[tid] = r;
             // r alternates between two buffers: a tile writes the one whose readers of two tiles ago
@@ -827,16 +815,16 @@ __global__ void __launch_bounds__(kDofThreads, 4)
             if (fr) {
                 const int o = (int)(w & 7u), size = (int)((w >> 3) & 7u) + 1;
                 const float *m = D.m + ((w >> 7) & 0x7ffu);
-                const TT *rb = s_r + (tid - o);
-                TT z = TT(0);
+                const double *rb = s_r + (tid - o);
+                double z = 0.0;
 #pragma unroll
                 for (int c = 0; c < kBjMax; ++c)
-                    if (c < size) z = fma((TT)m[c <= o ? o * (o + 1) / 2 + c : c * (c + 1) / 2 + o], rb[c], z);
-                const TT p = pnext(beta, g.b, g.a);
-                a.G[i] = DofPair<TT>{z, p};
-                a.R[i] = DofPair<TT>{r, rx.b + alpha * p};
-                rz += (double)r * (double)z;
-                rr += (double)r * (double)r;
+                    if (c < size) z = fma((double)m[c <= o ? o * (o + 1) / 2 + c : c * (c + 1) / 2 + o], rb[c], z);
+                const double p = pnext(beta, g.b, g.a);
+                a.G[i] = DofPair<double>{z, p};
+                a.R[i] = DofPair<double>{r, rx.b + alpha * p};
+                rz += r * z;
+                rr += r * r;
             }
             __syncwarp();
             if ((tid & 31) == 0) mbar_arrive(empty + s);
@@ -858,9 +846,8 @@ __global__ void __launch_bounds__(kDofThreads, 4)
     close_dof_pass(rz, rr, sh2, part, st, use_cond, cond);
 }
 
-template <typename TT>
 constexpr size_t dof_pass_smem() {
-    return kDofStages * sizeof(DofStage<TT>);
+    return kDofStages * sizeof(DofStage);
 }
 
 template <typename TT>
@@ -1814,9 +1801,16 @@ int ElemPcg<TT>::launch_iteration(const ElemTopology &top, const TT *T, const ui
                                   cudaGraphConditionalHandle cond) {
     const Chat<TT> ch = chat_of<TT>(top);
     const int32_t *slot_ptr = sizeof(TT) == 8 ? top.slot_ptr64() : top.inc_ptr.p;
-    const int staged_grid =
-        plan ? wave_grid(k_epass2_bj<TT>, (int64_t)plan->tiles * kDofThreads, kDofThreads, dof_pass_smem<TT>()) : 0;
-    const bool staged = plan && sizeof(TT) == 8 && plan->tiles >= 4 * staged_grid;
+    // the staged DoF pass in float64 from four tiles per block on: 39.5 against 40.3 us per iteration
+    // at 600k tets, 69.9 against 74.7 at 1.16M; below, 25.7 against 25.4 at 287k and 16.5 against
+    // 15.7 at 100k (in float32 it gained 1% at 1.16M and nothing at 38k)
+    int staged_grid = 0;
+    bool staged = false;
+    if constexpr (sizeof(TT) == 8)
+        if (plan) {
+            staged_grid = wave_grid(k_epass2_bj, (int64_t)plan->tiles * kDofThreads, kDofThreads, dof_pass_smem());
+            staged = plan->tiles >= 4 * staged_grid;
+        }
     // Where a pass lets the next one start before its block sums: in float32 (per iteration at 38k,
     // 150k and 300k tets 13.0, 16.3 and 21.7 us without, 12.3, 15.8 and 20.9 with; launches that do
     // not overlap 13.6, 16.8 and 22.3) and in float64 around the staged DoF pass (69.2 against 67.8
@@ -1824,39 +1818,33 @@ int ElemPcg<TT>::launch_iteration(const ElemTopology &top, const TT *T, const ui
     // 12.5, 18.5 and 24.7 without, 13.3, 19.2 and 25.5 with (12.7, 18.9 and 24.9 not overlapping).
     const int early = sizeof(TT) == 4 || staged ? 1 : 0;
     if constexpr (sizeof(TT) == 4)
-        launch_overlapping(true, k_epass1_pair<TT>, wave_grid(k_epass1_pair<TT>, 2 * ne, kEBlock), kEBlock, 0, s, ne,
-                           top.edof.p, top.pos.p, T, chat_ptr<TT>(top), G.p, Y.p, st.p, part.p, early);
+        launch_overlapping(true, k_epass1_pair, wave_grid(k_epass1_pair, 2 * ne, kEBlock), kEBlock, 0, s, ne, top.edof.p,
+                           top.pos.p, T, chat_ptr<float>(top), G.p, Y.p, st.p, part.p, early);
     else if (top.tile.te)
         launch_tile_pass(top, T, early, s);
     else
         launch_overlapping(true, k_epass1<TT>, wave_grid(k_epass1<TT>, ne, kEBlock), kEBlock, 0, s, ne, top.edof.p,
                            top.pos.p, T, ch, G.p, Y.p, st.p, part.p, early);
     SNP_LAUNCH_CHECK();
-    // the staged DoF pass in float64 from four tiles per block on: 39.5 against 40.3 us per iteration
-    // at 600k tets, 69.9 against 74.7 at 1.16M; below, 25.7 against 25.4 at 287k and 16.5 against
-    // 15.7 at 100k (float32: 52.4 against 53.1 at 1.16M, 13.3 against 13.3 at 38k)
-    if (plan && !staged) {
+    if (staged) {
+        if constexpr (sizeof(TT) == 8) {
+            DofPassArgs a;
+            a.tiles = plan->tiles;
+            a.word = plan->word.p;
+            a.tile_inc = plan->tile_inc.p;
+            a.tile_m = plan->tile_m.p;
+            a.inc_ptr = plan->wide ? slot_ptr : nullptr;
+            a.packed = plan->packed.p;
+            a.Y = Y.p;
+            a.G = G.p;
+            a.R = R.p;
+            launch_overlapping(true, k_epass2_bj, staged_grid, kDofThreads, dof_pass_smem(), s, a, st.p, part.p, use_cond,
+                               cond, early);
+        }
+    } else if (plan) {
         launch_overlapping(true, k_epass2_direct<TT>, wave_grid(k_epass2_direct<TT>, n, kEBlock), kEBlock, 0, s, n,
                            free_mask, slot_ptr, Y.p, plan->meta, plan->binv, G.p, R.p, st.p, part.p, use_cond,
                            cond, early);
-        SNP_LAUNCH_CHECK();
-        return SNP_OK;
-    }
-    if (plan) {
-        DofPassArgs<TT> a;
-        a.n = n;
-        a.tiles = plan->tiles;
-        a.word = plan->word.p;
-        a.tile_inc = plan->tile_inc.p;
-        a.tile_m = plan->tile_m.p;
-        a.inc_ptr = plan->wide ? slot_ptr : nullptr;
-        a.packed = plan->packed.p;
-        a.Y = Y.p;
-        a.G = G.p;
-        a.R = R.p;
-        const size_t smem = dof_pass_smem<TT>();
-        launch_overlapping(true, k_epass2_bj<TT>, staged_grid, kDofThreads, smem, s, a, st.p, part.p, use_cond, cond,
-                           early);
     } else {
         launch_overlapping(true, k_epass2<TT>, wave_grid(k_epass2<TT>, n, kEBlock), kEBlock, 0, s, n, free_mask,
                            slot_ptr, Y.p, G.p, R.p, D.p, st.p, part.p, use_cond, cond, early);

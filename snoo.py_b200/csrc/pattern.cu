@@ -235,11 +235,8 @@ int pattern_create(const int32_t *elem_dofs, int64_t n_elems, int32_t dpe, int32
             if ((rc = P->cid.alloc(n)) || (rc = P->cptr.alloc(P->nnz + 1))) return cleanup_fail(rc);
             if (dpe == 6)
                 k_pair_words<6><<<stride_grid(n, 256, 16), 256, 0, st>>>(n, dv.Current(), P->cid.p);
-            else if (dpe == 4)
+            else
                 k_pair_words<4><<<stride_grid(n, 256, 16), 256, 0, st>>>(n, dv.Current(), P->cid.p);
-            else if (cudaMemcpyAsync(P->cid.p, dv.Current(), sizeof(int32_t) * n, cudaMemcpyDeviceToDevice, st) !=
-                     cudaSuccess)
-                return cleanup_fail(fail(SNP_CUDA_ERROR, "snp_pattern_create: copy of the sorted couplings failed"));
             k_cptr<<<stride_grid(n, 256, 16), 256, 0, st>>>(head.p, pos.p, n, P->cptr.p);
             const int32_t nn = (int32_t)n;
             if (cudaMemcpyAsync(P->cptr.p + P->nnz, &nn, sizeof(int32_t), cudaMemcpyHostToDevice, st) != cudaSuccess ||
