@@ -189,15 +189,16 @@ def bytes_elem_pcg_iteration(ne, n, tb=8, block_jacobi=False):
     return ne * (24 + 6 * tb + 24) + (n + 1) * 4 + 9 * n * tb
 
 
-# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one matrix-free PCG iteration,
-# k_epass1 + k_epass2 (point Jacobi) or k_epass1 + k_epass2_bj (block Jacobi), from ncu
-# captures of the 1,164,240-tet workload (cold cache: ncu flushes L2 before every replay pass,
-# so slot values and DoF states that stay in L2 between the two passes of a live run are
-# counted as DRAM traffic here).  Summaries and commands: profiles/elem_pcg_passes_window_frame_1p2M.md
-# and profiles/elem_pcg_block_jacobi_window_frame_1p2M.md.  Scaled by the element count.
-MEASURED_TRAFFIC = {"ne": 1_164_240, "fp64": (143.15e6 + 129.10e6), "mixed": (100.94e6 + 62.43e6),
-                    "fp64_bj": (135.04e6 + 7.03e6 + 152.77e6 + 16.10e6),
-                    "mixed_bj": (95.13e6 + 4.47e6 + 103.08e6 + 2.18e6)}
+# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one matrix-free PCG iteration from
+# ncu captures of the 1,164,240-tet workload: float64 k_epass1_tile + k_epass2 (point Jacobi) or
+# k_epass2_bj (block Jacobi), mixed k_epass1_pair + k_epass2 or k_epass2_direct (cold cache: ncu flushes
+# L2 before a launch, so slot values and DoF states that stay in L2 between the two passes of a live run
+# are counted as DRAM traffic here).  Summary and commands:
+# profiles/elem_pcg_block_jacobi_window_frame_1p2M.md.  Scaled by the element count.
+MEASURED_TRAFFIC = {"ne": 1_164_240, "fp64": (138.88e6 + 4.12e6 + 83.21e6 + 1.04e6),
+                    "mixed": (95.02e6 + 5.02e6 + 62.01e6 + 0.01e6),
+                    "fp64_bj": (138.92e6 + 3.93e6 + 92.84e6 + 3.89e6),
+                    "mixed_bj": (95.08e6 + 5.23e6 + 103.46e6 + 1.96e6)}
 
 
 def measured_traffic(layout, precision, ne, block_jacobi=False):
@@ -311,9 +312,11 @@ def run_ours(args):
     if layout == "elem":
         b_it = bytes_elem_pcg_iteration(ne, n, vb, block_jacobi=bj)
         b_apply = bytes_elem_apply(ne, n, vb)
-        kern_name = ("pcg_iteration (k_epass1 element pass + k_epass2_bj block-Jacobi DoF pass; the block build of "
+        # the float64 forms of large meshes; smaller ones take k_epass1 and k_epass2_direct
+        pass1, pass2 = ("k_epass1_tile", "k_epass2_bj") if args.precision == "fp64" else ("k_epass1_pair", "k_epass2_direct")
+        kern_name = (f"pcg_iteration ({pass1} element pass + {pass2} block-Jacobi DoF pass; the block build of "
                      "each Newton step, k_bj_entries + k_bj_invert, inside the timed Krylov region)" if bj else
-                     "pcg_iteration (k_epass1 element pass + k_epass2 DoF pass)")
+                     f"pcg_iteration ({pass1} element pass + k_epass2 DoF pass)")
     else:
         b_it = bytes_pcg_iteration(nnz, n, vb, xb)
         b_apply = bytes_spmv(nnz, n, vb, xb)

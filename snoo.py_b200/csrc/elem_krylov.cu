@@ -662,15 +662,16 @@ __global__ void __launch_bounds__(kEBlock)
 
 // ---- DoF pass with block Jacobi, staged
 //
-// A tile's slot values, DoF words and packed block inverses are contiguous runs, which a ninth
-// warp copies into shared memory with bulk copies one to two tiles ahead.  Bound by memory: 126 MB
-// read and 44 MB written at 1.16M tets in float64 (25 MB less than with unpacked block rows), 26 us
-// where loads in each thread's own order took 30 (the slot run of a DoF is 40 bytes from the
-// next lane's, so their L1 slots were the limit).  Its start is longer by the copy engine's
-// latency, so it serves blocks with several tiles.
+// In float64.  A tile's slot values, DoF words and packed block inverses are contiguous runs, which a
+// ninth warp copies into shared memory with bulk copies one to two tiles ahead.  Bound by the latency
+// of a tile's wait and barrier and by its streams: with a tile plan 93 MB read from a cold cache at
+// 1.16M tets, 22.3 us (serialised); with a slot per element edge 126 MB read and 44 MB written, 26 us where
+// loads in each thread's own order took 30 (the slot run of a DoF is 40 bytes from the next lane's
+// there, so their L1 slots were the limit; with a plan it is 16).  Its start is longer by the copy
+// engine's latency, so it serves blocks with several tiles.
 constexpr int kDofThreads = kEBlock + 32;
 constexpr int kDofStages = 2;
-constexpr int kIncCap = 1536;  // slots of a tile staged in shared memory (1290 on average)
+constexpr int kIncCap = 1536;  // slots of a tile staged (window-frame meshes: 510 with a tile plan, 1280 without)
 constexpr int kPackMax = kBjTile / kBjMax * (kBjMax * (kBjMax + 1) / 2);  // packed entries of a tile, at most
 
 struct __align__(128) DofStage {
@@ -697,6 +698,7 @@ __device__ __forceinline__ bool consumer_sync_any(bool fail) {
         : "memory");
     return any != 0;
 }
+
 struct DofPassArgs {
     int32_t tiles;
     const uint32_t *word;
@@ -1801,9 +1803,10 @@ int ElemPcg<TT>::launch_iteration(const ElemTopology &top, const TT *T, const ui
                                   cudaGraphConditionalHandle cond) {
     const Chat<TT> ch = chat_of<TT>(top);
     const int32_t *slot_ptr = sizeof(TT) == 8 ? top.slot_ptr64() : top.inc_ptr.p;
-    // the staged DoF pass in float64 from four tiles per block on: 39.5 against 40.3 us per iteration
-    // at 600k tets, 69.9 against 74.7 at 1.16M; below, 25.7 against 25.4 at 287k and 16.5 against
-    // 15.7 at 100k (in float32 it gained 1% at 1.16M and nothing at 38k)
+    // The staged DoF pass in float64 from four tiles per block on.  Per iteration, block build included,
+    // 36.4 against 38.1 us at 583k tets and 59.2 against 63.9 at 1.16M; below, 26.8 against 26.4 at 287k (at
+    // 433k already 30.2 against 31.6: the line could lie lower), and before the tile plan 16.5
+    // against 15.7 at 100k.  In float32 it gained 1% at 1.16M and nothing at 38k.
     int staged_grid = 0;
     bool staged = false;
     if constexpr (sizeof(TT) == 8)

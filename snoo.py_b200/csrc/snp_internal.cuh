@@ -269,7 +269,7 @@ struct snp_pattern {
     snp::DevBuf<int32_t> row_ptr, col_idx, slots, diag_pos;
     // contributions of every CSR entry p: the element pairs (e, a, b) that add into it, in element
     // order, cid[cptr[p] .. cptr[p + 1]); as words e * 21 + (upper-triangle index of (a, b)) with 6
-    // DoFs per element, e * 16 + a * 4 + b with 4
+    // DoFs per element, e * 10 + (that index) with 4
     snp::DevBuf<int32_t> cid, cptr;
     bool has_contrib = false;
     // incidence lists of the rows (6 DoFs per element, fewer than 2^28 elements): row r's

@@ -129,8 +129,6 @@ struct Pcg {
 //                 y_e,k = s_k chat_k . v_e stored at their slots of the DoF-ordered incidence
 //   DoF pass      y_i = sum of the DoF's slots, a contiguous range
 
-// Element topology of the operator: DoFs with edge signs and the DoF -> (element, local
-// edge) incidence, built once per mesh.
 // Tiles of consecutive elements for the float64 element pass: the distinct DoFs of a tile ("pairs"
 // of tile and DoF), tile by tile, DoFs ascending.  A pair's terms are summed inside the tile and
 // leave as one slot value; slots are numbered by DoF, then tile.
@@ -145,6 +143,8 @@ struct TilePlan {
     DevBuf<int32_t> slot_ptr;   // [n + 1] first slot of each DoF
 };
 
+// Element topology of the operator: DoFs with edge signs and the DoF -> (element, local
+// edge) incidence, built once per mesh.
 struct ElemTopology {
     int64_t n_elems = 0;
     int32_t n = 0;
